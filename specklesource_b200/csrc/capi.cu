@@ -295,6 +295,18 @@ const float2* tw_table(sb_context* c, int N)
     return (const float2*)sb_table(c, "tw" + std::to_string(N), h);
 }
 
+const float2* batch_tw_table(sb_context* c, int N1, int N2)
+{
+    const int N = N1 * N2;
+    std::vector<float2> h(N);
+    for (int k1 = 0; k1 < N1; ++k1)
+        for (int n2 = 0; n2 < N2; ++n2) {
+            const double ang = -2.0 * kPi * (double)(k1 * n2) / (double)N;
+            h[k1 * N2 + n2] = make_float2((float)cos(ang), (float)sin(ang));
+        }
+    return (const float2*)sb_table(c, "twb" + std::to_string(N), h);
+}
+
 // tau_1[k'] = +exp(+2 pi i k'/(2W)) for k' < W/2, -exp(...) for k' >= W/2.
 const float2* tau_table(sb_context* c, int W)
 {

@@ -49,6 +49,10 @@ int sb_ctx_cuda(sb_context* c, cudaError_t e, const char* what);
 void* sb_ctx_buf(sb_context* c, const char* name, size_t bytes, cudaError_t* err);
 int sb_image_to_device(sb_context* c, const sb_image* im, const char* name, const void** dptr);
 const float2* tw_table(sb_context* c, int N);
+const float2* tau_table(sb_context* c, int W);
+// Twiddles of a batched line transform of N1 N2 points in step order
+// (fft_batch.cuh).
+const float2* batch_tw_table(sb_context* c, int N1, int N2);
 // Loads the allocation-free entry point's kernels and its file-scope workspace
 // on the current device (noalloc.cu).
 cudaError_t sb_noalloc_prepare();

@@ -125,7 +125,9 @@ __device__ __forceinline__ float2 twmul_rt(float2 v, const float2* __restrict__ 
 }
 
 // ---------------------------------------------------------------- register DFT
-template <int R, int DIR, int TN>
+// SYM: odd primes through sums and differences of the pairs t[q], t[P - q]
+// (real factors only: 60 operations at P = 7 against 140 for the direct sum).
+template <int R, int DIR, int TN, bool SYM = false>
 struct RegDFT {
     static_assert(TN % R == 0, "twiddle table size must be a multiple of R");
     static constexpr int P = (R % 4 == 0 && R > 4) ? 4 : smallest_factor(R);  // radix 4 first
@@ -152,10 +154,47 @@ struct RegDFT {
             o[2] = csub(a0, b0);
             o[1] = cadd(a1, jb1);
             o[3] = csub(a1, jb1);
+        } else if constexpr (SYM) {
+            constexpr int H = (Pp - 1) / 2;
+            float2 a[H], b[H];
+            o[0] = t[0];
+#pragma unroll
+            for (int q = 0; q < H; ++q) {
+                a[q] = cadd(t[q + 1], t[Pp - 1 - q]);
+                b[q] = csub(t[q + 1], t[Pp - 1 - q]);
+                o[0] = cadd(o[0], a[q]);
+            }
+            sym_rows<Pp, 1>(t[0], a, b, o);
         } else {
 #pragma unroll
             for (int r = 0; r < Pp; ++r) o[r] = t[0];
             small_dft_acc<Pp, 1>(t, o, tw);
+        }
+    }
+    // outputs r and Pp - r of the symmetric form: c -+ i s with
+    // c = t0 + sum a_q cos(2 pi q r / P), s = sum b_q sin(2 pi q r / P)
+    template <int Pp, int Rr, int H>
+    __device__ __forceinline__ static void sym_rows(float2 t0, float2 (&a)[H], float2 (&b)[H], float2 (&o)[Pp])
+    {
+        if constexpr (Rr <= H) {
+            float2 c = t0, s = make_float2(0.f, 0.f);
+            sym_terms<Pp, Rr, 1>(a, b, c, s);
+            const float2 js = DIR > 0 ? make_float2(-s.y, s.x) : make_float2(s.y, -s.x);
+            o[Rr] = cadd(c, js);
+            o[Pp - Rr] = csub(c, js);
+            sym_rows<Pp, Rr + 1>(t0, a, b, o);
+        }
+    }
+    template <int Pp, int Rr, int Q, int H>
+    __device__ __forceinline__ static void sym_terms(float2 (&a)[H], float2 (&b)[H], float2& c, float2& s)
+    {
+        if constexpr (Q <= H) {
+            constexpr CxPair w = cx_cossin(Q * Rr, Pp);
+            constexpr float wc = (float)w.c, ws = (float)w.s;
+            c = make_float2(fmaf(a[Q - 1].x, wc, c.x), fmaf(a[Q - 1].y, wc, c.y));
+            s = Q == 1 ? make_float2(b[0].x * ws, b[0].y * ws)
+                       : make_float2(fmaf(b[Q - 1].x, ws, s.x), fmaf(b[Q - 1].y, ws, s.y));
+            sym_terms<Pp, Rr, Q + 1>(a, b, c, s);
         }
     }
     template <int Pp, int Q>
@@ -218,7 +257,7 @@ struct RegDFT {
 #pragma unroll
                 for (int t = 0; t < M; ++t) sub[q][t] = v[q + P * t];
 #pragma unroll
-            for (int q = 0; q < P; ++q) RegDFT<M, DIR, TN>::run(sub[q], tw);
+            for (int q = 0; q < P; ++q) RegDFT<M, DIR, TN, SYM>::run(sub[q], tw);
             combine<0>(sub, v, tw);
         }
     }

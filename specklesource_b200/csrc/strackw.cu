@@ -1,26 +1,34 @@
-// strackw.cu -- corrTrackFast (Strackw/corrTrackFast.c:89-231) on the GPU:
-// one CTA per grid point, per-CTA workspace in global memory staged through
-// shared-memory tiles.
+// strackw.cu -- corrTrackFast (Strackw/corrTrackFast.c:89-231) on the GPU.
 //
-// Per point (W = wRa = wAa, N = 2W, E = edgePad + NFAST/4):
-//  1. W x W raw patches of both images; estDopCarrier1 on them (:340);
-//  2. forward W x W DFTs, zeroPad with the azimuth roll (:718-761) and the
-//     N x N inverse, done as four W x W parity transforms per image; the
-//     intensity |z|^2 * scale is kept (float), as detectPatch takes it;
+// Grid points go through the kernels below in chunks; every kernel spreads the
+// lines (or rows) of all points of the chunk over the chip.  Per point
+// (W = wRa = waa, N = 2W, e = edgePad + NFAST/4, chip c2 = N - 4e, lags
+// L = 4e + 1):
+//  1. estDopCarrier1 on the raw windows (:340; window_batch.cuh);
+//  2. upsampling by two (:718-761).  The 2W x 2W zero-padded inverse is
+//     separable, its even samples are the window's own samples (times a phase
+//     in azimuth that the detection removes) and its odd samples the window
+//     shifted by half a sample: sw_cols makes the azimuth-shifted window
+//     (forward line, roll, half-sample phase, inverse line), sw_rows the range
+//     shift of the raw and of the shifted rows.  Six line passes instead of
+//     the eight that four parity transforms of a 2-D spectrum take, and only
+//     the intensities |z|^2 * scale leave the chip;
 //  3. detectPatch (:765-839): optional (2 navg + 1)^2 box sums in float in the
-//     reference's order and clamps (the small chip's azimuth clamp uses
-//     edgePadR, as in the reference), sqrt; the chip of image 2 is embedded in
-//     zeros, image 1 is the full search area;
-//  4. computeMeanSigma (:407-477): chip mean/variance and the search window's
-//     mean/variance at every one of the (4E+1)^2 placements, in double, from
-//     row and column prefix sums;
-//  5. ampMatchEdge (:903-947): one forward N x N DFT of (search + i chip), the
-//     Hermitian cross spectrum, one inverse; with both images' means removed
-//     first, the result is the covariance term of getPeakCorr directly
+//     reference's order and clamps (the chip's azimuth clamp uses edgePadR),
+//     range sums in sw_rows, azimuth sums and sqrt in sw_amps; the chip of
+//     image 2 is embedded in zeros, image 1 is the full search area;
+//  4. computeMeanSigma (:407-477): chip mean and variance from sw_amps' sums;
+//     the search window's at every one of the L^2 placements in sw_stats, in
+//     double: running column windows started from 16-row sums, then prefix
+//     sums along the row;
+//  5. ampMatchEdge (:903-947): one packed forward transform of
+//     (search + i chip), the Hermitian cross spectrum and the real inverse on
+//     half the columns (sw_fwd, sw_corr, sw_ncc); with both images' means
+//     removed first, the result is the covariance term of getPeakCorr directly
 //     (an exact identity that avoids the float cancellation of
 //     c*scaleW - meanR*meanS);
-//  6. getPeakCorr (:862-899): normalised correlation on the (4E+1)^2 lags,
-//     argmax inside the user radius (row-major first maximum);
+//  6. getPeakCorr (:862-899): normalised correlation on the lags, argmax
+//     inside the user radius (row-major first maximum) in sw_ncc / sw_peak;
 //  7. overSampleC (:951-990): the 21 x 21 block's symmetric zero pad to
 //     336 x 336 evaluated on the searched 64 x 64 window only, as B X B^T with
 //     the real kernel B[n][t] = 1 + 2 sum_{f=1..10} cos(2 pi f (n - 16 t)/336),
@@ -33,6 +41,7 @@
 
 #include "capi_internal.h"
 #include "strack_device.cuh"
+#include "window_batch.cuh"
 
 namespace sbk {
 
@@ -40,21 +49,39 @@ constexpr int W_NOVER = 16;  // corrTrackFast.c:11
 constexpr int W_NFAST = 20;  // corrTrackFast.c:12
 constexpr int W_N1 = W_NFAST + 1;
 constexpr int W_OSW = 64;    // searched window [168-32, 168+32)
+constexpr int W_SEG = 16;    // rows per partial column sum
+
+// What sw_reduce makes of sw_amps' sums.
+struct SwMoments {
+    double meanR, sigmaR, meanS;
+};
 
 struct SwArgs {
-    const void* img1;
-    const void* img2;
-    int nr1, na1, nr2, na2;
-    int sampleType, byteOrder;
-    const int4* plan;  // r1, a1, r2, a2 of the points to match
-    const int* list;   // grid index of each entry
-    int nList;
-    int eR, eA;        // edge pads including the internal +5
+    WinArgs win;      // the chunk's windows
+    const int* list;  // grid index of each point of the chunk
+    const int* az;    // Doppler roll of each point
+    int e;            // edge pad including the internal +5
     int navgR, navgA;
+    int taps;         // box half width when both axes share it (2, 3), -1: no box, 0: any
     float scale;
-    float2* scratch;
-    size_t perCta;     // float2 elements
-    const double* B;   // 64 x 21 oversampling kernel
+    const float2* twW;
+    const float2* twN;
+    const float2* tau;
+    // planes, one per point of the chunk
+    float2* xv;       // 2 x W x W: azimuth half-sample shift of both windows
+    float* H;         // 2 x N x N: intensities, range box sums
+    float2* Z;        // N x N row transforms (over H, which is spent by then)
+    float* A1;        // N x N search amplitudes
+    float* A2;        // c2 x c2 chip amplitudes
+    double* seg;      // N/16 x 2 x N: sums of A1 and A1^2 over 16 rows
+    double* part;     // N/16 x 3 partial sums of the moments
+    SwMoments* mom;
+    double* norm;     // L x L: scaleW / sqrt(sigmaR sigmaS)
+    float2* T;        // L x corr_ts(N)
+    double* ncc;      // L x L
+    double* bestV;    // per row-pair tile
+    int* bestE;
+    const double* B;  // 64 x 21 oversampling kernel
     float* offR;
     float* offA;
     float* corr;
@@ -100,470 +127,494 @@ __device__ __forceinline__ DArg block_argmax_d(DArg a, double* dsc, int* isc)
     return b;
 }
 
-__device__ __forceinline__ float2 sw_sample(const void* img, int nr, int na, int row, int col, int st, int bo)
-{
-    if (row < 0 || row >= na || col < 0 || col >= nr) return make_float2(0.f, 0.f);
-    return load_sample(img, nr, row, col, st, bo);
-}
-
 template <int W>
 struct SwCfg {
     static constexpr int N = 2 * W;
-    // 256 threads with three CTAs per SM from W = 96 to 192 (a third CTA
-    // beat 384 threads at two: 32.1 against 40.0 ms at W = 128, 76.4 against
-    // 79.2 at 192 on the 2000 x 4000 shear pair); 384 threads at two CTAs at
-    // 224 and 256 (114.3 against 116.9 ms at 224)
-    static constexpr int NT = W >= 224 ? 384 : 256;
-    static constexpr int TILE = sbfft::StagedTile<N, true>::elems > sbfft::StagedTile<W, true>::elems
-                                    ? sbfft::StagedTile<N, true>::elems
-                                    : sbfft::StagedTile<W, true>::elems;
-    static constexpr int TILEB = TILE;  // out-of-place tile of the three-step transforms
-    // oversampling kernel B (64 x 21), block X (21 x 21) and T (21 x 64), doubles
-    static constexpr int OSD = W_OSW * W_N1 + W_N1 * W_N1 + W_N1 * W_OSW;
-    // from W = 96 up they live in the (then idle) tiles, so that three CTAs fit an SM
-    static constexpr bool OS_IN_TILE = 2 * TILE >= OSD;
-    static constexpr size_t smem = sizeof(float2) * (TILE + TILEB + W + N + W) +
-                                   (OS_IN_TILE ? 0 : sizeof(double) * OSD) + sizeof(double) * (NT / 32 + 1) * 8 +
-                                   sizeof(int) * (3 * (NT / 32) + 8) + 64;
-    // CTAs per SM (228 KB of shared memory, 1 KB reserved per CTA)
-    static constexpr int CTAS = W >= 96 && W <= 192 && OS_IN_TILE && 3 * (smem + 1024) <= 228 * 1024 ? 3 : 2;
-    static_assert((NT / 32) * 2 * N <= W * W, "per-warp prefix slices must fit in `work`");
-    // workspace (float2 units): F1, F2, work (W^2 each), I1, I2 (N^2 floats
-    // each), z (N^2), row sums RS1, RS2 (N x L doubles each), meanS, sigmaS,
-    // ncc (L^2 doubles each) with L = 4E + 1, then H1, H2 (N^2 floats each)
-    static size_t perCta(int L)
-    {
-        return (size_t)3 * W * W + (size_t)N * N + (size_t)N * N + (size_t)2 * N * L + (size_t)3 * L * L +
-               (size_t)N * N + 64;
-    }
+    static constexpr int G = 8;                    // lines per CTA of sw_cols, sw_rows, sw_fwd, sw_ncc
+    static constexpr int NTW = 128;                // threads for lines of W points
+    static constexpr int NTN = 128;                // threads for lines of N points
+    using CW = sbfft::LineTile<W, G, false>;
+    using RW = sbfft::LineTile<W, G, true>;
+    using RN = sbfft::LineTile<N, G, true>;
+    static_assert(G * 16 <= NTW, "lines of W points: one item a thread and step");
+    static constexpr size_t smCols = sizeof(float2) * CW::elems;
+    static constexpr size_t smRows = sizeof(float2) * RW::elems;  // and the intensities
+    static constexpr size_t smFwd = sizeof(float2) * RN::elems;
+    static constexpr size_t smNcc = smFwd + sizeof(double) * (NTN / 32) + sizeof(int) * (NTN / 32);
+    static constexpr int NTS = N <= 256 ? N : N / 2;  // sw_stats: one or two columns a thread
+    static constexpr int CL = N / 32;              // columns per lane of its prefix sums
+    static constexpr int PS = N + 32;              // padded prefix row
+    static constexpr size_t smStats = sizeof(double) * 8 * PS;
 };
 
-template <int W>
-__global__ void __launch_bounds__(SwCfg<W>::NT, SwCfg<W>::CTAS) strackw_kernel(SwArgs a)
+// Azimuth half-sample shift of columns c0 .. c0+7 of one window: forward line,
+// X'[k] = F[(k + roll) mod W] tau[k], inverse line.
+template <int W, bool F32>
+__global__ void __launch_bounds__(128) sw_cols_kernel(SwArgs a)
 {
     using C = SwCfg<W>;
-    constexpr int N = C::N, NT = C::NT;
+    constexpr int G = C::G, NT = C::NTW, TILES = W / G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* tile = reinterpret_cast<float2*>(smem_raw);
-    float2* tileB = tile + C::TILE;
-    float2* twW = tileB + C::TILEB;
-    float2* twN = twW + W;
-    float2* tau = twN + N;
-    double* osBase = C::OS_IN_TILE ? reinterpret_cast<double*>(tile) : reinterpret_cast<double*>(tau + W);
-    double* Bm = osBase;                                    // 64 x 21
-    double* X = Bm + W_OSW * W_N1;                          // 21 x 21 block
-    double* T = X + W_N1 * W_N1;                            // 21 x 64
-    double* red = C::OS_IN_TILE ? reinterpret_cast<double*>(tau + W) : T + W_N1 * W_OSW;
-    int* isc = reinterpret_cast<int*>(red + (NT / 32 + 1) * 8);
-    const int tid = threadIdx.x;
-
-    for (int e = tid; e < W; e += NT) {
-        double s, c;
-        sincospi(-2.0 * e / W, &s, &c);
-        twW[e] = make_float2((float)c, (float)s);
-        sincospi((double)e / W, &s, &c);
-        const double sg = e < W / 2 ? 1.0 : -1.0;
-        tau[e] = make_float2((float)(sg * c), (float)(sg * s));
-    }
-    for (int e = tid; e < N; e += NT) {
-        double s, c;
-        sincospi(-2.0 * e / N, &s, &c);
-        twN[e] = make_float2((float)c, (float)s);
-    }
-    if constexpr (!C::OS_IN_TILE)
-        for (int e = tid; e < W_OSW * W_N1; e += NT) Bm[e] = a.B[e];
+    float2* s = reinterpret_cast<float2*>(smem_raw);
+    const int tile = blockIdx.x % TILES, q = blockIdx.x / TILES % 2, pt = blockIdx.x / (2 * TILES);
+    const Window<F32> win(a.win, q, a.win.win[pt], W);
+    const int c0 = tile * G;
+    int da = a.az[pt];
+    if (da < 0 || da >= W) da = 0;
+    sbfft::line_fft<W, -1, G, NT, false, false, true>(
+        s, a.twW, [&](int l, int k) { return win(k, c0 + l); },
+        [&](int l, int k, float2 v) {
+            const int r = k - da < 0 ? k - da + W : k - da;
+            s[r * G + l] = sbfft::cmul(v, __ldg(a.tau + r));
+        });
     __syncthreads();
+    float2* out = a.xv + ((size_t)pt * 2 + q) * W * W + c0;
+    sbfft::line_fft<W, 1, G, NT, false, true, false>(
+        s, a.twW, [&](int l, int k) { return s[k * G + l]; },
+        [&](int l, int k, float2 v) { out[k * W + l] = v; });
+}
 
-    const int eR = a.eR, eA = a.eA;
-    const int L = 4 * eR + 1, LA = 4 * eA + 1;  // lags (range, azimuth)
-    const int wR2 = (W - 2 * eR) * OS, wA2 = (W - 2 * eA) * OS;
-    float2* F1 = a.scratch + (size_t)blockIdx.x * a.perCta;
-    float2* F2 = F1 + W * W;
-    float2* work = F2 + W * W;
-    float* I1 = reinterpret_cast<float*>(work + W * W);
-    float* I2 = I1 + (size_t)N * N;
-    float2* z = reinterpret_cast<float2*>(I2 + (size_t)N * N);
-    double* RS1 = reinterpret_cast<double*>(z + (size_t)N * N);
-    double* RS2 = RS1 + (size_t)N * L;
-    double* meanS = RS2 + (size_t)N * L;
-    double* sigmaS = meanS + (size_t)LA * L;
-    double* ncc = sigmaS + (size_t)LA * L;
-    float* H1 = reinterpret_cast<float*>(ncc + (size_t)LA * L);
-    float* H2 = H1 + (size_t)N * N;
-    const bool smooth = a.navgA > 1 || a.navgR > 1;
+// Rows j of the doubled window (even: the raw window's, odd: the shifted
+// one's): range half-sample shift, intensities of the N samples, range box
+// sums.  Rows [0, N) of image 1; of image 2 those whose box sums the chip
+// reads.  The intensity rows carry `pad` copies of their end values on both
+// sides, so that the sums need no clamps (the chip's own clamps, kmax and lmax
+// of detectPatch, never bind inside the N x N area).
+template <int W, bool F32>
+__global__ void __launch_bounds__(128) sw_rows_kernel(SwArgs a, int hr0, int hr1, int pad)
+{
+    using C = SwCfg<W>;
+    constexpr int N = C::N, G = C::G, NT = C::NTW, TILES = N / G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* s = reinterpret_cast<float2*>(smem_raw);
+    float* in = reinterpret_cast<float*>(s + C::RW::elems) + pad;
+    const int PR = N + 2 * pad;  // intensity row
+    const int tiles2 = (hr1 - hr0 + G) / G, per = TILES + tiles2;
+    const int pt = blockIdx.x / per, b = blockIdx.x % per;
+    const int q = b >= TILES;
+    const int j0 = q ? hr0 + (b - TILES) * G : b * G;
+    const Window<F32> win(a.win, q, a.win.win[pt], W);
+    const float2* xv = a.xv + ((size_t)pt * 2 + q) * W * W;
+    // every line pass is unnormalised (a factor W an axis, W^4 in intensity)
+    const float s0 = a.scale * ((float)W * W * W * W), s1 = a.scale * ((float)W * W);
+    // lines 0 .. 3 are the raw rows of the tile and 4 .. 7 the shifted ones
+    // (j0 is even), so that a warp loads from one of the two
+    auto row = [](int l) { return l < G / 2 ? 2 * l : 2 * l - G + 1; };
+    sbfft::line_fft<W, -1, G, NT, true, false, true>(
+        s, a.twW,
+        [&](int l, int k) {
+            const int i = min((j0 >> 1) + (l & (G / 2 - 1)), W - 1);
+            return l < G / 2 ? win(i, k) : xv[i * W + k];
+        },
+        [&](int l, int k, float2 v) { s[l * C::RW::L + k] = sbfft::cmul(v, __ldg(a.tau + k)); },
+        [&](int l, int k, float2 v) {
+            in[row(l) * PR + 2 * k] = (v.x * v.x + v.y * v.y) * (l < G / 2 ? s0 : s1);
+        });
+    __syncthreads();
+    sbfft::line_fft<W, 1, G, NT, true, true, false>(
+        s, a.twW, [&](int l, int k) { return s[l * C::RW::L + k]; },
+        [&](int l, int k, float2 v) {
+            in[row(l) * PR + 2 * k + 1] = (v.x * v.x + v.y * v.y) * (l < G / 2 ? s1 : a.scale);
+        });
+    __syncthreads();
+    if (pad) {
+        for (int e = threadIdx.x; e < 2 * G * pad; e += NT) {
+            const int l = e % G, m = e / G;
+            if (m < pad) in[l * PR - 1 - m] = in[l * PR];
+            else in[l * PR + N + m - pad] = in[l * PR + N - 1];
+        }
+        __syncthreads();
+    }
+    float* H = a.H + ((size_t)pt * 2 + q) * N * N;
+    const int c0 = q ? 2 * a.e : 0, c1 = q ? N - 2 * a.e : N;  // image 2: the chip's columns
+    const int rows = q ? min(G, hr1 - j0 + 1) : G;
+    const int lane = threadIdx.x & 31;
+    for (int l = threadIdx.x >> 5; l < rows; l += NT / 32) {
+        const float* p = in + l * PR;
+        float* h = H + (size_t)(j0 + l) * N;
+        if (a.taps == 2) {
+            for (int j = c0 + lane; j < c1; j += 32) h[j] = p[j - 2] + p[j - 1] + p[j] + p[j + 1] + p[j + 2];
+        } else if (a.taps < 0) {
+            for (int j = c0 + lane; j < c1; j += 32) h[j] = p[j];
+        } else {
+            for (int j = c0 + lane; j < c1; j += 32) {
+                float t = 0.f;
+                for (int m = -a.navgR; m <= a.navgR; m++) t += p[min(max(j + m, -pad), N - 1 + pad)];
+                h[j] = t;
+            }
+        }
+    }
+}
 
-    for (int it = blockIdx.x; it < a.nList; it += gridDim.x) {
-        const int4 pl = a.plan[it];  // r1, a1, r2, a2
-        // ------------------------------------------------ patches, Doppler
-        double m[4] = {0, 0, 0, 0};
-        for (int e = tid; e < W * W; e += NT) {
-            const int i = e / W, j = e % W;
-            const float2 z1 = sw_sample(a.img1, a.nr1, a.na1, pl.y + i, pl.x + j, a.sampleType, a.byteOrder);
-            const float2 z2 = sw_sample(a.img2, a.nr2, a.na2, pl.w + i, pl.z + j, a.sampleType, a.byteOrder);
-            F1[e] = z1;
-            F2[e] = z2;
-            m[0] += z1.x; m[1] += z1.y; m[2] += z2.x; m[3] += z2.y;
-        }
-        block_allsum<4, NT>(m, red);
-        {
-            const double n = (double)(W * W);
-            const double m1r = m[0] / n, m1i = m[1] / n, m2r = m[2] / n, m2i = m[3] / n;
-            double d[4] = {0, 0, 0, 0};
-            for (int e = tid; e < (W - 1) * W; e += NT) {
-                const float2 p0 = F1[e], p1 = F1[e + W];
-                double ar = (double)p1.x - m1r, ai = (double)p1.y - m1i, br = (double)p0.x - m1r,
-                       bi = (double)p0.y - m1i;
-                d[0] += ar * br + ai * bi;
-                d[1] += ai * br - ar * bi;
-                const float2 q0 = F2[e], q1 = F2[e + W];
-                ar = (double)q1.x - m2r; ai = (double)q1.y - m2i; br = (double)q0.x - m2r; bi = (double)q0.y - m2i;
-                d[2] += ar * br + ai * bi;
-                d[3] += ai * br - ar * bi;
-            }
-            block_allsum<4, NT>(d, red);
-            m[0] = (double)dop_shift(d[0], d[1], d[2], d[3], W, W);
-        }
-        int da = (int)m[0];
-        if (da < 0 || da >= W) da = 0;
-        sbfft::fft2d_staged<W, -1, NT, true>(F1, tile, twW, tileB);
-        sbfft::fft2d_staged<W, -1, NT, true>(F2, tile, twW, tileB);
-        // ------------------------------------------------ upsampled intensities
-        // The 2W x 2W padded inverse as four parity transforms
-        // c_e[m1][m2] = IDFT_W(X' tau_e1[k1] tau_e2[k2]), X'[k1] = F[(k1 + da) mod W]:
-        // the row factor tau_e1 and the row roll commute with the row
-        // transform, so two unrolled row passes (R0 = rows of F, R1 = rows of
-        // F tau) serve the four parities, and each column pass reads its R with
-        // the roll and tau_e1 folded into the gather and writes |c|^2 * scale
-        // straight into the intensity plane.
-        // intensity columns of image 2 that detectPatch reads: the chip
-        // [eR OS, eR OS + wR2) widened by the range box sum (navgR) and one
-        // column of slack, as parity-plane columns
-        constexpr int GW = sbfft::StagedTile<W, true>::G;
-        const int cLo = max(0, eR * OS - a.navgR - 1) / 2;
-        const int cHi = min(N - 1, eR * OS + wR2 + a.navgR) / 2;
-#pragma unroll 1
-        for (int q = 0; q < 2; ++q) {
-            float2* F = q == 0 ? F1 : F2;
-            float* I = q == 0 ? I1 : I2;
-            const float sc = a.scale;
-            sbfft::staged_rows<W, 1, NT, true>(
-                work, [F](int r, int k) { return F[(size_t)r * W + k]; }, tile, tileB, twW);
-            sbfft::staged_rows<W, 1, NT, true>(
-                F, [F, tau](int r, int k) { return sbfft::cmul(F[(size_t)r * W + k], tau[k]); }, tile, tileB, twW);
-#pragma unroll 1
-            for (int par = 0; par < 4; ++par) {
-                const int e1 = par >> 1, e2 = par & 1;
-                const float2* R = e2 ? F : work;
-                auto src = [R, tau, da, e1](int k, int c) {
-                    int r = k + da;
-                    r = r >= W ? r - W : r;
-                    const float2 v = R[(size_t)r * W + c];
-                    return e1 ? sbfft::cmul(v, tau[k]) : v;
-                };
-                auto dst = [I, sc, e1, e2](int k, int c, float2 v) {
-                    I[(size_t)(2 * k + e1) * N + 2 * c + e2] = (v.x * v.x + v.y * v.y) * sc;
-                };
-                // the chip (image 2) reads only the intensity columns of the
-                // chip and its box-sum margin: column c of a parity plane
-                // lands in intensity columns 2c and 2c + 1, so tiles of c
-                // outside [cLo, cHi] are skipped (image 1: every column)
-                sbfft::staged_cols_if<W, 1, NT, true>(
-                    src, dst, [q, cLo, cHi](int c0) { return q == 0 || (c0 + GW - 1 >= cLo && c0 <= cHi); }, tile,
-                    tileB, twW);
-            }
-        }
-        // ------------------------------------------------ detectPatch
-        // The (2 navg + 1)^2 box sums are separable: range sums into H1/H2
-        // first, then azimuth sums of those, with the reference's clamps
-        // (image 1: the N x N area; the chip: kmax/lmax, the azimuth limit
-        // built from edgePadR as at :795).
-        const int kmax = eR * OS + wA2 + a.navgA - 1;
-        const int lmax = eR * OS + wR2 + a.navgR - 1;
-        if (smooth) {
-            // the chip's azimuth sums read H2 only on rows clamp(i + m, 0,
-            // kmax) of the chip rows i and on the chip columns: H2 is formed
-            // there (one row and column of slack), H1 everywhere
-            const int hr0 = max(0, min(kmax, eA * OS - a.navgA) - 1);
-            const int hr1 = min(N - 1, min(kmax, eA * OS + wA2 - 1 + a.navgA) + 1);
-            const int hc0 = max(0, eR * OS - 1), hc1 = min(N - 1, eR * OS + wR2);
-            for (int e = tid; e < N * N; e += NT) {
-                const int i = e / N, j = e % N;
-                const bool need2 = i >= hr0 && i <= hr1 && j >= hc0 && j <= hc1;
-                float h1 = 0.f, h2 = 0.f;
-                for (int nn = -a.navgR; nn <= a.navgR; nn++) {
-                    int l = j + nn;
-                    l = l > 0 ? l : 0;
-                    const int l1 = l < N - 1 ? l : N - 1;
-                    const int l2 = l < lmax ? l : lmax;
-                    h1 += I1[(size_t)i * N + l1];
-                    if (need2) h2 += I2[(size_t)i * N + l2];
-                }
-                H1[e] = h1;
-                if (need2) H2[e] = h2;
-            }
-            __syncthreads();
-        }
-        double cs[3] = {0, 0, 0};
-        for (int e = tid; e < N * N; e += NT) {
-            const int i = e / N, j = e % N;
-            // large patch (image 1): edge pads 0, clamps to the N x N area
-            float v1;
-            if (smooth) {
-                float acc = 0.f;
-                for (int mm = -a.navgA; mm <= a.navgA; mm++) {
-                    int k = i + mm;
-                    k = k > 0 ? k : 0;
-                    k = k < N - 1 ? k : N - 1;
-                    acc += H1[(size_t)k * N + j];
-                }
-                v1 = acc;
-            } else {
-                v1 = I1[e];
-            }
-            // small chip (image 2) embedded in zeros
-            float v2 = 0.f;
-            const int ci = i - eA * OS, cj = j - eR * OS;
-            if (ci >= 0 && ci < wA2 && cj >= 0 && cj < wR2) {
-                if (smooth) {
-                    float acc = 0.f;
-                    for (int mm = -a.navgA; mm <= a.navgA; mm++) {
-                        int k = i + mm;
-                        k = k > 0 ? k : 0;
-                        k = k < kmax ? k : kmax;
-                        acc += H2[(size_t)k * N + j];
-                    }
-                    v2 = acc;
-                } else {
-                    v2 = I2[e];
-                }
-                v2 = sqrtf(v2);
-                cs[0] += v2;
-                cs[1] += (double)(v2 * v2);
-            }
-            v1 = sqrtf(v1);
-            cs[2] += v1;
-            z[e] = make_float2(v1, v2);
-        }
-        block_allsum<3, NT>(cs, red);
-        const double nchip = (double)(wR2 * wA2);
-        const double meanR = cs[0] / nchip;
-        const double sigmaR = cs[1] / (double)(wR2 * wA2 - 1.) - meanR * meanR;
-        // ------------------------------------------------ search-window statistics
-        // RS[l][s1] = sum_{s = s1 .. s1 + wR2 - 1} A1[l][s] (and of A1^2), one warp per row
-        {
-            const int lane = tid & 31, warp = tid >> 5;
-            double* Pw = reinterpret_cast<double*>(work) + (size_t)warp * 2 * N;  // 16 N bytes per warp
-            for (int row = warp; row < N; row += NT / 32) {
-                double c1 = 0, c2 = 0;  // running carry of the prefix scan
-                // prefix sums computed in chunks of 32 columns
-                for (int base = 0; base < N; base += 32) {
-                    const int s = base + lane;
-                    const float x = z[(size_t)row * N + s].x;
-                    double p1 = x, p2 = (double)(x * x);
+// Azimuth box sums and amplitudes, a thread per column and 16 rows a CTA; the
+// sums that the moments and sw_stats start from.  TAPS: the half width of the
+// box (-1: none), so that a thread loads each row once and adds from
+// registers; 0: any, as separate loads.
+template <int W, int TAPS>
+__global__ void __launch_bounds__(2 * W) sw_amps_kernel(SwArgs a)
+{
+    constexpr int N = 2 * W, NT = N;
+    __shared__ double red[(NT / 32 + 1) * 3];
+    const int pt = blockIdx.x / (N / W_SEG), sg = blockIdx.x % (N / W_SEG), j = threadIdx.x;
+    const int e2 = 2 * a.e, c2 = N - 2 * e2;
+    const float* H1 = a.H + (size_t)pt * 2 * N * N + j;
+    const float* H2 = H1 + (size_t)N * N;
+    float* A1 = a.A1 + (size_t)pt * N * N + j;
+    float* A2 = a.A2 + (size_t)pt * c2 * c2 + (j - e2);
+    double cs[3] = {0, 0, 0}, q1 = 0, q2 = 0;
+    const bool col = j >= e2 && j < e2 + c2;
+    const int i0 = sg * W_SEG;
+    // amplitudes of 16 rows of one plane
+    auto rows = [&](const float* H, float (&v)[W_SEG]) {
+        if constexpr (TAPS < 0) {
 #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const double t1 = __shfl_up_sync(0xffffffffu, p1, o);
-                        const double t2 = __shfl_up_sync(0xffffffffu, p2, o);
-                        if (lane >= o) {
-                            p1 += t1;
-                            p2 += t2;
-                        }
-                    }
-                    p1 += c1;
-                    p2 += c2;
-                    Pw[2 * s] = p1;  // inclusive prefix, this warp's slice of `work`
-                    Pw[2 * s + 1] = p2;
-                    c1 = __shfl_sync(0xffffffffu, p1, 31);
-                    c2 = __shfl_sync(0xffffffffu, p2, 31);
-                }
-                __syncwarp();
-                for (int s1 = lane; s1 < L; s1 += 32) {
-                    const double* P = Pw;
-                    const int hi = s1 + wR2 - 1;
-                    const double a1 = P[2 * hi] - (s1 > 0 ? P[2 * (s1 - 1)] : 0.0);
-                    const double a2 = P[2 * hi + 1] - (s1 > 0 ? P[2 * (s1 - 1) + 1] : 0.0);
-                    RS1[(size_t)row * L + s1] = a1;
-                    RS2[(size_t)row * L + s1] = a2;
-                }
-                __syncwarp();
+            for (int r = 0; r < W_SEG; ++r) v[r] = H[(i0 + r) * N];
+        } else if constexpr (TAPS > 0) {
+            float h[W_SEG + 2 * TAPS];
+#pragma unroll
+            for (int r = 0; r < W_SEG + 2 * TAPS; ++r) h[r] = H[min(max(i0 + r - TAPS, 0), N - 1) * N];
+#pragma unroll
+            for (int r = 0; r < W_SEG; ++r) {
+                v[r] = h[r];
+#pragma unroll
+                for (int m = 1; m <= 2 * TAPS; ++m) v[r] += h[r + m];
             }
-            __syncthreads();
+        } else {
+            for (int r = 0; r < W_SEG; ++r) {
+                v[r] = 0.f;
+                for (int m = -a.navgA; m <= a.navgA; m++) v[r] += H[min(max(i0 + r + m, 0), N - 1) * N];
+            }
         }
-        // column prefix sums of the row-window sums (one thread per lag column;
-        // rows unrolled so the loads run ahead of the dependent adds), then the
-        // wA2-row window of every placement as a difference of two prefixes
+    };
+    float v[W_SEG];
+    rows(H1, v);
+#pragma unroll
+    for (int r = 0; r < W_SEG; ++r) {
+        const float x = sqrtf(v[r]);
+        A1[(i0 + r) * N] = x;
+        q1 += x;
+        q2 += (double)(x * x);
+    }
+    if (col && i0 + W_SEG > e2 && i0 < e2 + c2) {
+        rows(H2, v);
+#pragma unroll
+        for (int r = 0; r < W_SEG; ++r) {
+            const int ci = i0 + r - e2;
+            if (ci >= 0 && ci < c2) {
+                const float x = sqrtf(v[r]);
+                A2[ci * c2] = x;
+                cs[0] += x;
+                cs[1] += (double)(x * x);
+            }
+        }
+    }
+    double* seg = a.seg + ((size_t)pt * (N / W_SEG) + sg) * 2 * N;
+    seg[j] = q1;
+    seg[N + j] = q2;
+    cs[2] = q1;
+    block_allsum<3, NT>(cs, red);
+    if (j == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a.part[(size_t)blockIdx.x * 3 + k] = cs[k];
+}
+
+// Moments of a point (a warp each).
+template <int W>
+__global__ void sw_reduce_kernel(SwArgs a)
+{
+    constexpr int N = 2 * W, NS = N / W_SEG;
+    const int pt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (pt >= a.win.n) return;
+    double cs[3] = {0, 0, 0};
+    if (lane < NS)
+        for (int k = 0; k < 3; ++k) cs[k] = a.part[((size_t)pt * NS + lane) * 3 + k];
+    for (int k = 0; k < 3; ++k) cs[k] = warp_allsum(cs[k]);
+    if (lane == 0) {
+        const int c2 = N - 4 * a.e;
+        const double nchip = (double)(c2 * c2);
+        SwMoments m;
+        m.meanR = cs[0] / nchip;
+        m.sigmaR = cs[1] / (nchip - 1.) - m.meanR * m.meanR;
+        m.meanS = cs[2] / ((double)N * N);
+        a.mom[pt] = m;
+    }
+}
+
+// scaleW / sqrt(sigmaR sigmaS) of 16 lag rows a CTA.  A thread keeps the c2-row
+// window sums of its columns of A1 and A1^2, started from the 16-row sums and
+// moved down a row at a time; four rows of both go to shared memory, where a
+// warp each turns them into prefix sums, and the L windows along the row are
+// differences of two prefixes.
+template <int W>
+__global__ void __launch_bounds__(SwCfg<W>::NTS) sw_stats_kernel(SwArgs a)
+{
+    using C = SwCfg<W>;
+    constexpr int N = C::N, NT = C::NTS, CPT = N / NT, CL = C::CL, PS = C::PS, NW = NT / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* P = reinterpret_cast<double*>(smem_raw);  // 4 rows x 2 sums, PS each; column s at s + s / CL
+    const int L = 4 * a.e + 1, c2 = N - 4 * a.e, tiles = (L + W_SEG - 1) / W_SEG;
+    const int pt = blockIdx.x / tiles, tile = blockIdx.x % tiles;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const float* A1 = a.A1 + (size_t)pt * N * N;
+    const SwMoments mom = a.mom[pt];
+    const double nchip = (double)(c2 * c2);
+    const double inv0 = 1.0 / nchip, inv1 = 1.0 / (nchip - 1);
+    const double wp = W - 2 * a.e;
+    const double scaleW = 1.0 / ((OS * OS * OS * OS) * W * wp * W * wp);
+    const int l0 = tile * W_SEG, lEnd = min(L, l0 + W_SEG);
+    double v1[CPT], v2[CPT];
+#pragma unroll
+    for (int u = 0; u < CPT; ++u) {
+        const int s = tid + u * NT;
+        const double* seg = a.seg + ((size_t)pt * (N / W_SEG) + tile) * 2 * N;
+        double t1 = 0, t2 = 0;
+        for (int g = 0; g < c2 / W_SEG; ++g) {
+            t1 += seg[(size_t)g * 2 * N + s];
+            t2 += seg[(size_t)g * 2 * N + N + s];
+        }
+        for (int r = l0 + c2 / W_SEG * W_SEG; r < l0 + c2; ++r) {
+            const float x = A1[(size_t)r * N + s];
+            t1 += x;
+            t2 += (double)(x * x);
+        }
+        v1[u] = t1;
+        v2[u] = t2;
+    }
+    for (int lb = l0; lb < lEnd; lb += 4) {
+        const int nr = min(4, lEnd - lb);
+        float in[CPT][4], out[CPT][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int u = 0; u < CPT; ++u) {
+                const bool more = lb + r + 1 < lEnd;
+                in[u][r] = more ? A1[(size_t)(lb + r + c2) * N + tid + u * NT] : 0.f;
+                out[u][r] = more ? A1[(size_t)(lb + r) * N + tid + u * NT] : 0.f;
+            }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int u = 0; u < CPT; ++u) {
+                const int s = tid + u * NT;
+                P[(2 * r) * PS + s + s / CL] = v1[u];
+                P[(2 * r + 1) * PS + s + s / CL] = v2[u];
+                v1[u] += (double)in[u][r] - (double)out[u][r];
+                v2[u] += (double)(in[u][r] * in[u][r]) - (double)(out[u][r] * out[u][r]);
+            }
+        __syncthreads();
+        for (int row = warp; row < 2 * nr; row += NW) {  // inclusive prefix sums
+            double* p = P + row * PS + lane * (CL + 1);
+            double t = 0, x[CL];
+#pragma unroll
+            for (int c = 0; c < CL; ++c) {
+                t += p[c];
+                x[c] = t;
+            }
+            double sc = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const double y = __shfl_up_sync(0xffffffffu, sc, o);
+                if (lane >= o) sc += y;
+            }
+            sc -= t;
+#pragma unroll
+            for (int c = 0; c < CL; ++c) p[c] = x[c] + sc;
+        }
+        __syncthreads();
+        for (int r = 0; r < nr; ++r)
         for (int s1 = tid; s1 < L; s1 += NT) {
-            double c1 = 0.0, c2 = 0.0;
-            int l = 0;
-            for (; l + 8 <= N; l += 8) {
-                double v1[8], v2[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    v1[u] = RS1[(size_t)(l + u) * L + s1];
-                    v2[u] = RS2[(size_t)(l + u) * L + s1];
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    c1 += v1[u];
-                    c2 += v2[u];
-                    RS1[(size_t)(l + u) * L + s1] = c1;
-                    RS2[(size_t)(l + u) * L + s1] = c2;
-                }
+            const int hi = s1 + c2 - 1;
+            const double* p = P + 2 * r * PS;
+            double a1 = p[hi + hi / CL], a2 = p[PS + hi + hi / CL];
+            if (s1 > 0) {
+                a1 -= p[s1 - 1 + (s1 - 1) / CL];
+                a2 -= p[PS + s1 - 1 + (s1 - 1) / CL];
             }
-            for (; l < N; ++l) {
-                c1 += RS1[(size_t)l * L + s1];
-                c2 += RS2[(size_t)l * L + s1];
-                RS1[(size_t)l * L + s1] = c1;
-                RS2[(size_t)l * L + s1] = c2;
-            }
+            const double ms = a1 * inv0;
+            const double sg = a2 * inv1 - ms * ms;
+            a.norm[((size_t)pt * L + lb + r) * L + s1] = scaleW * rsqrt(mom.sigmaR * sg);
         }
         __syncthreads();
-        for (int e = tid; e < LA * L; e += NT) {
-            const int l1 = e / L, s1 = e % L;
-            const size_t hi = (size_t)(l1 + wA2 - 1) * L + s1, lo = (size_t)(l1 - 1) * L + s1;
-            const double a1 = RS1[hi] - (l1 > 0 ? RS1[lo] : 0.0);
-            const double a2 = RS2[hi] - (l1 > 0 ? RS2[lo] : 0.0);
-            const double ms = a1 / nchip;
-            meanS[e] = ms;
-            sigmaS[e] = a2 / (double)(wR2 * wA2 - 1) - ms * ms;
-        }
-        __syncthreads();
-        // ------------------------------------------------ correlation
-        // getPeakCorr forms c*scaleW - meanR*meanS with c the correlation of
-        // the raw amplitudes; both terms are ~mean^2 and their difference is
-        // the covariance.  Correlating the chip minus its mean (on its
-        // support) with the search image minus its global mean gives that
-        // difference directly, because sum(chip - meanR) = 0 over the support:
-        //   sum_x (chip[x] - meanR)(A1[x+t] - mA1) = c[t] - meanR * n * meanS[t].
-        // Same quantity, without the float cancellation.
-        // The mean removal is folded into the forward row pass; the Hermitian
-        // split of the packed pair and the cross spectrum into the inverse row
-        // pass, which reads Z[k] and Z[-k] and writes out of place into the
-        // free H1/H2 area (Zi); the last column pass keeps only the lag rows
-        // and columns getPeakCorr reads.
-        {
-            const float mA1 = (float)(cs[2] / ((double)N * N));
-            const float mR = (float)meanR;
-            const int cA = eA * OS, cR = eR * OS;
-            auto srcFwd = [z, mA1, mR, cA, cR, wA2, wR2](int r, int k) {
-                float2 v = z[(size_t)r * N + k];
-                const int ci = r - cA, cj = k - cR;
-                const bool in = ci >= 0 && ci < wA2 && cj >= 0 && cj < wR2;
-                v.x -= mA1;
-                v.y = in ? v.y - mR : 0.f;
-                return v;
-            };
-            sbfft::staged_rows<N, -1, NT, true>(z, srcFwd, tile, tileB, twN);
-            sbfft::staged_cols<N, -1, NT, true>([z](int k, int c) { return z[(size_t)k * N + c]; },
-                                                [z](int k, int c, float2 v) { z[(size_t)k * N + c] = v; }, tile,
-                                                tileB, twN);
-        }
-        float2* Zi = reinterpret_cast<float2*>(H1);
-        {
-            auto srcInv = [z](int r, int k) {
-                const float2 Zk = z[(size_t)r * N + k];
-                const float2 Zm = z[(size_t)(r == 0 ? 0 : N - r) * N + (k == 0 ? 0 : N - k)];
-                const float2 f1 = make_float2(0.5f * (Zk.x + Zm.x), 0.5f * (Zk.y - Zm.y));
-                const float2 f2 = make_float2(0.5f * (Zk.y + Zm.y), -0.5f * (Zk.x - Zm.x));
-                return sbfft::cconjmul(f1, f2);
-            };
-            sbfft::staged_rows<N, 1, NT, true>(Zi, srcInv, tile, tileB, twN);
-            const int nLo = LA - OS * eA, nHi = N - OS * eA;  // lag rows/cols used: [0, nLo) and [nHi, N)
-            auto need = [nLo, nHi](int x) { return x < nLo || x >= nHi; };
-            // tiles of columns that hold no lag are not transformed
-            constexpr int GN = sbfft::StagedTile<N, true>::G;
-            sbfft::staged_cols_if<N, 1, NT, true>([Zi](int k, int c) { return Zi[(size_t)k * N + c]; },
-                                                  [Zi, need](int k, int c, float2 v) {
-                                                      if (need(k) && need(c)) Zi[(size_t)k * N + c] = v;
-                                                  },
-                                                  [nLo, nHi](int c0) { return c0 < nLo || c0 + GN - 1 >= nHi; },
-                                                  tile, tileB, twN);
-        }
-        // ------------------------------------------------ getPeakCorr
-        const double wR2p = W - 2 * eR, wA2p = W - 2 * eA;
-        const double scaleW = 1.0 / ((OS * OS * OS * OS) * W * wA2p * W * wR2p);
-        const int lim = OS * (eA - W_NFAST / 4), limR = OS * (eR - W_NFAST / 4);
-        DArg best;
-        best.v = -1e30;
-        best.rank = 0x7fffffff;
-        for (int e = tid; e < LA * L; e += NT) {
-            const int i = e / L, j = e % L;
-            const int l = i - OS * eA, s = j - OS * eR;
-            const int cy = l < 0 ? l + N : l, cx = s < 0 ? s + N : s;
-            const float2 c = Zi[(size_t)cy * N + cx];
-            double v = (double)c.x * scaleW;  // = |c| * scaleW - meanR * meanS (the covariance)
-            v = v / sqrt(sigmaR * sigmaS[e]);
-            ncc[e] = v;
-            if (l >= -lim && s >= -limR && l <= lim && s <= limR && darg_better(v, e, best.v, best.rank)) {
-                best.v = v;
-                best.rank = e;
+    }
+}
+
+// Row transforms of (search - mean) + i (chip - mean, zeros around it).
+// getPeakCorr forms c*scaleW - meanR*meanS with c the correlation of the raw
+// amplitudes; both terms are ~mean^2 and their difference is the covariance.
+// Correlating the chip minus its mean (on its support) with the search image
+// minus any constant gives that difference directly, because
+// sum(chip - meanR) = 0 over the support.
+template <int W>
+__global__ void __launch_bounds__(SwCfg<W>::NTN) sw_fwd_kernel(SwArgs a)
+{
+    using C = SwCfg<W>;
+    constexpr int N = C::N, G = C::G, NT = C::NTN, TILES = N / G;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* s = reinterpret_cast<float2*>(smem_raw);
+    const int pt = blockIdx.x / TILES, r0 = blockIdx.x % TILES * G;
+    const int e2 = 2 * a.e, c2 = N - 2 * e2;
+    const float* A1 = a.A1 + (size_t)pt * N * N;
+    const float* A2 = a.A2 + (size_t)pt * c2 * c2;
+    const float mS = (float)a.mom[pt].meanS, mR = (float)a.mom[pt].meanR;
+    float2* Z = a.Z + (size_t)pt * N * N;
+    sbfft::line_fft<N, -1, G, NT, true, false, false>(
+        s, a.twN,
+        [&](int l, int k) {
+            const int ci = r0 + l - e2, cj = k - e2;
+            float2 v = make_float2(A1[(size_t)(r0 + l) * N + k] - mS, 0.f);
+            if (ci >= 0 && ci < c2 && cj >= 0 && cj < c2) v.y = A2[(size_t)ci * c2 + cj] - mR;
+            return v;
+        },
+        [&](int l, int k, float2 v) { Z[(size_t)(r0 + l) * N + k] = v; });
+}
+
+// Forward columns, cross spectrum, inverse columns of the lag rows.
+template <int W>
+__global__ void __launch_bounds__(ColCfg<2 * W>::NT) sw_corr_kernel(SwArgs a)
+{
+    constexpr int N = 2 * W;
+    using C = ColCfg<N>;
+    const int pt = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
+    const int L = 4 * a.e + 1, e2 = 2 * a.e;
+    corr_columns<N>(a.Z + (size_t)pt * N * N, a.T + (size_t)pt * L * corr_ts(N), tile, a.twN,
+                    [e2](int m) { return m <= e2 ? m + e2 : m >= N - e2 ? m - (N - e2) : -1; });
+}
+
+// Inverse rows of pairs of lag rows, normalised correlation, the best
+// position inside the user radius of each CTA's 16 rows.
+template <int W>
+__global__ void __launch_bounds__(SwCfg<W>::NTN) sw_ncc_kernel(SwArgs a)
+{
+    using C = SwCfg<W>;
+    constexpr int N = C::N, G = C::G, NT = C::NTN, TS = corr_ts(N);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2* s = reinterpret_cast<float2*>(smem_raw);
+    double* dsc = reinterpret_cast<double*>(s + C::RN::elems);
+    int* isc = reinterpret_cast<int*>(dsc + NT / 32);
+    const int L = 4 * a.e + 1, e2 = 2 * a.e, tiles = (L + 2 * G - 1) / (2 * G);
+    const int pt = blockIdx.x / tiles, i0 = blockIdx.x % tiles * 2 * G;
+    const float2* T = a.T + (size_t)pt * L * TS;
+    const double* norm = a.norm + (size_t)pt * L * L;
+    double* ncc = a.ncc + (size_t)pt * L * L;
+    const int lim = e2 - OS * (W_NFAST / 4);
+    float* c = reinterpret_cast<float*>(s);  // 2 G rows of covariances, over the spent line slots
+    sbfft::line_fft<N, 1, G, NT, true, false, true>(
+        s, a.twN,
+        [&](int l, int k) {
+            const int ra = min(i0 + 2 * l, L - 1), rb = min(i0 + 2 * l + 1, L - 1);
+            return pair_row_input<N>(T + (size_t)ra * TS, T + (size_t)rb * TS, k);
+        },
+        [&](int l, int k, float2 v) {
+            const int j = k <= e2 ? k + e2 : k >= N - e2 ? k - (N - e2) : -1;
+            if (j < 0) return;
+            c[2 * l * N + j] = v.x;
+            c[(2 * l + 1) * N + j] = v.y;
+        });
+    __syncthreads();
+    DArg best;
+    best.v = -1e30;
+    best.rank = 0x7fffffff;
+    const int lane = threadIdx.x & 31;
+    for (int h = threadIdx.x >> 5; h < 2 * G; h += NT / 32) {
+        const int i = i0 + h;
+        if (i >= L) break;
+        const bool in = abs(i - e2) <= lim;
+#pragma unroll 4
+        for (int j = lane; j < L; j += 32) {
+            const double x = (double)c[h * N + j] * __ldg(norm + i * L + j);
+            ncc[i * L + j] = x;
+            if (in && abs(j - e2) <= lim && darg_better(x, i * L + j, best.v, best.rank)) {
+                best.v = x;
+                best.rank = i * L + j;
             }
         }
-        best = block_argmax_d<NT>(best, red, isc);
-        const int gidx = a.list[it];
-        if (!(best.v >= 0.0) || best.rank == 0x7fffffff) {  // maxCorr < 0: no match (:511-512)
-            if (tid == 0) {
-                a.offR[gidx] = -2.0e9f;
-                a.offA[gidx] = -2.0e9f;
-                a.corr[gidx] = 0.0f;
-                a.type[gidx] = SB_AMPMATCH;
-                atomicAdd(&a.stats[1], 1ull);
-            }
-            __syncthreads();
-            continue;
+    }
+    best = block_argmax_d<NT>(best, dsc, isc);
+    if (threadIdx.x == 0) {
+        a.bestV[blockIdx.x] = best.v;
+        a.bestE[blockIdx.x] = best.rank;
+    }
+}
+
+// The peak of a point, oversampled; its outputs.
+__global__ void __launch_bounds__(512) sw_peak_kernel(SwArgs a, int tiles)
+{
+    constexpr int NT = 512;
+    __shared__ double Bm[W_OSW * W_N1], X[W_N1 * W_N1], T[W_N1 * W_OSW], dsc[NT / 32];
+    __shared__ int isc[NT / 32];
+    const int pt = blockIdx.x, tid = threadIdx.x, L = 4 * a.e + 1;
+    DArg best;
+    best.v = -1e30;
+    best.rank = 0x7fffffff;
+    for (int t = tid; t < tiles; t += NT) {
+        const double v = a.bestV[(size_t)pt * tiles + t];
+        const int r = a.bestE[(size_t)pt * tiles + t];
+        if (darg_better(v, r, best.v, best.rank)) {
+            best.v = v;
+            best.rank = r;
         }
-        const int iMax = best.rank / L, jMax = best.rank % L;
-        if constexpr (C::OS_IN_TILE)  // the tiles are idle until the next point's transforms
-            for (int e = tid; e < W_OSW * W_N1; e += NT) Bm[e] = __ldg(a.B + e);
-        for (int e = tid; e < W_N1 * W_N1; e += NT) {
-            const int bi = e / W_N1, bj = e % W_N1;
-            X[e] = ncc[(size_t)(iMax - W_NFAST / 2 + bi) * L + (jMax - W_NFAST / 2 + bj)];
-        }
-        __syncthreads();
-        // T[t1][n2] = sum_t2 X[t1][t2] B[n2][t2]
-        for (int e = tid; e < W_N1 * W_OSW; e += NT) {
-            const int t1 = e / W_OSW, n2 = e % W_OSW;
-            double acc = 0.0;
-            for (int t2 = 0; t2 < W_N1; ++t2) acc += X[t1 * W_N1 + t2] * Bm[n2 * W_N1 + t2];
-            T[e] = acc;
-        }
-        __syncthreads();
-        DArg ob;
-        ob.v = -1.0e30;
-        ob.rank = 0x7fffffff;
-        for (int e = tid; e < W_OSW * W_OSW; e += NT) {
-            const int n1 = e / W_OSW, n2 = e % W_OSW;
-            double acc = 0.0;
-            for (int t1 = 0; t1 < W_N1; ++t1) acc += Bm[n1 * W_N1 + t1] * T[t1 * W_OSW + n2];
-            const double v = acc * acc;
-            if (darg_better(v, e, ob.v, ob.rank)) {
-                ob.v = v;
-                ob.rank = e;
-            }
-        }
-        ob = block_argmax_d<NT>(ob, red, isc);
+    }
+    best = block_argmax_d<NT>(best, dsc, isc);
+    const int gidx = a.list[pt];
+    if (!(best.v >= 0.0) || best.rank == 0x7fffffff) {  // maxCorr < 0: no match (:511-512)
         if (tid == 0) {
-            const int c0 = (W_N1 * W_NOVER) / 2 - W_NOVER * 2;  // 136
-            const int iMax1 = ob.rank / W_OSW + c0, jMax1 = ob.rank % W_OSW + c0;
-            const float cMax = (float)(sqrt(ob.v) / (W_N1 * W_N1));
-            const int iMo = iMax * W_NOVER + iMax1 - (W_NOVER * W_NFAST) / 2;
-            const int jMo = jMax * W_NOVER + jMax1 - (W_NOVER * W_NFAST) / 2;
-            const float rShift1 = ((float)jMo - eR * OS * W_NOVER) / (W_NOVER * OS);
-            const float aShift1 = ((float)iMo - eA * OS * W_NOVER) / (W_NOVER * OS);
-            const float rShift = (float)(pl.z - pl.x), aShift = (float)(pl.w - pl.y);
-            if (cMax > 0.0f) {
-                a.offR[gidx] = rShift - rShift1;
-                a.offA[gidx] = aShift - aShift1;
-                atomicAdd(&a.stats[0], 1ull);
-            } else {
-                a.offR[gidx] = -2.0e9f;
-                a.offA[gidx] = -2.0e9f;
-                atomicAdd(&a.stats[1], 1ull);
-            }
-            a.corr[gidx] = cMax;
+            a.offR[gidx] = -2.0e9f;
+            a.offA[gidx] = -2.0e9f;
+            a.corr[gidx] = 0.0f;
             a.type[gidx] = SB_AMPMATCH;
+            atomicAdd(&a.stats[1], 1ull);
         }
-        __syncthreads();
+        return;
+    }
+    const int iMax = best.rank / L, jMax = best.rank % L;
+    const double* ncc = a.ncc + (size_t)pt * L * L;
+    for (int e = tid; e < W_OSW * W_N1; e += NT) Bm[e] = __ldg(a.B + e);
+    for (int e = tid; e < W_N1 * W_N1; e += NT)
+        X[e] = ncc[(size_t)(iMax - W_NFAST / 2 + e / W_N1) * L + (jMax - W_NFAST / 2 + e % W_N1)];
+    __syncthreads();
+    // T[t1][n2] = sum_t2 X[t1][t2] B[n2][t2]
+    for (int e = tid; e < W_N1 * W_OSW; e += NT) {
+        const int t1 = e / W_OSW, n2 = e % W_OSW;
+        double acc = 0.0;
+        for (int t2 = 0; t2 < W_N1; ++t2) acc += X[t1 * W_N1 + t2] * Bm[n2 * W_N1 + t2];
+        T[e] = acc;
+    }
+    __syncthreads();
+    DArg ob;
+    ob.v = -1.0e30;
+    ob.rank = 0x7fffffff;
+    for (int e = tid; e < W_OSW * W_OSW; e += NT) {
+        const int n1 = e / W_OSW, n2 = e % W_OSW;
+        double acc = 0.0;
+        for (int t1 = 0; t1 < W_N1; ++t1) acc += Bm[n1 * W_N1 + t1] * T[t1 * W_OSW + n2];
+        const double v = acc * acc;
+        if (darg_better(v, e, ob.v, ob.rank)) {
+            ob.v = v;
+            ob.rank = e;
+        }
+    }
+    ob = block_argmax_d<NT>(ob, dsc, isc);
+    if (tid == 0) {
+        const int4 pl = a.win.win[pt];
+        const int c0 = (W_N1 * W_NOVER) / 2 - W_NOVER * 2;  // 136
+        const int iMax1 = ob.rank / W_OSW + c0, jMax1 = ob.rank % W_OSW + c0;
+        const float cMax = (float)(sqrt(ob.v) / (W_N1 * W_N1));
+        const int iMo = iMax * W_NOVER + iMax1 - (W_NOVER * W_NFAST) / 2;
+        const int jMo = jMax * W_NOVER + jMax1 - (W_NOVER * W_NFAST) / 2;
+        const float rShift1 = ((float)jMo - a.e * OS * W_NOVER) / (W_NOVER * OS);
+        const float aShift1 = ((float)iMo - a.e * OS * W_NOVER) / (W_NOVER * OS);
+        const float rShift = (float)(pl.z - pl.x), aShift = (float)(pl.w - pl.y);
+        if (cMax > 0.0f) {
+            a.offR[gidx] = rShift - rShift1;
+            a.offA[gidx] = aShift - aShift1;
+            atomicAdd(&a.stats[0], 1ull);
+        } else {
+            a.offR[gidx] = -2.0e9f;
+            a.offA[gidx] = -2.0e9f;
+            atomicAdd(&a.stats[1], 1ull);
+        }
+        a.corr[gidx] = cMax;
+        a.type[gidx] = SB_AMPMATCH;
     }
 }
 
@@ -577,58 +628,158 @@ __global__ void strackw_init_kernel(float* offR, float* offA, float* corr, uint8
     type[k] = SB_BAD;
 }
 
-template <int W>
-static cudaError_t launch_sw(const SwArgs& a, int nCta, cudaStream_t st)
-{
-    using C = SwCfg<W>;
-    cudaError_t e = cudaFuncSetAttribute(strackw_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem);
-    if (e != cudaSuccess) return e;
-    strackw_kernel<W><<<nCta, C::NT, C::smem, st>>>(a);
-    return cudaGetLastError();
-}
+// Planes in flight: large chunks, so that each launch is many waves of CTAs.
+// The 2000 x 4000 pair at W = 224 takes 48.0 ms with 128 MB of planes (about
+// L2), 36.0 with 512 MB, 30.0 with 1 GB and 28.6 with 2 GB: the kernels are
+// short of instruction issue and shared-memory bandwidth, not of DRAM
+// (10 to 45 % of its rate), so staying in L2 does not pay for short launches.
+// serve.py's memory estimate uses the same figure.
+constexpr size_t SW_CHUNK_BYTES = (size_t)1 << 30;
 
-static int sw_ctas(int W)
-{
-    switch (W) {
-    case 32: return SwCfg<32>::CTAS;
-    case 48: return SwCfg<48>::CTAS;
-    case 64: return SwCfg<64>::CTAS;
-    case 96: return SwCfg<96>::CTAS;
-    case 128: return SwCfg<128>::CTAS;
-    case 192: return SwCfg<192>::CTAS;
-    case 224: return SwCfg<224>::CTAS;
-    default: return SwCfg<256>::CTAS;
+// Workspace of a chunk, carved from one buffer; base null: returns its size.
+struct SwSpace {
+    char* base;
+    size_t used = 0;
+    template <typename T>
+    T* take(size_t n)
+    {
+        T* p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (n * sizeof(T) + 255) / 256 * 256;
+        return p;
     }
-}
+};
+
+template <int W>
+struct SwRun {
+    using C = SwCfg<W>;
+    static constexpr int N = 2 * W;
+
+    static size_t layout(SwArgs& a, int n, char* base, double** dop, int** az)
+    {
+        const size_t L = 4 * a.e + 1, c2 = N - 4 * a.e, NN = (size_t)N * N;
+        SwSpace s{base};
+        a.xv = s.take<float2>((size_t)n * 2 * W * W);
+        a.H = s.take<float>((size_t)n * 2 * NN);
+        a.Z = reinterpret_cast<float2*>(a.H);
+        a.A1 = s.take<float>((size_t)n * NN);
+        a.A2 = s.take<float>((size_t)n * c2 * c2);
+        a.seg = s.take<double>((size_t)n * (N / W_SEG) * 2 * N);
+        a.part = s.take<double>((size_t)n * (N / W_SEG) * 3);
+        a.mom = s.take<SwMoments>(n);
+        a.norm = s.take<double>((size_t)n * L * L);
+        a.T = s.take<float2>((size_t)n * L * corr_ts(N));
+        a.ncc = s.take<double>((size_t)n * L * L);
+        a.bestV = s.take<double>((size_t)n * (L + 15) / 16 + n);
+        a.bestE = s.take<int>((size_t)n * (L + 15) / 16 + n);
+        *dop = s.take<double>(dop_scratch_doubles<W>(n));
+        *az = s.take<int>(n);
+        return s.used;
+    }
+
+    // Copies of the end values beside an intensity row: the box half width,
+    // as far as shared memory goes (a wider box clamps its reads).
+    static int row_pad(const SwArgs& a) { return a.taps < 0 ? 0 : a.navgR < 0 ? 0 : a.navgR < 32 ? a.navgR : 32; }
+
+    template <bool F32>
+    static cudaError_t attributes()
+    {
+        struct { const void* f; size_t sm; } k[] = {
+            {(const void*)sw_cols_kernel<W, F32>, C::smCols},
+            {(const void*)sw_rows_kernel<W, F32>, C::smRows + sizeof(float) * C::G * (N + 64)},
+            {(const void*)sw_stats_kernel<W>, C::smStats}, {(const void*)sw_fwd_kernel<W>, C::smFwd},
+            {(const void*)sw_corr_kernel<W>, ColCfg<N>::smem}, {(const void*)sw_ncc_kernel<W>, C::smNcc}};
+        for (auto& x : k) {
+            const cudaError_t e = cudaFuncSetAttribute(x.f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x.sm);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+
+    // One chunk of a.win.n points.
+    template <bool F32>
+    static cudaError_t chunk(const SwArgs& a, double* dop, int* az, cudaStream_t st, int64_t* launches)
+    {
+        const int n = a.win.n, e2 = 2 * a.e, c2 = N - 2 * e2, L = 2 * e2 + 1;
+        // rows of image 2 whose range sums the chip's azimuth sums read
+        const int g = a.taps >= 0 && a.navgA > 0 ? a.navgA : 0;
+        const int hr0 = e2 - g < 0 ? 0 : (e2 - g) & ~1, hr1 = e2 + c2 - 1 + g < N - 1 ? e2 + c2 - 1 + g : N - 1;
+        const int tiles2 = (hr1 - hr0 + C::G) / C::G, tilesL = (L + 15) / 16, pad = row_pad(a);
+        cudaError_t e = launch_dop<W>(a.win, W, dop, az, st);
+        if (e != cudaSuccess) return e;
+        sw_cols_kernel<W, F32><<<n * 2 * (W / C::G), C::NTW, C::smCols, st>>>(a);
+        sw_rows_kernel<W, F32><<<n * (N / C::G + tiles2), C::NTW, C::smRows + sizeof(float) * C::G * (N + 2 * pad), st>>>(
+            a, hr0, hr1, pad);
+        const int ga = n * (N / W_SEG);
+        switch (a.taps) {
+        case -1: sw_amps_kernel<W, -1><<<ga, N, 0, st>>>(a); break;
+        case 2: sw_amps_kernel<W, 2><<<ga, N, 0, st>>>(a); break;
+        case 3: sw_amps_kernel<W, 3><<<ga, N, 0, st>>>(a); break;
+        default: sw_amps_kernel<W, 0><<<ga, N, 0, st>>>(a); break;
+        }
+        sw_reduce_kernel<W><<<(n + 3) / 4, 128, 0, st>>>(a);
+        sw_stats_kernel<W><<<n * tilesL, C::NTS, C::smStats, st>>>(a);
+        sw_fwd_kernel<W><<<n * (N / C::G), C::NTN, C::smFwd, st>>>(a);
+        sw_corr_kernel<W><<<n * ColCfg<N>::TILES, ColCfg<N>::NT, ColCfg<N>::smem, st>>>(a);
+        sw_ncc_kernel<W><<<n * tilesL, C::NTN, C::smNcc, st>>>(a);
+        sw_peak_kernel<<<n, 512, 0, st>>>(a, tilesL);
+        *launches += 12;
+        return cudaGetLastError();
+    }
+};
 
 static bool sw_supported(int W)
 {
     return W == 32 || W == 48 || W == 64 || W == 96 || W == 128 || W == 192 || W == 224 || W == 256;
 }
-static size_t sw_per_cta(int W, int L)
+
+// Matches nl planned points (win, list: device) in chunks.
+template <int W>
+static int run_sw(sb_context* c, SwArgs a, int nl)
 {
-    switch (W) {
-    case 32: return SwCfg<32>::perCta(L);
-    case 48: return SwCfg<48>::perCta(L);
-    case 64: return SwCfg<64>::perCta(L);
-    case 96: return SwCfg<96>::perCta(L);
-    case 128: return SwCfg<128>::perCta(L);
-    case 192: return SwCfg<192>::perCta(L);
-    case 224: return SwCfg<224>::perCta(L);
-    default: return SwCfg<256>::perCta(L);
+    const bool f32 = a.win.sampleType == SB_CFLOAT32;
+    cudaError_t e = f32 ? SwRun<W>::template attributes<true>() : SwRun<W>::template attributes<false>();
+    if (e != cudaSuccess) return sb_ctx_cuda(c, e, "strackw attributes");
+    a.twW = batch_tw_table<W>(c);
+    a.twN = batch_tw_table<2 * W>(c);
+    a.tau = tau_table(c, W);
+    if (!a.twW || !a.twN || !a.tau) return sb_ctx_fail(c, SB_ERR_NOMEM, "table allocation failed");
+    double* dop;
+    int* az;
+    SwArgs probe = a;
+    const size_t one = SwRun<W>::layout(probe, 16, nullptr, &dop, &az) / 16 + 1;
+    int B = (int)(SW_CHUNK_BYTES / one);
+    B = B < 16 ? 16 : B;
+    const int chunks = (nl + B - 1) / B;
+    B = (nl + chunks - 1) / chunks;  // equal chunks: no short last one
+    const size_t bytes = SwRun<W>::layout(a, B, nullptr, &dop, &az);
+    char* base = (char*)sb_ctx_buf(c, "w_scratch", bytes, &e);
+    if (!base) return sb_ctx_fail(c, SB_ERR_NOMEM, "strackw workspace allocation failed");
+    SwRun<W>::layout(a, B, base, &dop, &az);
+    a.az = az;
+    const int4* win = a.win.win;
+    const int* list = a.list;
+    for (int off = 0; off < nl; off += B) {
+        a.win.win = win + off;
+        a.list = list + off;
+        a.win.n = nl - off < B ? nl - off : B;
+        e = f32 ? SwRun<W>::template chunk<true>(a, dop, az, c->stream, &c->launches)
+                : SwRun<W>::template chunk<false>(a, dop, az, c->stream, &c->launches);
+        if (e != cudaSuccess) return sb_ctx_cuda(c, e, "strackw");
     }
+    return SB_OK;
 }
-static cudaError_t launch_sw_any(int W, const SwArgs& a, int nCta, cudaStream_t st)
+
+static int run_sw_any(int W, sb_context* c, const SwArgs& a, int nl)
 {
     switch (W) {
-    case 32: return launch_sw<32>(a, nCta, st);
-    case 48: return launch_sw<48>(a, nCta, st);
-    case 64: return launch_sw<64>(a, nCta, st);
-    case 96: return launch_sw<96>(a, nCta, st);
-    case 128: return launch_sw<128>(a, nCta, st);
-    case 192: return launch_sw<192>(a, nCta, st);
-    case 224: return launch_sw<224>(a, nCta, st);
-    default: return launch_sw<256>(a, nCta, st);
+    case 32: return run_sw<32>(c, a, nl);
+    case 48: return run_sw<48>(c, a, nl);
+    case 64: return run_sw<64>(c, a, nl);
+    case 96: return run_sw<96>(c, a, nl);
+    case 128: return run_sw<128>(c, a, nl);
+    case 192: return run_sw<192>(c, a, nl);
+    case 224: return run_sw<224>(c, a, nl);
+    default: return run_sw<256>(c, a, nl);
     }
 }
 
@@ -781,34 +932,27 @@ extern "C" int sb_strackw(sb_context* c, const sb_track_params* p, const sb_imag
     CKW(cudaGetLastError(), "strackw_init");
     c->launches++;
     if (nl) {
-        SwArgs a;
-        a.img1 = d1;
-        a.img2 = d2;
-        a.nr1 = img1->nr; a.na1 = img1->na; a.nr2 = img2->nr; a.na2 = img2->na;
-        a.sampleType = img1->sampleType;
-        a.byteOrder = img1->byteOrder;
-        a.plan = dplan;
+        SwArgs a = {};
+        a.win.img1 = d1;
+        a.win.img2 = d2;
+        a.win.nr1 = img1->nr; a.win.na1 = img1->na; a.win.nr2 = img2->nr; a.win.na2 = img2->na;
+        a.win.sampleType = img1->sampleType;
+        a.win.byteOrder = img1->byteOrder;
+        a.win.win = dplan;
         a.list = dlist;
-        a.nList = nl;
-        a.eR = eR;
-        a.eA = eA;
+        a.e = eR;
         a.navgR = p->navgR;
         a.navgA = p->navgA;
+        a.taps = p->navgA <= 1 && p->navgR <= 1 ? -1
+                 : p->navgA == p->navgR && (p->navgR == 2 || p->navgR == 3) ? p->navgR : 0;
         a.scale = 1.f / ((float)W * (float)W * (float)W * (float)W * (float)(OS * OS * OS * OS) *
                          (float)(OS * OS * (p->navgA + 1) * (p->navgR + 1)));
         a.B = dB;
         a.offR = dR; a.offA = dA; a.corr = dC; a.type = dT;
         a.stats = dst;
-        const int L = 4 * eR + 1;
-        a.perCta = sw_per_cta(W, L);
-        int nCta = c->numSM * sw_ctas(W);
-        if (nCta > nl) nCta = nl;
-        a.scratch = (float2*)sb_ctx_buf(c, "w_scratch", sizeof(float2) * a.perCta * nCta, &e);
-        if (!a.scratch) return sb_ctx_fail(c, SB_ERR_NOMEM, "strackw workspace allocation failed");
         cudaEventRecord(c->sev[0], c->stream);
-        CKW(launch_sw_any(W, a, nCta, c->stream), "strackw");
+        if ((rc = run_sw_any(W, c, a, nl)) != SB_OK) return rc;
         cudaEventRecord(c->sev[1], c->stream);
-        c->launches++;
     }
     cudaEventRecord(c->ev[2], c->stream);
     const int od = out->onDevice;

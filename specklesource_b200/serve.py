@@ -38,6 +38,8 @@ _AMP_SCRATCH = {16: 3 * 16 * 16 + 32 * 32 * 3 // 2, 24: 3 * 24 * 24 + 48 * 48 * 
                 32: 3 * 32 * 32 + 64 * 64 * 3 // 2, 48: 3 * 48 * 48 + 96 * 96 * 3 // 2,
                 64: 3 * 64 * 64 + 128 * 128 * 3 // 2, 96: 3 * 96 * 96 + 192 * 192 * 3 // 2,
                 128: 3 * 128 * 128 + 256 * 256 * 3 // 2}
+# planes of strackw in flight (SW_CHUNK_BYTES, csrc/strackw.cu)
+_SW_CHUNK = 1 << 30
 
 
 @dataclass
@@ -87,7 +89,9 @@ def job_device_bytes(job, num_sm=148):
         W = int(p.wRa)
         N = 2 * W
         L = 4 * (int(p.edgePadR) + 5) + 1
-        b += n * 40 + ctas * 8 * (3 * W * W + 3 * N * N + 2 * N * L + 3 * L * L)
+        # planes of a chunk of points (strackw.cu)
+        point = 21 * N * N + 16 * L * L + 8 * L * (N // 2 + 8) + 4096
+        b += n * 40 + min(n * point, max(_SW_CHUNK, 16 * point))
     if job.cull is not None:
         b += n * 64
     return int(b)

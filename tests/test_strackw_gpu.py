@@ -65,6 +65,18 @@ def test_strackw_config3_geometry(ctx, shear):
     assert (o["type"] == abi.SB_AMPMATCH).sum() == 12
 
 
+@pytest.mark.parametrize("W,pad,navg,n,step", [(32, 5, 1, (9, 11), 31), (48, 7, 3, (7, 9), 37), (64, 21, 5, (5, 7), 41),
+                                                (96, 33, 3, (4, 5), 61), (128, 5, 1, (3, 4), 83),
+                                                (256, 40, 4, (2, 2), 150), (64, 8, 2, (1, 1), 1)])
+def test_strackw_every_window_and_box(ctx, shear, W, pad, navg, n, step):
+    """The line lengths, box widths and lag counts the other tests leave out,
+    complex float32 and int16, one point to several row-pair tiles."""
+    a, b = shear
+    _check(ctx, _p(W, pad, navg, n=n, step=step), a, b)
+    ai, bi = (np.stack([np.round(z.real * 2000), np.round(z.imag * 2000)], -1).astype(np.int16) for z in (a, b))
+    _check(ctx, _p(W, pad, navg, n=n, step=step), ai, bi)
+
+
 def test_strackw_int16_msb_and_mask(ctx, shear):
     a, b = shear
     ai = np.stack([np.round(a.real * 2000), np.round(a.imag * 2000)], -1).astype(">i2")
