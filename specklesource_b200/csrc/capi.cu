@@ -614,6 +614,18 @@ static FitArgs make_fit_args(const sb_track_params* p, FitJob* fit, int nList, i
         if (_e != cudaSuccess) return sb_ctx_cuda(c, _e, what);      \
     } while (0)
 
+// One amplitude try over a.nList entries.
+static int amp_try(sb_context* c, int Ws, const AmpArgs& a)
+{
+    if (!amps_supported(Ws)) return run_strack_amp(c, Ws, a, a.nList);
+    int nCta = c->numSM * amps_ctas(c, Ws);
+    if (nCta > a.nList) nCta = a.nList;
+    if (nCta < 1) return sb_ctx_fail(c, SB_ERR_CUDA, "amplitude kernel cannot be resident (Ws=%d)", Ws);
+    CK(launch_strack_amps(Ws, a, nCta, c->stream), "strack_amps");
+    c->launches++;
+    return SB_OK;
+}
+
 // ---------------------------------------------------------------- strack
 
 extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image* img1, const sb_image* img2,
@@ -918,8 +930,8 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         CK(cudaMemcpyAsync(dStageCnt + stage, dCnt, sizeof(int), cudaMemcpyDeviceToDevice, c->stream), "count");
         const int Ws = WA * (stage == 1 ? 1 : LA);
         // small windows (shared-memory kernel): launched for the whole grid,
-        // the list length read on the device; larger windows size a per-CTA
-        // workspace by the list, so their length is read back first
+        // the list length read on the device; larger windows run the list in
+        // chunks, so their length is read back first
         const bool onChip = amps_supported(Ws);
         int cnt = n;
         if (!onChip) {
@@ -957,28 +969,14 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         a.twWs = tw_table(c, Ws);
         a.tw2Ws = tw_table(c, 2 * Ws);
         a.tau = tau_table(c, Ws);
-        a.osA = osA_table(c);
         a.osD = osD_table(c);
         a.gauss = p->gaussFlag ? 1 : 0;
         a.rec = drec;
         a.fit = dfit;
-        // small windows: everything in shared memory; larger: per-CTA
-        // workspace in global memory staged through shared tiles
-        int nCta = c->numSM * (onChip ? amps_ctas(c, Ws) : amp_blocks_per_sm(Ws));
-        if (nCta > cnt) nCta = cnt;
-        if (nCta < 1) return sb_ctx_fail(c, SB_ERR_CUDA, "amplitude kernel cannot be resident (Ws=%d)", Ws);
-        if (!onChip) {
-            a.scratchPerCta = amp_scratch_elems(Ws);
-            a.scratch = (float2*)sb_ctx_buf(c, "ampScratch", sizeof(float2) * a.scratchPerCta * nCta, &e);
-        }
-        if ((!onChip && !a.scratch) || !a.twWs || !a.tw2Ws || !a.tau || !a.osA || !a.osD)
+        if (!a.twWs || !a.tw2Ws || !a.tau || !a.osD)
             return sb_ctx_fail(c, SB_ERR_NOMEM, "amplitude workspace allocation failed");
         cudaEventRecord(c->sev[2 + 2 * stage], c->stream);
-        if (onChip)
-            CK(launch_strack_amps(Ws, a, nCta, c->stream), "strack_amps");
-        else
-            CK(launch_strack_amp(Ws, a, nCta, c->stream), "strack_amp");
-        c->launches++;
+        if ((rc = amp_try(c, Ws, a)) != SB_OK) return rc;
         cudaEventRecord(c->sev[3 + 2 * stage], c->stream);
         FitArgs f = make_fit_args(p, dfit, cnt, stage, drec);
         f.nListDev = onChip ? dCnt : nullptr;
@@ -1408,7 +1406,7 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
             CK(cudaMemcpyAsync(dStageCnt + 3 * bi + stage, dCnt, sizeof(int), cudaMemcpyDeviceToDevice, c->stream),
                "count");
             const int Ws = WA * (stage == 1 ? 1 : LA);
-            // as in sb_strack: the length is read back only for the staged kernel
+            // as in sb_strack: the length is read back only for the chunked kernels
             const bool onChip = amps_supported(Ws);
             int cnt = nB;  // upper bound
             if (!onChip) {
@@ -1446,25 +1444,13 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
             a.twWs = tw_table(c, Ws);
             a.tw2Ws = tw_table(c, 2 * Ws);
             a.tau = tau_table(c, Ws);
-            a.osA = osA_table(c);
             a.osD = osD_table(c);
             a.gauss = p->gaussFlag ? 1 : 0;
             a.rec = brec;
             a.fit = dfit;
-            int nCta = c->numSM * (onChip ? amps_ctas(c, Ws) : amp_blocks_per_sm(Ws));
-            if (nCta > cnt) nCta = cnt;
-            if (nCta < 1) return sb_ctx_fail(c, SB_ERR_CUDA, "amplitude kernel cannot be resident (Ws=%d)", Ws);
-            if (!onChip) {
-                a.scratchPerCta = amp_scratch_elems(Ws);
-                a.scratch = (float2*)sb_ctx_buf(c, "ampScratch", sizeof(float2) * a.scratchPerCta * nCta, &e);
-            }
-            if ((!onChip && !a.scratch) || !a.twWs || !a.tw2Ws || !a.tau || !a.osA || !a.osD)
+            if (!a.twWs || !a.tw2Ws || !a.tau || !a.osD)
                 return sb_ctx_fail(c, SB_ERR_NOMEM, "amplitude workspace allocation failed");
-            if (onChip)
-                CK(launch_strack_amps(Ws, a, nCta, c->stream), "strack_amps");
-            else
-                CK(launch_strack_amp(Ws, a, nCta, c->stream), "strack_amp");
-            c->launches++;
+            if ((rc = amp_try(c, Ws, a)) != SB_OK) return rc;
             FitArgs f = make_fit_args(p, dfit, cnt, stage, brec);
             f.nListDev = onChip ? dCnt : nullptr;
             CK(launch_strack_fit(f, c->stream), "strack_fit");

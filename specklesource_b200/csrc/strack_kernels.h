@@ -6,6 +6,8 @@
 
 #include "strack_common.cuh"
 
+struct sb_context;
+
 namespace sbk {
 
 // The neighbourhood of a complex-match peak, handed from the complex kernel
@@ -94,10 +96,7 @@ struct AmpArgs {
     const float2* twWs;   // W_Ws table (Ws = wa*s)
     const float2* tw2Ws;  // W_{2Ws} table
     const float2* tau;    // parity twiddles for Ws
-    const float2* osA;
-    const float2* osD;    // real form of the oversampling matrix (shared-memory kernel)
-    float2* scratch;      // per-CTA workspace
-    size_t scratchPerCta; // float2 elements
+    const float2* osD;    // real form of the oversampling matrix
     PointRec* rec;
     FitJob* fit;
     int gauss;            // -gauss: 2-D Gaussian fit instead of the oversampling
@@ -118,10 +117,9 @@ int cmplx_tc_blocks_per_sm();
 cudaError_t launch_strack_cmplx_tc(const CmplxArgs& a, int nCta, cudaStream_t st);
 
 bool amp_supported(int Ws);
-size_t amp_scratch_elems(int Ws);
-int amp_blocks_per_sm(int Ws);  // resident CTAs per SM of the staged amplitude kernel
-int amp_threads(int Ws);
-cudaError_t launch_strack_amp(int Ws, const AmpArgs& a, int nCta, cudaStream_t st);
+// Tries of windows above 64 (strack_amp.cu) for the cnt entries of a.list, on
+// the context's stream, its workspace and its launch count.
+int run_strack_amp(sb_context* c, int Ws, const AmpArgs& a, int cnt);
 
 // shared-memory-resident amplitude tries for small windows
 bool amps_supported(int Ws);
