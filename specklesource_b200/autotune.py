@@ -9,9 +9,9 @@ CUDA-event timing, median of `reps` calls after a warm-up call):
   * FP32 complex stage, windows 16, 24, 32, 48, 64: both compiled thread
     counts x every resident CTA count per SM (amplitude tries off);
   * split-BF16 complex stage, window 64: 1 or 2 CTAs per SM;
-  * shared-memory amplitude try, windows 16, 24, 32, 48: every resident CTA
-    count per SM (-noComplex, one try; window 64 fits one CTA per SM, so
-    there is nothing to choose).
+  * shared-memory amplitude try, windows 16, 24, 32: every resident CTA count
+    per SM (-noComplex, one try; larger windows run in chunks without a launch
+    shape).
 
 and writes the fastest shape per bucket, with every candidate's time, to a
 JSON table.  runtime.Context applies the table of the device it runs on
@@ -79,7 +79,7 @@ def tune(device=0, reps=3, na=2048, nr=4096):
     entries.append(_try_shapes(ctx, "complex_tc", 64, (0,), _grid(64, na, nr, maxTries=0), s1, s2, "cmplx_ms",
                                reps))
     ctx.set_form(abi.SB_FORM_FP32)
-    for W in (16, 24, 32, 48):
+    for W in (16, 24, 32):
         p = _grid(W, na, nr, noComplex=1, maxTries=1)
         entries.append(_try_shapes(ctx, "amplitude", W, (0,), p, s1, s2, "amp_small_ms", reps))
     ctx.close()

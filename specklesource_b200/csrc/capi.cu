@@ -212,9 +212,10 @@ extern "C" int sb_set_tuning(sb_context* c, int kernel, int window, int threads,
         return SB_OK;
     }
     if (kernel == SB_TUNE_AMPLITUDE) {
-        if (wi < 0 || !amps_supported(window) || threads != 0)
-            return sb_ctx_fail(c, SB_ERR_UNSUPPORTED, "shared-memory amplitude try: windows 16-64, default threads");
-        const int mx = amps_blocks_per_sm(window);
+        if (wi < 0 || threads != 0)
+            return sb_ctx_fail(c, SB_ERR_UNSUPPORTED, "amplitude try: windows 16-64, default threads");
+        // windows 48 and 64 run in chunks without a launch shape: accepted, no effect
+        const int mx = amps_supported(window) ? amps_blocks_per_sm(window) : 1;
         if (ctasPerSm > mx) return sb_ctx_fail(c, SB_ERR_ARG, "at most %d CTAs per SM", mx);
         c->tuneAmpsCtas[wi] = ctasPerSm;
         return SB_OK;
@@ -317,24 +318,6 @@ const float2* tau_table(sb_context* c, int W)
         h[k] = make_float2((float)(sgn * cos(ang)), (float)(sgn * sin(ang)));
     }
     return (const float2*)sb_table(c, "tau" + std::to_string(W), h);
-}
-
-// A[n][t] = sum_{f=-4..3} exp(+2 pi i f (n - 12 t)/96), n = 24..71.
-const float2* osA_table(sb_context* c)
-{
-    std::vector<float2> h(OSW * NFAST);
-    for (int n = 0; n < OSW; ++n)
-        for (int t = 0; t < NFAST; ++t) {
-            double re = 0, im = 0;
-            const int d = (n + 24) - NOVER * t;
-            for (int f = -NFAST / 2; f < NFAST / 2; ++f) {
-                double ang = 2.0 * kPi * (double)f * (double)d / (double)(NFAST * NOVER);
-                re += cos(ang);
-                im += sin(ang);
-            }
-            h[n * NFAST + t] = make_float2((float)re, (float)im);
-        }
-    return (const float2*)sb_table(c, "osA", h);
 }
 
 // Real form of the oversampling matrix: A[n][t] = p(n) exp(+i pi t/8) D[n][t]
@@ -793,7 +776,6 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         a.hanCorr = p->hanningFlag ? 1.5 : 1.0;
         a.twW = tw_table(c, W);
         a.tau = tau_table(c, W);
-        a.osA = osA_table(c);
         a.osD = osD_table(c);
         a.gauss = p->gaussFlag ? 1 : 0;
         a.azThresh = p->azDefocusThresh;
@@ -827,7 +809,7 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
             a.twP = tw_table(c, intPs);
             if (!a.twP) return sb_ctx_fail(c, SB_ERR_NOMEM, "table allocation failed");
         }
-        if (!a.twW || !a.tau || !a.osA || !a.osD || (p->hanningFlag && !a.hanning))
+        if (!a.twW || !a.tau || !a.osD || (p->hanningFlag && !a.hanning))
             return sb_ctx_fail(c, SB_ERR_NOMEM, "table allocation failed");
         // the split-BF16 tensor-core form where it applies (see sb_set_form)
         const bool tcForm = c->form == SB_FORM_SPLIT_BF16 && cmplx_tc_supported(W) && !baseOn && !p->intf &&
@@ -1332,14 +1314,13 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
             a.hanCorr = p->hanningFlag ? 1.5 : 1.0;
             a.twW = tw_table(c, W);
             a.tau = tau_table(c, W);
-            a.osA = osA_table(c);
-            a.osD = osD_table(c);
+                a.osD = osD_table(c);
             a.gauss = p->gaussFlag ? 1 : 0;
             a.azThresh = p->azDefocusThresh;
             a.checkAzFocus = p->checkAzFocus;
             a.noComplex = p->noComplex;
             a.rec = drec;
-            if (!a.twW || !a.tau || !a.osA || !a.osD || (p->hanningFlag && !a.hanning))
+            if (!a.twW || !a.tau || !a.osD || (p->hanningFlag && !a.hanning))
                 return sb_ctx_fail(c, SB_ERR_NOMEM, "table allocation failed");
             const bool tcForm = form == SB_FORM_SPLIT_BF16 && cmplx_tc_supported(W) && !p->gaussFlag && c->smMajor >= 10;
             if (tcForm) {

@@ -1,5 +1,6 @@
-// strack_amp.cu -- amplitude tries of strack whose windows are too large for
-// one CTA's shared memory (small window s = 1, large window s = LA = 2).
+// strack_amp.cu -- amplitude tries of strack with windows from 48 up (small
+// window s = 1, large window s = LA = 2); strack_amps.cu keeps the smaller ones
+// in one CTA's shared memory.
 //
 // Follows getAmpPatches (Strack/speckleTrack.c:1006-1189), ampMatch
 // (:398-484) and ampTrackFast (:489-597).  List entries go through the kernels
@@ -480,11 +481,13 @@ struct AmRun {
     }
 };
 
-bool amp_supported(int Ws) { return amps_supported(Ws) || Ws == 96 || Ws == 128; }
+bool amp_supported(int Ws) { return amps_supported(Ws) || Ws == 48 || Ws == 64 || Ws == 96 || Ws == 128; }
 
 int run_strack_amp(sb_context* c, int Ws, const AmpArgs& a, int cnt)
 {
     switch (Ws) {
+    case 48: return AmRun<48>::run(c, a, cnt);
+    case 64: return AmRun<64>::run(c, a, cnt);
     case 96: return AmRun<96>::run(c, a, cnt);
     case 128: return AmRun<128>::run(c, a, cnt);
     default: return sb_ctx_fail(c, SB_ERR_UNSUPPORTED, "amplitude window %d not supported", Ws);

@@ -51,8 +51,7 @@ struct CmplxArgs {
     double hanCorr;        // 1.5 with Hanning, else 1.0
     const float2* twW;     // W_W^e forward twiddles, W entries
     const float2* tau;     // parity twiddles, W entries
-    const float2* osA;     // 48 x 8 oversampling matrix
-    const float2* osD;     // real form of it: 48 x 8 floats D, then 16 phases
+    const float2* osD;     // real oversampling matrix: 48 x 8 floats D, then 16 phases
     float azThresh;
     int checkAzFocus, noComplex;
     int baseOn;
@@ -117,11 +116,11 @@ int cmplx_tc_blocks_per_sm();
 cudaError_t launch_strack_cmplx_tc(const CmplxArgs& a, int nCta, cudaStream_t st);
 
 bool amp_supported(int Ws);
-// Tries of windows above 64 (strack_amp.cu) for the cnt entries of a.list, on
+// Tries of windows 48 to 128 (strack_amp.cu) for the cnt entries of a.list, on
 // the context's stream, its workspace and its launch count.
 int run_strack_amp(sb_context* c, int Ws, const AmpArgs& a, int cnt);
 
-// shared-memory-resident amplitude tries for small windows
+// shared-memory-resident amplitude tries (windows 16, 24 and 32)
 bool amps_supported(int Ws);
 int amps_blocks_per_sm(int Ws);
 cudaError_t launch_strack_amps(int Ws, const AmpArgs& a, int nCta, cudaStream_t st);

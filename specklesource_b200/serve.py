@@ -33,7 +33,7 @@ _STRACK_POINT_BYTES = 20 + 80 + 16 + 160 + 17 + 64
 # most one list chunk (kPeakChunk in csrc/capi.cu)
 _PEAK_JOB_BYTES = 960
 _PEAK_CHUNK = 1 << 19
-# planes in flight of the amplitude tries above window 64 and of strackw
+# planes in flight of the amplitude tries from window 48 up and of strackw
 # (AM_CHUNK_BYTES, csrc/strack_amp.cu; SW_CHUNK_BYTES, csrc/strackw.cu)
 _AMP_CHUNK = 512 << 20
 _SW_CHUNK = 1 << 30
@@ -79,7 +79,7 @@ def job_device_bytes(job, num_sm=148):
         if p.maxTries > 0:
             wa = int(p.wRa)
             ws = wa if p.maxTries < 2 else 2 * wa  # the larger try's planes (one buffer)
-            if ws > 64:
+            if ws > 32:
                 point = 96 * ws * ws + 256 * ws + 8192
                 b += min(n * point, max(_AMP_CHUNK, 16 * point))
     else:

@@ -96,6 +96,26 @@ def test_low_coherence_exercises_fallbacks(ctx):
     assert o["stats"]["nAmp"] + o["stats"]["nAmpL"] > 0
 
 
+@pytest.mark.parametrize("kw,i16", [
+    (dict(wR=48, wA=48, wRa=48, wAa=48, deltaR=61, deltaA=53, nR=28, nA=14), False),  # tries at 48 and 96
+    (dict(wR=48, wA=48, wRa=48, wAa=48, deltaR=61, deltaA=53, nR=28, nA=14, noComplex=1), True),
+    (dict(wR=32, wA=32, wRa=96, wAa=96, deltaR=97, deltaA=83, nR=15, nA=8, noComplex=1, maxTries=1), False),
+    (dict(wR=64, wA=64, wRa=128, wAa=128, deltaR=160, deltaA=160, nR=9, nA=5, noComplex=1, maxTries=1), True),
+    (dict(wR=64, wA=64, wRa=64, wAa=64, deltaR=32, deltaA=32, nR=54, nA=26), False),  # over one chunk of large tries
+])
+def test_amplitude_tries_from_window_48(ctx, kw, i16):
+    """Small and large tries of the chunked kernels, own and inherited rolls,
+    both sample types, a pair that decorrelates from left to right."""
+    s1, s2 = synth.make_pair(1024, 2048, 21, dr=lambda y, x: 1.4 + 0 * x, da=lambda y, x: -0.7 + 0 * x,
+                             coherence=lambda y, x: 0.9 - 0.85 * x / 2048)
+    a, b = synth.to_numpy(s1), synth.to_numpy(s2)
+    if i16:
+        a, b = (np.stack([np.round(z.real * 2000), np.round(z.imag * 2000)], -1).astype(np.int16) for z in (a, b))
+    g, o, st = _check(ctx, _p(rStart=130, aStart=130, **kw), a, b)
+    for k in ("nComplex", "nAmp", "nAmpL"):
+        assert abs(g["stats"][k] - o["stats"][k]) <= max(2, 0.005 * o["stats"]["nAttempted"])
+
+
 def test_big_endian_and_int16_inputs(ctx, small_pair_np):
     a, b = small_pair_np
     p = _p()
