@@ -84,6 +84,31 @@ def test_cull_mask_single_mt_and_sim(ctx):
     _check(g, o)
 
 
+@pytest.mark.parametrize("nA,nR,kw", [
+    (1, 1, dict(bR=1, bA=1, nGood=0)),
+    (7, 5, dict(bR=9, bA=9, nGood=4)),                         # box larger than the grid
+    (33, 65, dict(bR=3, bA=9, nGood=2, maxR=0.05, maxA=2.0)),   # one row and column past a block
+    (64, 31, dict(bR=11, bA=11, nGood=0, maxR=0.0, maxA=0.0)),  # 121 values; everything off the median goes
+    (70, 90, dict(bR=2, bA=4, nGood=1, nCullPasses=1)),
+    (200, 300, dict(bR=5, bA=5, nGood=10, maxR=0.06, maxA=0.06, nCullPasses=5)),  # long chains of culls
+])
+def test_cull_fixpoint_edges(ctx, nA, nR, kw):
+    """Decisions by counting against medians: grids and boxes at the block
+    edges, limits of zero, values that differ by the limit, infinities."""
+    rng = np.random.default_rng(nA * nR)
+    offR = np.round(rng.normal(0, 0.1, (nA, nR)) * 20).astype(np.float32) / np.float32(20)
+    offA = rng.normal(0, 0.1, (nA, nR)).astype(np.float32)
+    for v in (np.nan, np.inf, -2e9):
+        offR[rng.random((nA, nR)) < 0.02] = v
+    offA[rng.random((nA, nR)) < 0.01] = np.inf
+    corr = np.ones((nA, nR), np.float32)
+    mt = np.ones((nA, nR), np.uint8)
+    p = abi.CullParams(nR=nR, nA=nA, **kw)
+    g = ctx.cull(p, offR, offA, corr, mt, passes=("st",))
+    o = oracle.cull(p, offR, offA, corr, mt, passes=("st",))
+    assert _same(g["offR"], o["offR"]) and _same(g["offA"], o["offA"]) and g["nCulled"] == o["nCulled"]
+
+
 def test_cull_large_grid_keep_mask(ctx):
     """Keep masks on a 700 x 993 grid (rows of the large strack workload's grid)."""
     nA, nR = 700, 993
