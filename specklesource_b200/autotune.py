@@ -31,7 +31,7 @@ from . import abi, runtime, synth
 HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_TABLE = os.path.join(HERE, "tuning.json")
 
-COMPLEX_THREADS = {16: (64, 128), 24: (96, 192), 32: (256, 128), 48: (192, 384), 64: (256, 512)}
+COMPLEX_THREADS = {16: (64, 128), 24: (96, 192), 32: (128, 256), 48: (192, 384), 64: (256, 512)}
 KERNEL_IDS = {"complex": abi.SB_TUNE_COMPLEX, "complex_tc": abi.SB_TUNE_COMPLEX_TC,
               "amplitude": abi.SB_TUNE_AMPLITUDE}
 
@@ -55,7 +55,7 @@ def _time(ctx, p, s1, s2, key, reps):
 def _try_shapes(ctx, kernel, W, threads_list, p, s1, s2, key, reps):
     cands = []
     for threads in threads_list:
-        for ctas in range(1, 5):
+        for ctas in range(1, 17):
             rc = ctx.lib.sb_set_tuning(ctx.h, KERNEL_IDS[kernel], W, threads, ctas)
             if rc != abi.SB_OK:
                 break  # above the resident maximum

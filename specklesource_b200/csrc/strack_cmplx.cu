@@ -12,13 +12,13 @@
 // non-zero quadrants folded to X'[k1'][k2'] = S[(k1'+azShift) % W][k2'],
 //   c[2 m1 + e1][2 m2 + e2] = IDFT_W(X' tau_e1[k1'] tau_e2[k2'])[m1][m2],
 //   tau_0 = 1, tau_1[k'] = +-exp(+2 pi i k' / 2W) (minus for k' >= W/2),
-// which is the same sum regrouped.  Only |c| is kept (four W x W float planes).
+// which is the same sum regrouped.  Only |c|^2 is kept (2W x 2W floats).
 //
 // After findCPeak the kernel hands the coarse peak and the |c|^2 samples
 // around it to strack_peak.cu (overSampleC and the gaussPeak1D samples, a warp
 // per patch); with -gauss (GAUSS) the 2-D fit runs here instead.  Thread
-// counts per window are set where the kernel is launched (4W threads, 8W at
-// W = 32), measured per window.
+// counts per window are set where the kernel is launched (4W threads),
+// measured per window.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -28,30 +28,127 @@
 
 namespace sbk {
 
+// Work split of the transforms.  Every line of W = N1 N2 points (rows and
+// columns alike) belongs to one warp: LG lines at a time, four lines side by
+// side times N2 (first step) or N1 (second step) threads a line, so the
+// exchange between the two steps needs a warp barrier instead of a block
+// barrier, and a thread's n2 -- and with it its inter-step twiddles, which it
+// keeps in registers -- never changes.  Row stride W + 4 and the order
+// n2 ^ k1 inside the k1 blocks make every access of both passes
+// conflict-free: four lines start 4 slots apart modulo 16, in a row pass the
+// lanes of a half warp add four neighbouring slots, in a column pass rows are
+// 4 apart.
+// Against block-wide passes over three buffers (two CTAs per SM at W = 64):
+// complex and peak kernels over 2400 x 4800 pairs take 0.58 ms for 0.86 at
+// W = 16 (58,608 patches), 1.02 for 1.46 at 24, 1.23 for 1.47 at 32, 3.53 for
+// 4.24 at 48 (75,264) and 5.04 for 5.65 at 64 (73,332).
 template <int W, int NT>
-struct CmplxSmem {
-    static constexpr int RS = W + 1;    // odd row stride: row passes are bank-conflict free
-    static constexpr int IMG = W * RS;  // float2 per buffer; three buffers X, Y, Z
-    static constexpr int OSD = OSW * NFAST / 2 + 16;  // float2 of the real oversampling table
-    static constexpr size_t bytes = sizeof(float2) * (3 * IMG + 2 * W + OSD + NFAST * NFAST + NFAST * OSW) +
-                                    sizeof(float) * (NFAST * NFAST) + sizeof(double) * (NT / 32 + 1) * 8 + 64 + 16;
+struct CmplxSplit {
+    static constexpr int N1 = sbfft::Split<W>::N1, N2 = sbfft::Split<W>::N2;
+    // lines a warp takes at a time: eight where a warp's second step then has
+    // all (16, 32) or three quarters (24, 48) of its lanes busy, four where
+    // that would leave warps without lines
+    static constexpr int LG = W == 64 || W == 48 || (W == 32 && NT > 128) ? 4 : 8;
+    static constexpr int R1 = LG * N2 / 32;         // rounds of the first step
+    static constexpr int R2 = (LG * N1 + 31) / 32;  // rounds of the second step
+    static_assert(N2 == 4 || N2 == 8, "power of two: the exchange order is an xor");
+    static_assert(LG * N2 % 32 == 0 && W % LG == 0, "whole rounds and groups");
 };
 
-// |c|^2 of the 2W x 2W surface at unshifted index (cy, cx).  The parity plane
-// (e1, e2) = (cy & 1, cx & 1) is a W x W float array at float offset poff(q),
-// q = 2 e1 + e2, from the start of shared memory (buffers X | Y | Z of 2W(W+1)
-// floats each): (0,0) X[0, W^2), (0,1) X[W^2, 2W^2), (1,0) the last W^2 floats
-// of Y, (1,1) Z[0, W^2).
-template <int W>
-__device__ __forceinline__ int poff(int q)
+template <int W, int NT>
+struct CmplxSmem {
+    static constexpr int RS = W + 4;    // row stride, float2
+    static constexpr int IMG = W * RS;  // float2 per buffer; two buffers X, Z
+    static constexpr size_t bytes = sizeof(float2) * (2 * IMG + W + NFAST * OSW) + sizeof(float) * (NFAST * NFAST) +
+                                    sizeof(double) * (NT / 32 + 1) * 8 + 64 + 16;
+};
+
+// A warp's share of a pass: which line and sub-index a lane has in a round.
+template <int W, int NT>
+struct CmplxLane {
+    using C = CmplxSplit<W, NT>;
+    static constexpr int N1 = C::N1, N2 = C::N2, RS = CmplxSmem<W, NT>::RS;
+    int lane;
+    float2 tw[N1];  // W_W^{k1 n2}
+    __device__ __forceinline__ int l1(int r) const { return (lane & 3) + 4 * ((r * 32 + lane) / (4 * N2)); }
+    __device__ __forceinline__ int n2() const { return (lane >> 2) % N2; }
+    // lanes past the last item of the second step repeat it: the same values
+    // into the same slots (a predicate around the step costs 300 to 450 bytes
+    // of spills at 80 registers)
+    __device__ __forceinline__ int item2(int r) const { return min(r * 32 + lane, C::LG * N1 - 1); }
+    __device__ __forceinline__ int l2(int r) const { return (item2(r) & 3) + 4 * (item2(r) / (4 * N1)); }
+    __device__ __forceinline__ int k1(int r) const { return (item2(r) >> 2) % N1; }
+    // o[k] = (m ^ k) S for k < N, one addition each: flipping bit b of k moves
+    // m ^ k by +-2^b
+    template <int N, int S>
+    __device__ __forceinline__ static void xor_offsets(int (&o)[N], int m)
+    {
+        const int d[3] = {m & 1 ? -S : S, m & 2 ? -2 * S : 2 * S, m & 4 ? -4 * S : 4 * S};
+        o[0] = m * S;
+#pragma unroll
+        for (int k = 1; k < N; ++k) o[k] = o[k & (k - 1)] + d[k & 1 ? 0 : k & 2 ? 1 : 2];
+    }
+    // first step of one line's share: v in, the lane's exchange slots out
+    template <int DIR, bool COL>
+    __device__ __forceinline__ void first(float2 (&v)[N1], float2* b, int l) const
+    {
+        constexpr int S = COL ? RS : 1;
+        sbfft::RegDFT<N1, DIR, W, true>::run(v, nullptr);
+        int o[N1];
+        xor_offsets<N1, S>(o, n2());
+        float2* p = b + (COL ? l : l * RS);
+#pragma unroll
+        for (int k = 0; k < N1; ++k) {
+            float2 w = tw[k];
+            if (DIR > 0) w.y = -w.y;
+            p[N2 * k * S + o[k]] = k ? sbfft::cmul(v[k], w) : v[0];
+        }
+    }
+    // second step: the lane's exchange slots in, outputs k1 + N1 k2 in u[k2]
+    template <int DIR, bool COL>
+    __device__ __forceinline__ void second(float2 (&u)[N2], const float2* b, int l, int k) const
+    {
+        constexpr int S = COL ? RS : 1;
+        int o[N2];
+        xor_offsets<N2, S>(o, k & (N2 - 1));
+        const float2* p = b + (COL ? l : l * RS) + N2 * k * S;
+#pragma unroll
+        for (int j = 0; j < N2; ++j) u[j] = p[o[j]];
+        sbfft::RegDFT<N2, DIR, W, true>::run(u, nullptr);
+    }
+};
+
+// Transform of a group of lines l0 .. l0 + LG - 1 by one warp, through the
+// lines' slots in b: inputs v[r] of the warp's rounds, outputs to
+// out(l, k, value) once every lane has read its slots.
+template <int W, int NT, int DIR, bool COL, typename Out>
+__device__ __forceinline__ void warp_lines(const CmplxLane<W, NT>& ln,
+                                           float2 (&v)[CmplxSplit<W, NT>::R1][CmplxSplit<W, NT>::N1], float2* b, int l0,
+                                           Out out)
 {
-    constexpr int IMGF = 2 * W * (W + 1);
-    return q == 0 ? 0 : (q == 1 ? W * W : (q == 2 ? 2 * IMGF - W * W : 2 * IMGF));
+    using C = CmplxSplit<W, NT>;
+#pragma unroll
+    for (int r = 0; r < C::R1; ++r) ln.template first<DIR, COL>(v[r], b, l0 + ln.l1(r));
+    __syncwarp();
+    float2 u[C::R2][C::N2];
+#pragma unroll
+    for (int r = 0; r < C::R2; ++r)
+        ln.template second<DIR, COL>(u[r], b, l0 + ln.l2(r), ln.k1(r));
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < C::R2; ++r)
+#pragma unroll
+        for (int k = 0; k < C::N2; ++k) out(l0 + ln.l2(r), ln.k1(r) + C::N1 * k, u[r][k], r, k);
 }
+
+// |c|^2 of the 2W x 2W surface at unshifted index (cy, cx): columns of parity
+// e2 = cx & 1 in X or Z, the rows 2k and 2k + 1 of a column as the two halves
+// of slot (k, cx / 2).
 template <int W>
 __device__ __forceinline__ float cmap(const float* sm, int cy, int cx)
 {
-    return sm[poff<W>(((cy & 1) << 1) | (cx & 1)) + (cy >> 1) * W + (cx >> 1)];
+    constexpr int RS = W + 4;
+    return sm[(cx & 1) * (2 * W * RS) + ((cy >> 1) * RS + (cx >> 1)) * 2 + (cy & 1)];
 }
 // fftshifted surface corrF[y][x] (findCPeak's layout)
 template <int W>
@@ -88,28 +185,7 @@ __device__ __forceinline__ float2 decode_sample(typename std::conditional<F32, u
     }
 }
 
-// Final store of a pair of column passes of the padded inverse, parities
-// (0, E2) and (1, E2) (line l < W: e1 = 0, else e1 = 1, column l mod W):
-// |c|^2 goes to the parity plane and the thread's running maximum of it is
-// kept.  (|c| = sqrtf(|c|^2) is taken where a value is used; the argmax over
-// |c| with findCPeak's tie order is recovered exactly afterwards, see
-// cpeak_from_planes.)  fmaxf ignores NaN, so NaN never wins.
-template <int W, int N1, int N2, int E2>
-struct MagMax {
-    float* plane0;  // parity (0, E2)
-    float* plane1;  // parity (1, E2)
-    float& pmax;
-    __device__ __forceinline__ void operator()(int l, int k1, int k2, float2 z) const
-    {
-        const int e1 = l >= W;
-        const int col = l - (e1 ? W : 0);
-        const float p = z.x * z.x + z.y * z.y;
-        (e1 ? plane1 : plane0)[(k1 + N1 * k2) * W + col] = p;
-        pmax = fmaxf(pmax, p);
-    }
-};
-
-// findCPeak (speckleTrack.c:744-805) over the four |c|^2 planes, given the
+// findCPeak (speckleTrack.c:744-805) over the |c|^2 surface, given the
 // block maximum pmax of |c|^2: the peak is the largest |c| = sqrtf(|c|^2)
 // (> 0), ties to the first position in findCPeak's scan order (cpeak_rank).
 // sqrtf is correctly rounded and monotone, so every position whose sqrtf
@@ -118,7 +194,7 @@ struct MagMax {
 // above 0.  iscr: 2 NT/32 words, one set per reduction; the caller puts a
 // block barrier between this and the next write to them.
 template <int W, int NT>
-__device__ __forceinline__ void cpeak_from_planes(const float* smf, float pmax, unsigned* iscr, int& iMax, int& jMax)
+__device__ __forceinline__ void cpeak_from_surface(const float* smf, float pmax, unsigned* iscr, int& iMax, int& jMax)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned u = __reduce_max_sync(0xffffffffu, __float_as_uint(pmax));  // |c|^2 >= 0: bits order as values
@@ -134,16 +210,16 @@ __device__ __forceinline__ void cpeak_from_planes(const float* smf, float pmax, 
     const float sm = sqrtf(pm);
     const float lo = pm * (1.0f - 1.0f / 1048576.0f);
     unsigned best = 0xffffffffu;
-    constexpr int Q4 = W * W / 4;  // float4 per plane
+    constexpr int Q4 = W / 2;      // float4 per buffer row
     constexpr int U = 4;           // float4 loads in flight per thread
-    for (int e0 = tid; e0 < 4 * Q4; e0 += U * NT) {
+    for (int e0 = tid; e0 < 2 * W * Q4; e0 += U * NT) {
         float4 v[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int e = e0 + u * NT;
-            const int q = e / Q4, i4 = e - q * Q4;
-            v[u] = e < 4 * Q4 ? reinterpret_cast<const float4*>(smf + poff<W>(q))[i4]
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
+            const int row = e / Q4, i4 = e - row * Q4;  // rows 0 .. W-1 of X, then of Z
+            v[u] = e < 2 * W * Q4 ? reinterpret_cast<const float4*>(smf + row * (2 * (W + 4)))[i4]
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -152,13 +228,13 @@ __device__ __forceinline__ void cpeak_from_planes(const float* smf, float pmax, 
             // plain per-value test, sqrtf included)
             if (fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)) < lo) continue;
             const int e = e0 + u * NT;
-            const int q = e / Q4, i4 = e - q * Q4;
+            const int row = e / Q4, i4 = e - row * Q4;
             const float vv[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 if (vv[c] >= lo && sqrtf(vv[c]) == sm) {
-                    const int idx = 4 * i4 + c;
-                    const int cy = 2 * (idx / W) + (q >> 1), cx = 2 * (idx % W) + (q & 1);
+                    const int z = row >= W;
+                    const int cy = 2 * (row - (z ? W : 0)) + (c & 1), cx = 2 * (2 * i4 + (c >> 1)) + z;
                     const int y = cy < W ? cy + W : cy - W, x = cx < W ? cx + W : cx - W;
                     best = min(best, (unsigned)cpeak_rank(y, x, W));
                 }
@@ -184,7 +260,7 @@ __device__ __forceinline__ void cpeak_from_planes(const float* smf, float pmax, 
 // array (for odd ps the last row and column are not copied) and the inverse
 // transform is evaluated directly at the window's pixels; patch 1 is
 // multiplied by conj(P) / |P| (or left alone where |P| < 1e-6).  The small
-// forward DFT and the peak list use `work` (2 ps^2 float2, the free Y buffer).
+// forward DFT and the peak list use `work` (2 ps^2 float2).
 template <int W, int RS, int NT>
 __device__ __forceinline__ void phase_correct_int(const CmplxArgs& a, const PointPlan& pl, float2* X, float2* work,
                                                   double* red)
@@ -312,33 +388,45 @@ __device__ __forceinline__ void phase_correct_int(const CmplxArgs& a, const Poin
     __syncthreads();
 }
 
+// CTAs per SM the registers are limited for.  More CTAs gain little once issue
+// slots and shared-memory bandwidth are about 70 % busy (W = 64: 5.09 ms with
+// two, 5.04 with three, 73,332 patches; W = 48: 3.77 with three, 3.53 with
+// four, 3.79 with five; W = 24: 1.08, 1.05, 1.02 with five, six, eight); the
+// -gauss fit wants registers instead.
+template <bool GAUSS>
+__host__ __device__ constexpr int cmplx_min_ctas(int W, int NT)
+{
+    if (GAUSS) return W == 64 ? (NT == 256 ? 2 : 1) : 3;
+    return W == 64 ? (NT == 256 ? 3 : 1) : W == 48 ? (NT == 192 ? 4 : 2) : W == 32 ? (NT == 128 ? 6 : 3)
+           : W == 24 ? (NT == 96 ? 8 : 4) : (NT == 64 ? 12 : 6);
+}
+
 template <int W, int NT, bool F32, bool GAUSS>
-__global__ void __launch_bounds__(NT, (W >= 64 ? 2 : 3)) strack_cmplx_kernel(CmplxArgs a)
+__global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx_kernel(CmplxArgs a)
 {
     using S = CmplxSmem<W, NT>;
     constexpr int RS = S::RS, IMG = S::IMG;
     constexpr int W2 = 2 * W;
-    constexpr int N1 = sbfft::Split<W>::N1, N2 = sbfft::Split<W>::N2;
+    using C = CmplxSplit<W, NT>;
+    using L = CmplxLane<W, NT>;
+    constexpr int N1 = C::N1, N2 = C::N2, LG = C::LG, NW = NT / 32;
     static_assert((W * W) % NT == 0 && NT % W == 0, "whole rows per thread");
     constexpr int RPT = W * W / NT;  // consecutive rows per thread in the load phase
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* X = reinterpret_cast<float2*>(smem_raw);
-    float2* Y = X + IMG;
-    float2* Z = Y + IMG;
-    float2* twW = Z + IMG;
-    float2* tau = twW + W;
-    float2* osD2 = tau + W;  // 16-byte aligned: every region before it is a multiple of 16 bytes
-    float2* Yb = osD2 + S::OSD;
-    float2* T = Yb + NFAST * NFAST;
+    float2* Z = X + IMG;
+    float2* tau = Z + IMG;
+    float2* T = tau + W;
     float* blk = reinterpret_cast<float*>(T + NFAST * OSW);
     double* red = reinterpret_cast<double*>(blk + NFAST * NFAST);
     int* azs = reinterpret_cast<int*>(red + (NT / 32 + 1) * 8);  // the patch's roll, set by thread 0
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5;
 
-    for (int e = tid; e < W; e += NT) {
-        twW[e] = a.twW[e];
-        tau[e] = a.tau[e];
-    }
+    for (int e = tid; e < W; e += NT) tau[e] = a.tau[e];
+    L ln;
+    ln.lane = tid & 31;
+#pragma unroll
+    for (int k = 0; k < N1; ++k) ln.tw[k] = a.twW[k * ln.n2()];
     __syncthreads();
 
     float* smf = reinterpret_cast<float*>(smem_raw);
@@ -474,47 +562,104 @@ __global__ void __launch_bounds__(NT, (W >= 64 ? 2 : 3)) strack_cmplx_kernel(Cmp
             }
             __syncthreads();
         }
-        if (a.intf) phase_correct_int<W, RS, NT>(a, pl, X, Y, red);
+        if (a.intf)  // its work space follows the kernel's own (launch_cmplx_t)
+            phase_correct_int<W, RS, NT>(a, pl, X, reinterpret_cast<float2*>(smem_raw + S::bytes / 16 * 16 + 16), red);
         // ---------------------------------------------------- spectra of both patches (X and Z)
-        sbfft::fft2d_smem<W, -1, 2, NT, RS, 2 * IMG>(X, twW);
-        const int azShift = *azs;
-        // ---------------------------------------------------- padded inverse
-        // One dual row pass (over k2) makes R0 (e2 = 0, into Y) and R1 (e2 = 1,
-        // times tau[k2], into Z) from the cross spectrum X conj(Z) with the
-        // Doppler row shift folded in.  The per-row factor tau_e1[k1] commutes
-        // with the row transform and is applied in the column passes, so two
-        // row transforms serve the four parities.
-        {
-            const int sh = azShift;
-            auto srcS = [X, Z, sh](int l, int k) {
-                const int r = l + sh;
-                const int o = (r >= W ? r - W : r) * RS + k;
-                return sbfft::cconjmul(X[o], Z[o]);
-            };
-            auto mulTau = [tau](int, int k) { return tau[k]; };
-            auto rowStore = [Y](int l, int k1, int k2, float2 z) {
-                Y[(l % W) * RS + (l / W) * IMG + k1 + N1 * k2] = z;
-            };
-            sbfft::fft_lines_dual<N1, N2, 1, W, NT, RS, 1, IMG, true>(Y, srcS, mulTau, rowStore, twW);
+        // rows, then columns; the column pass stores row k of a spectrum at
+        // row (k - azShift) mod W, which folds the Doppler roll in (the block
+        // sums above ordered the windows' stores and the lag sums' loads)
+#pragma unroll 1
+        for (int g = warp; g < 2 * W / LG; g += NW) {
+            float2* b = g < W / LG ? X : Z;
+            const int l0 = (g % (W / LG)) * LG;
+            float2 v[C::R1][N1];
+#pragma unroll
+            for (int r = 0; r < C::R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n) v[r][n] = b[(l0 + ln.l1(r)) * RS + N2 * n + ln.n2()];
+            __syncwarp();
+            warp_lines<W, NT, -1, false>(ln, v, b, l0, [b](int l, int k, float2 z, int, int) { b[l * RS + k] = z; });
         }
-        // Dual column passes (over k1): R0 (Y) -> parities (0,0) into X and
-        // (1,0) in place; R1 (Z) -> (0,1) into D and (1,1) in place.  Each ends
-        // in |c| and the running argmax; the buffers are placed so that no pass
-        // overwrites an input still needed or a finished plane.
+        __syncthreads();
+        const int azShift = *azs;
+#pragma unroll 1
+        for (int g = warp; g < 2 * W / LG; g += NW) {
+            float2* b = g < W / LG ? X : Z;
+            const int l0 = (g % (W / LG)) * LG;
+            float2 v[C::R1][N1];
+#pragma unroll
+            for (int r = 0; r < C::R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n) v[r][n] = b[(N2 * n + ln.n2()) * RS + l0 + ln.l1(r)];
+            __syncwarp();
+            warp_lines<W, NT, -1, true>(ln, v, b, l0, [b, azShift](int l, int k, float2 z, int, int) {
+                b[(k < azShift ? k - azShift + W : k - azShift) * RS + l] = z;
+            });
+        }
+        __syncthreads();
+        // ---------------------------------------------------- padded inverse
+        // Row transforms (over k2) of the cross spectrum X conj(Z): R0 (e2 = 0)
+        // into X and R1 (e2 = 1, times tau[k2]) into Z.  The per-row factor
+        // tau_e1[k1] commutes with the row transform and is applied in the
+        // column passes, so two row transforms serve the four parities.
+#pragma unroll 1
+        for (int g = warp; g < W / LG; g += NW) {
+            const int l0 = g * LG;
+            float2 u[C::R1][N1], v[C::R1][N1];
+#pragma unroll
+            for (int r = 0; r < C::R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n) {
+                    const int o = (l0 + ln.l1(r)) * RS + N2 * n + ln.n2();
+                    u[r][n] = v[r][n] = sbfft::cconjmul(X[o], Z[o]);
+                }
+            __syncwarp();
+            warp_lines<W, NT, 1, false>(ln, v, X, l0, [X](int l, int k, float2 z, int, int) { X[l * RS + k] = z; });
+#pragma unroll
+            for (int r = 0; r < C::R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n) u[r][n] = sbfft::cmul(u[r][n], tau[N2 * n + ln.n2()]);
+            warp_lines<W, NT, 1, false>(ln, u, Z, l0, [Z](int l, int k, float2 z, int, int) { Z[l * RS + k] = z; });
+        }
+        __syncthreads();
+        // Column transforms (over k1) of R0 and R1, plain and times tau, through
+        // the column's own slots: a column's inputs stay in registers between
+        // the two, so no third buffer is needed and three CTAs fit an SM at
+        // W = 64.  Only |c|^2 is kept, the pair (e1 = 0, 1) as the two halves
+        // of a slot.  Each thread keeps the maximum of its |c|^2.  (|c| =
+        // sqrtf(|c|^2) is taken where a value is used; the argmax over |c| with
+        // findCPeak's tie order is recovered exactly afterwards, see
+        // cpeak_from_surface.)  fmaxf ignores NaN, so NaN never wins.
         float pmax = 0.f;
-        {
-            auto mulTau = [tau](int, int k) { return tau[k]; };
-            auto colY = [Y](int l, int k) { return Y[k * RS + l]; };
-            sbfft::fft_lines_dual<N1, N2, 1, W, NT, 1, RS, IMG, false>(
-                X, colY, mulTau, MagMax<W, N1, N2, 0>{smf + poff<W>(0), smf + poff<W>(2), pmax}, twW);
-            float2* D = X + (W * W) / 2;  // spans the end of X and the start of Y
-            auto colZ = [Z](int l, int k) { return Z[k * RS + l]; };
-            sbfft::fft_lines_dual<N1, N2, 1, W, NT, 1, RS, 2 * IMG - (W * W) / 2, false>(
-                D, colZ, mulTau, MagMax<W, N1, N2, 1>{smf + poff<W>(1), smf + poff<W>(3), pmax}, twW);
+#pragma unroll 1
+        for (int g = warp; g < 2 * W / LG; g += NW) {
+            float2* b = g < W / LG ? X : Z;
+            const int l0 = (g % (W / LG)) * LG;
+            float2 u[C::R1][N1], v[C::R1][N1];
+            float p0[C::R2][N2];
+#pragma unroll
+            for (int r = 0; r < C::R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n)
+                    u[r][n] = v[r][n] = b[(N2 * n + ln.n2()) * RS + l0 + ln.l1(r)];
+            __syncwarp();
+            warp_lines<W, NT, 1, true>(ln, v, b, l0, [&](int, int, float2 z, int r, int k) {
+                p0[r][k] = z.x * z.x + z.y * z.y;
+                pmax = fmaxf(pmax, p0[r][k]);
+            });
+#pragma unroll
+            for (int r = 0; r < C::R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n) u[r][n] = sbfft::cmul(u[r][n], tau[N2 * n + ln.n2()]);
+            warp_lines<W, NT, 1, true>(ln, u, b, l0, [&](int l, int k, float2 z, int r, int kk) {
+                const float q = z.x * z.x + z.y * z.y;
+                pmax = fmaxf(pmax, q);
+                b[k * RS + l] = make_float2(p0[r][kk], q);
+            });
         }
         // ---------------------------------------------------- findCPeak
         int iMax, jMax;
-        cpeak_from_planes<W, NT>(smf, pmax, reinterpret_cast<unsigned*>(red), iMax, jMax);
+        cpeak_from_surface<W, NT>(smf, pmax, reinterpret_cast<unsigned*>(red), iMax, jMax);
         double cMax;
         const bool rejected = (iMax < (NFAST / 2) || iMax > (W2 - NFAST / 2) || jMax < (NFAST / 2) ||
                                jMax > (W2 - NFAST / 2));
@@ -602,7 +747,9 @@ __global__ void __launch_bounds__(NT, (W >= 64 ? 2 : 3)) strack_cmplx_kernel(Cmp
 template <int W, int NT, bool F32, bool GAUSS>
 static cudaError_t launch_cmplx_t(const CmplxArgs& a, int nCta, cudaStream_t st)
 {
-    const size_t sm = CmplxSmem<W, NT>::bytes;
+    size_t sm = CmplxSmem<W, NT>::bytes;
+    // phase_correct_int works on 2 ps^2 float2 behind the kernel's own
+    if (a.intf) sm = sm / 16 * 16 + 16 + sizeof(float2) * 2 * a.intPs * a.intPs;
     cudaError_t e = cudaFuncSetAttribute(strack_cmplx_kernel<W, NT, F32, GAUSS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
@@ -646,7 +793,7 @@ int cmplx_default_threads(int W)
     switch (W) {
     case 16: return 64;
     case 24: return 96;
-    case 32: return 256;
+    case 32: return 128;
     case 48: return 192;
     case 64: return 256;
     default: return 0;
@@ -658,7 +805,7 @@ int cmplx_alt_threads(int W)
     switch (W) {
     case 16: return 128;
     case 24: return 192;
-    case 32: return 128;
+    case 32: return 256;
     case 48: return 384;
     case 64: return 512;
     default: return 0;
@@ -671,7 +818,7 @@ int cmplx_blocks_per_sm(int W, int threads)
     switch (W) {
     case 16: return alt ? occupancy_cmplx<16, 128>() : occupancy_cmplx<16, 64>();
     case 24: return alt ? occupancy_cmplx<24, 192>() : occupancy_cmplx<24, 96>();
-    case 32: return alt ? occupancy_cmplx<32, 128>() : occupancy_cmplx<32, 256>();
+    case 32: return alt ? occupancy_cmplx<32, 256>() : occupancy_cmplx<32, 128>();
     case 48: return alt ? occupancy_cmplx<48, 384>() : occupancy_cmplx<48, 192>();
     case 64: return alt ? occupancy_cmplx<64, 512>() : occupancy_cmplx<64, 256>();
     default: return 0;
@@ -684,7 +831,7 @@ cudaError_t launch_strack_cmplx(int W, const CmplxArgs& a, int nCta, cudaStream_
     switch (W) {
     case 16: return alt ? launch_cmplx_alt<16, 128>(a, nCta, st) : launch_cmplx<16, 64>(a, nCta, st);
     case 24: return alt ? launch_cmplx_alt<24, 192>(a, nCta, st) : launch_cmplx<24, 96>(a, nCta, st);
-    case 32: return alt ? launch_cmplx_alt<32, 128>(a, nCta, st) : launch_cmplx<32, 256>(a, nCta, st);
+    case 32: return alt ? launch_cmplx_alt<32, 256>(a, nCta, st) : launch_cmplx<32, 128>(a, nCta, st);
     case 48: return alt ? launch_cmplx_alt<48, 384>(a, nCta, st) : launch_cmplx<48, 192>(a, nCta, st);
     case 64: return alt ? launch_cmplx_alt<64, 512>(a, nCta, st) : launch_cmplx<64, 256>(a, nCta, st);
     default: return cudaErrorInvalidValue;
