@@ -1,7 +1,6 @@
 // strack_fit.cu -- Gaussian peak-width fits of a strack stage and the
-// decisions that depend on them.  One thread per fit (two per list entry:
-// even lane = range profile, odd lane = azimuth profile), all in registers,
-// double precision (gaussPeak1D + mrqminMod, Strack/speckleTrack.c:2137-2202,
+// decisions that depend on them.  Four lanes per fit, two fits per list entry
+// (range profile, azimuth profile), all in registers, double precision (gaussPeak1D + mrqminMod, Strack/speckleTrack.c:2137-2202,
 // 2309-2416).
 //   complex stage:   aZDefocus = sigmaAz/sigmaRg when the NGAUSS gate passed;
 //                    finalizeCmpxMatch only inside the gate and, with
@@ -26,14 +25,25 @@ struct Cof {
     double chisq;
 };
 
-__device__ __forceinline__ Cof cof18(const double (&x)[NGAUSS], const double (&y)[NGAUSS], double A, double mu,
-                                     double sig)
+// Sum over the LPF lanes of a fit (every lane gets the same bits).
+template <int LPF>
+__device__ __forceinline__ double fit_sum(double v, unsigned mask)
+{
+#pragma unroll
+    for (int o = LPF / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+    return v;
+}
+
+template <int LPF, int NS>
+__device__ __forceinline__ Cof cof18(const double (&x)[NS], const double (&y)[NS], int ns, double A, double mu,
+                                     double sig, unsigned mask)
 {
     Cof c = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const double sig2i = 1.0 / (0.1 * 0.1);
     const double s2 = sig * sig, s3 = s2 * sig;
 #pragma unroll
-    for (int k = 0; k < NGAUSS; ++k) {
+    for (int k = 0; k < NS; ++k) {
+        if (k >= ns) continue;
         const double t = x[k] - mu;
         const double ex = exp(-(0.5 * t * t / s2));
         const double ymod = A * ex;
@@ -51,24 +61,39 @@ __device__ __forceinline__ Cof cof18(const double (&x)[NGAUSS], const double (&y
         c.b3 += dy * w3;
         c.chisq += dy * dy * sig2i;
     }
+    c.a11 = fit_sum<LPF>(c.a11, mask);
+    c.a21 = fit_sum<LPF>(c.a21, mask);
+    c.a22 = fit_sum<LPF>(c.a22, mask);
+    c.a31 = fit_sum<LPF>(c.a31, mask);
+    c.a32 = fit_sum<LPF>(c.a32, mask);
+    c.a33 = fit_sum<LPF>(c.a33, mask);
+    c.b1 = fit_sum<LPF>(c.b1, mask);
+    c.b2 = fit_sum<LPF>(c.b2, mask);
+    c.b3 = fit_sum<LPF>(c.b3, mask);
+    c.chisq = fit_sum<LPF>(c.chisq, mask);
     return c;
 }
 
-// sigma = a[3]/2 of the fit to 18 samples at x0, x0+1, ...
-__device__ double fit_sigma(const float* samp, int x0)
+// sigma = a[3]/2 of the fit to 18 samples at x0, x0+1, ...; lane sub of the
+// fit's LPF lanes takes samples sub, sub + LPF, ...
+template <int LPF>
+__device__ double fit_sigma(const float* samp, int x0, int sub, unsigned mask)
 {
-    double x[NGAUSS], y[NGAUSS];
+    constexpr int NS = (NGAUSS + LPF - 1) / LPF;
+    const int ns = (NGAUSS - sub + LPF - 1) / LPF;
+    double x[NS], y[NS];
     float mx = 0.f;
 #pragma unroll
     for (int k = 0; k < NGAUSS; ++k) mx = fmaxf(mx, samp[k]);
 #pragma unroll
-    for (int k = 0; k < NGAUSS; ++k) {
-        x[k] = (double)(x0 + k);
-        y[k] = (double)samp[k] / (double)mx;
+    for (int k = 0; k < NS; ++k) {
+        const int q = k < ns ? sub + k * LPF : 0;
+        x[k] = (double)(x0 + q);
+        y[k] = (double)samp[q] / (double)mx;
     }
     double A = 1.0, mu = (double)(x0 + NGAUSS / 2), sg = 2.0;
     double alamda = 0.001;
-    Cof al = cof18(x, y, A, mu, sg);
+    Cof al = cof18<LPF, NS>(x, y, ns, A, mu, sg, mask);
     double ochisq = al.chisq;
     double lasti = 2e9;
     for (int it = 0; it < 5; ++it) {
@@ -84,7 +109,7 @@ __device__ double fit_sigma(const float* samp, int x0)
         const double d3 = (m11 * (m22 * al.b3 - m32 * al.b2) - m21 * (m21 * al.b3 - al.b2 * m31) +
                            al.b1 * (m21 * m32 - m22 * m31)) / det;
         const double At = A + d1, mt = mu + d2, st = sg + d3;
-        const Cof tr = cof18(x, y, At, mt, st);
+        const Cof tr = cof18<LPF, NS>(x, y, ns, At, mt, st, mask);
         if (tr.chisq < ochisq) {
             alamda *= 0.1;
             ochisq = tr.chisq;
@@ -101,10 +126,17 @@ __device__ double fit_sigma(const float* samp, int x0)
     return sg * .5;
 }
 
+// LPF lanes a fit.  A fit is a chain of up to six sums of 18 double
+// exponentials: with one lane a fit a list takes the chain's 35 us however short
+// it is.  Whole calls with 1, 2, 4, 8 lanes: 1.022, 0.998, 0.979, 0.990 ms
+// (1024 x 2048, window 32), 5.34, 5.16, 5.12, 5.12 ms (24 tiles in one call),
+// 42.1, 41.6, 41.6, 42.0 ms (6000 x 12000, window 64).
+template <int LPF>
 __global__ void __launch_bounds__(128) strack_fit_kernel(FitArgs a)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int job = t >> 1, f = t & 1;
+    const int sub = t % LPF, job = t / (2 * LPF), f = t / LPF & 1;
+    const unsigned mask = (LPF == 32 ? 0xffffffffu : (1u << LPF) - 1u) << (threadIdx.x & 31 & ~(LPF - 1));
     const int nList = a.nListDev ? min(a.nList, *a.nListDev) : a.nList;
     const bool live = job < nList;
     int gate = 0;
@@ -112,10 +144,11 @@ __global__ void __launch_bounds__(128) strack_fit_kernel(FitArgs a)
     if (live) {
         const FitJob* fj = &a.fit[job];
         gate = fj->gate;
-        if (gate > 0) s = fit_sigma(fj->samp[f], fj->x0[f]);
+        if (gate > 0) s = fit_sigma<LPF>(fj->samp[f], fj->x0[f], sub, mask);
     }
-    const double sAz = __shfl_down_sync(0xffffffffu, s, 1);
-    if (!live || f != 0 || gate < 0) return;
+    __syncwarp();
+    const double sAz = __shfl_down_sync(0xffffffffu, s, LPF);
+    if (!live || f != 0 || sub != 0 || gate < 0) return;
     const int p = a.fit[job].point;
     PointRec* r = &a.rec[p];
     if (a.stage == 0) {
@@ -149,8 +182,9 @@ __global__ void __launch_bounds__(128) strack_fit_kernel(FitArgs a)
 cudaError_t launch_strack_fit(const FitArgs& a, cudaStream_t st)
 {
     if (a.nList <= 0) return cudaSuccess;
-    const long long threads = 2LL * a.nList;
-    strack_fit_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(a);
+    constexpr int LPF = 4;
+    const long long threads = 2LL * a.nList * LPF;
+    strack_fit_kernel<LPF><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(a);
     return cudaGetLastError();
 }
 
