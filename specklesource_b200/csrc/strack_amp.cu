@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(128) am_peak_kernel(AmChunk c)
         const int iMax1 = ob.pos / OSW + (NFAST * NOVER) / 2 - 2 * NOVER;
         const int jMax1 = ob.pos % OSW + (NFAST * NOVER) / 2 - 2 * NOVER;
         cMax = (double)ob.v;
-        cMax = cMax / (pow((double)N, 2) * pow((double)N, 2) * pow((double)NFAST, 2));
+        cMax = cMax / ((double)N * N * N * N * NFAST * NFAST);  // exact
         cMax = cMax / sqrt(p1 * p2);
         iMax = (iMax * NOVER) + iMax1 - (NOVER * NFAST) / 2;
         jMax = (jMax * NOVER) + jMax1 - (NOVER * NFAST) / 2;

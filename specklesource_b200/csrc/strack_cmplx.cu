@@ -25,35 +25,19 @@
 
 #include "strack_device.cuh"
 #include "strack_kernels.h"
+#include "warp_lines.cuh"
 
 namespace sbk {
 
-// Work split of the transforms.  Every line of W = N1 N2 points (rows and
-// columns alike) belongs to one warp: LG lines at a time, four lines side by
-// side times N2 (first step) or N1 (second step) threads a line, so the
-// exchange between the two steps needs a warp barrier instead of a block
-// barrier, and a thread's n2 -- and with it its inter-step twiddles, which it
-// keeps in registers -- never changes.  Row stride W + 4 and the order
-// n2 ^ k1 inside the k1 blocks make every access of both passes
-// conflict-free: four lines start 4 slots apart modulo 16, in a row pass the
-// lanes of a half warp add four neighbouring slots, in a column pass rows are
-// 4 apart.
-// Against block-wide passes over three buffers (two CTAs per SM at W = 64):
-// complex and peak kernels over 2400 x 4800 pairs take 0.58 ms for 0.86 at
-// W = 16 (58,608 patches), 1.02 for 1.46 at 24, 1.23 for 1.47 at 32, 3.53 for
-// 4.24 at 48 (75,264) and 5.04 for 5.65 at 64 (73,332).
+// Lines of a warp at a time (warp_lines.cuh): eight where a warp's second step
+// then has all (16, 32) or three quarters (24) of its lanes busy, four where
+// that would leave warps without lines.  Against block-wide passes over three
+// buffers (two CTAs per SM at W = 64): complex and peak kernels over 2400 x 4800
+// pairs take 0.58 ms for 0.86 at W = 16 (58,608 patches), 1.02 for 1.46 at 24,
+// 1.23 for 1.47 at 32, 3.53 for 4.24 at 48 (75,264) and 5.04 for 5.65 at 64
+// (73,332).
 template <int W, int NT>
-struct CmplxSplit {
-    static constexpr int N1 = sbfft::Split<W>::N1, N2 = sbfft::Split<W>::N2;
-    // lines a warp takes at a time: eight where a warp's second step then has
-    // all (16, 32) or three quarters (24, 48) of its lanes busy, four where
-    // that would leave warps without lines
-    static constexpr int LG = W == 64 || W == 48 || (W == 32 && NT > 128) ? 4 : 8;
-    static constexpr int R1 = LG * N2 / 32;         // rounds of the first step
-    static constexpr int R2 = (LG * N1 + 31) / 32;  // rounds of the second step
-    static_assert(N2 == 4 || N2 == 8, "power of two: the exchange order is an xor");
-    static_assert(LG * N2 % 32 == 0 && W % LG == 0, "whole rounds and groups");
-};
+using CmplxLines = sbfft::WarpLines<W, W == 64 || W == 48 || (W == 32 && NT > 128) ? 4 : 8>;
 
 template <int W, int NT>
 struct CmplxSmem {
@@ -62,84 +46,6 @@ struct CmplxSmem {
     static constexpr size_t bytes = sizeof(float2) * (2 * IMG + W + NFAST * OSW) + sizeof(float) * (NFAST * NFAST) +
                                     sizeof(double) * (NT / 32 + 1) * 8 + 64 + 16;
 };
-
-// A warp's share of a pass: which line and sub-index a lane has in a round.
-template <int W, int NT>
-struct CmplxLane {
-    using C = CmplxSplit<W, NT>;
-    static constexpr int N1 = C::N1, N2 = C::N2, RS = CmplxSmem<W, NT>::RS;
-    int lane;
-    float2 tw[N1];  // W_W^{k1 n2}
-    __device__ __forceinline__ int l1(int r) const { return (lane & 3) + 4 * ((r * 32 + lane) / (4 * N2)); }
-    __device__ __forceinline__ int n2() const { return (lane >> 2) % N2; }
-    // lanes past the last item of the second step repeat it: the same values
-    // into the same slots (a predicate around the step costs 300 to 450 bytes
-    // of spills at 80 registers)
-    __device__ __forceinline__ int item2(int r) const { return min(r * 32 + lane, C::LG * N1 - 1); }
-    __device__ __forceinline__ int l2(int r) const { return (item2(r) & 3) + 4 * (item2(r) / (4 * N1)); }
-    __device__ __forceinline__ int k1(int r) const { return (item2(r) >> 2) % N1; }
-    // o[k] = (m ^ k) S for k < N, one addition each: flipping bit b of k moves
-    // m ^ k by +-2^b
-    template <int N, int S>
-    __device__ __forceinline__ static void xor_offsets(int (&o)[N], int m)
-    {
-        const int d[3] = {m & 1 ? -S : S, m & 2 ? -2 * S : 2 * S, m & 4 ? -4 * S : 4 * S};
-        o[0] = m * S;
-#pragma unroll
-        for (int k = 1; k < N; ++k) o[k] = o[k & (k - 1)] + d[k & 1 ? 0 : k & 2 ? 1 : 2];
-    }
-    // first step of one line's share: v in, the lane's exchange slots out
-    template <int DIR, bool COL>
-    __device__ __forceinline__ void first(float2 (&v)[N1], float2* b, int l) const
-    {
-        constexpr int S = COL ? RS : 1;
-        sbfft::RegDFT<N1, DIR, W, true>::run(v, nullptr);
-        int o[N1];
-        xor_offsets<N1, S>(o, n2());
-        float2* p = b + (COL ? l : l * RS);
-#pragma unroll
-        for (int k = 0; k < N1; ++k) {
-            float2 w = tw[k];
-            if (DIR > 0) w.y = -w.y;
-            p[N2 * k * S + o[k]] = k ? sbfft::cmul(v[k], w) : v[0];
-        }
-    }
-    // second step: the lane's exchange slots in, outputs k1 + N1 k2 in u[k2]
-    template <int DIR, bool COL>
-    __device__ __forceinline__ void second(float2 (&u)[N2], const float2* b, int l, int k) const
-    {
-        constexpr int S = COL ? RS : 1;
-        int o[N2];
-        xor_offsets<N2, S>(o, k & (N2 - 1));
-        const float2* p = b + (COL ? l : l * RS) + N2 * k * S;
-#pragma unroll
-        for (int j = 0; j < N2; ++j) u[j] = p[o[j]];
-        sbfft::RegDFT<N2, DIR, W, true>::run(u, nullptr);
-    }
-};
-
-// Transform of a group of lines l0 .. l0 + LG - 1 by one warp, through the
-// lines' slots in b: inputs v[r] of the warp's rounds, outputs to
-// out(l, k, value) once every lane has read its slots.
-template <int W, int NT, int DIR, bool COL, typename Out>
-__device__ __forceinline__ void warp_lines(const CmplxLane<W, NT>& ln,
-                                           float2 (&v)[CmplxSplit<W, NT>::R1][CmplxSplit<W, NT>::N1], float2* b, int l0,
-                                           Out out)
-{
-    using C = CmplxSplit<W, NT>;
-#pragma unroll
-    for (int r = 0; r < C::R1; ++r) ln.template first<DIR, COL>(v[r], b, l0 + ln.l1(r));
-    __syncwarp();
-    float2 u[C::R2][C::N2];
-#pragma unroll
-    for (int r = 0; r < C::R2; ++r)
-        ln.template second<DIR, COL>(u[r], b, l0 + ln.l2(r), ln.k1(r));
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < C::R2; ++r)
-#pragma unroll
-        for (int k = 0; k < C::N2; ++k) out(l0 + ln.l2(r), ln.k1(r) + C::N1 * k, u[r][k], r, k);
-}
 
 // |c|^2 of the 2W x 2W surface at unshifted index (cy, cx): columns of parity
 // e2 = cx & 1 in X or Z, the rows 2k and 2k + 1 of a column as the two halves
@@ -407,9 +313,8 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
     using S = CmplxSmem<W, NT>;
     constexpr int RS = S::RS, IMG = S::IMG;
     constexpr int W2 = 2 * W;
-    using C = CmplxSplit<W, NT>;
-    using L = CmplxLane<W, NT>;
-    constexpr int N1 = C::N1, N2 = C::N2, LG = C::LG, NW = NT / 32;
+    using L = CmplxLines<W, NT>;
+    constexpr int N1 = L::N1, N2 = L::N2, LG = L::LG, R1 = L::R1, R2 = L::R2, NW = NT / 32;
     static_assert((W * W) % NT == 0 && NT % W == 0, "whole rows per thread");
     constexpr int RPT = W * W / NT;  // consecutive rows per thread in the load phase
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -423,10 +328,7 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
     const int tid = threadIdx.x, warp = tid >> 5;
 
     for (int e = tid; e < W; e += NT) tau[e] = a.tau[e];
-    L ln;
-    ln.lane = tid & 31;
-#pragma unroll
-    for (int k = 0; k < N1; ++k) ln.tw[k] = a.twW[k * ln.n2()];
+    const L ln(a.twW);
     __syncthreads();
 
     float* smf = reinterpret_cast<float*>(smem_raw);
@@ -570,29 +472,22 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
         // sums above ordered the windows' stores and the lag sums' loads)
 #pragma unroll 1
         for (int g = warp; g < 2 * W / LG; g += NW) {
-            float2* b = g < W / LG ? X : Z;
-            const int l0 = (g % (W / LG)) * LG;
-            float2 v[C::R1][N1];
-#pragma unroll
-            for (int r = 0; r < C::R1; ++r)
-#pragma unroll
-                for (int n = 0; n < N1; ++n) v[r][n] = b[(l0 + ln.l1(r)) * RS + N2 * n + ln.n2()];
+            float2* b = (g < W / LG ? X : Z) + (g % (W / LG)) * LG * RS;
+            float2 v[R1][N1];
+            ln.load(v, [b](int l, int k) { return b[l * RS + k]; });
             __syncwarp();
-            warp_lines<W, NT, -1, false>(ln, v, b, l0, [b](int l, int k, float2 z, int, int) { b[l * RS + k] = z; });
+            ln.template run<-1, 1>(v, [b](int l) { return b + l * RS; },
+                                   [b](int l, int k, float2 z, int, int) { b[l * RS + k] = z; });
         }
         __syncthreads();
         const int azShift = *azs;
 #pragma unroll 1
         for (int g = warp; g < 2 * W / LG; g += NW) {
-            float2* b = g < W / LG ? X : Z;
-            const int l0 = (g % (W / LG)) * LG;
-            float2 v[C::R1][N1];
-#pragma unroll
-            for (int r = 0; r < C::R1; ++r)
-#pragma unroll
-                for (int n = 0; n < N1; ++n) v[r][n] = b[(N2 * n + ln.n2()) * RS + l0 + ln.l1(r)];
+            float2* b = (g < W / LG ? X : Z) + (g % (W / LG)) * LG;
+            float2 v[R1][N1];
+            ln.load(v, [b](int l, int k) { return b[k * RS + l]; });
             __syncwarp();
-            warp_lines<W, NT, -1, true>(ln, v, b, l0, [b, azShift](int l, int k, float2 z, int, int) {
+            ln.template run<-1, RS>(v, [b](int l) { return b + l; }, [b, azShift](int l, int k, float2 z, int, int) {
                 b[(k < azShift ? k - azShift + W : k - azShift) * RS + l] = z;
             });
         }
@@ -602,24 +497,27 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
         // into X and R1 (e2 = 1, times tau[k2]) into Z.  The per-row factor
         // tau_e1[k1] commutes with the row transform and is applied in the
         // column passes, so two row transforms serve the four parities.
-#pragma unroll 1
-        for (int g = warp; g < W / LG; g += NW) {
-            const int l0 = g * LG;
-            float2 u[C::R1][N1], v[C::R1][N1];
+        auto times_tau = [&](float2(&u)[R1][N1]) {
 #pragma unroll
-            for (int r = 0; r < C::R1; ++r)
-#pragma unroll
-                for (int n = 0; n < N1; ++n) {
-                    const int o = (l0 + ln.l1(r)) * RS + N2 * n + ln.n2();
-                    u[r][n] = v[r][n] = sbfft::cconjmul(X[o], Z[o]);
-                }
-            __syncwarp();
-            warp_lines<W, NT, 1, false>(ln, v, X, l0, [X](int l, int k, float2 z, int, int) { X[l * RS + k] = z; });
-#pragma unroll
-            for (int r = 0; r < C::R1; ++r)
+            for (int r = 0; r < R1; ++r)
 #pragma unroll
                 for (int n = 0; n < N1; ++n) u[r][n] = sbfft::cmul(u[r][n], tau[N2 * n + ln.n2()]);
-            warp_lines<W, NT, 1, false>(ln, u, Z, l0, [Z](int l, int k, float2 z, int, int) { Z[l * RS + k] = z; });
+        };
+#pragma unroll 1
+        for (int g = warp; g < W / LG; g += NW) {
+            float2 *x = X + g * LG * RS, *z = Z + g * LG * RS;
+            float2 u[R1][N1], v[R1][N1];
+            ln.load(u, [x, z](int l, int k) { return sbfft::cconjmul(x[l * RS + k], z[l * RS + k]); });
+#pragma unroll
+            for (int r = 0; r < R1; ++r)
+#pragma unroll
+                for (int n = 0; n < N1; ++n) v[r][n] = u[r][n];
+            __syncwarp();
+            ln.template run<1, 1>(v, [x](int l) { return x + l * RS; },
+                                  [x](int l, int k, float2 c, int, int) { x[l * RS + k] = c; });
+            times_tau(u);
+            ln.template run<1, 1>(u, [z](int l) { return z + l * RS; },
+                                  [z](int l, int k, float2 c, int, int) { z[l * RS + k] = c; });
         }
         __syncthreads();
         // Column transforms (over k1) of R0 and R1, plain and times tau, through
@@ -633,28 +531,25 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
         float pmax = 0.f;
 #pragma unroll 1
         for (int g = warp; g < 2 * W / LG; g += NW) {
-            float2* b = g < W / LG ? X : Z;
-            const int l0 = (g % (W / LG)) * LG;
-            float2 u[C::R1][N1], v[C::R1][N1];
-            float p0[C::R2][N2];
+            float2* b = (g < W / LG ? X : Z) + (g % (W / LG)) * LG;
+            auto line = [b](int l) { return b + l; };
+            float2 u[R1][N1], v[R1][N1];
+            float p0[R2][N2];
+            ln.load(u, [b](int l, int k) { return b[k * RS + l]; });
 #pragma unroll
-            for (int r = 0; r < C::R1; ++r)
+            for (int r = 0; r < R1; ++r)
 #pragma unroll
-                for (int n = 0; n < N1; ++n)
-                    u[r][n] = v[r][n] = b[(N2 * n + ln.n2()) * RS + l0 + ln.l1(r)];
+                for (int n = 0; n < N1; ++n) v[r][n] = u[r][n];
             __syncwarp();
-            warp_lines<W, NT, 1, true>(ln, v, b, l0, [&](int, int, float2 z, int r, int k) {
-                p0[r][k] = z.x * z.x + z.y * z.y;
-                pmax = fmaxf(pmax, p0[r][k]);
+            ln.template run<1, RS>(v, line, [&](int, int, float2 z, int r, int k2) {
+                p0[r][k2] = z.x * z.x + z.y * z.y;
+                pmax = fmaxf(pmax, p0[r][k2]);
             });
-#pragma unroll
-            for (int r = 0; r < C::R1; ++r)
-#pragma unroll
-                for (int n = 0; n < N1; ++n) u[r][n] = sbfft::cmul(u[r][n], tau[N2 * n + ln.n2()]);
-            warp_lines<W, NT, 1, true>(ln, u, b, l0, [&](int l, int k, float2 z, int r, int kk) {
+            times_tau(u);
+            ln.template run<1, RS>(u, line, [&](int l, int k, float2 z, int r, int k2) {
                 const float q = z.x * z.x + z.y * z.y;
                 pmax = fmaxf(pmax, q);
-                b[k * RS + l] = make_float2(p0[r][kk], q);
+                b[k * RS + l] = make_float2(p0[r][k2], q);
             });
         }
         // ---------------------------------------------------- findCPeak

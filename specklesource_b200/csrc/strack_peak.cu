@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(32 * kPeakWarps) strack_peak_kernel(PeakArgs a
             const int iMax1 = ob.pos / OSW + (NFAST * NOVER) / 2 - 2 * NOVER;
             const int jMax1 = ob.pos % OSW + (NFAST * NOVER) / 2 - 2 * NOVER;
             cMax = (double)ob.v / (NFAST * NFAST);
-            cMax = a.hanCorr * cMax / (sqrt(pj->p1 * pj->p2) * pow((double)(a.W * a.W), 2));
+            cMax = a.hanCorr * cMax / (sqrt(pj->p1 * pj->p2) * ((double)(a.W * a.W) * (double)(a.W * a.W)));
             iMax = (iC * NOVER) + iMax1 - (NOVER * NFAST) / 2;
             jMax = (jC * NOVER) + jMax1 - (NOVER * NFAST) / 2;
             // samples for gaussPeak1D x 2 through the coarse cell of the peak:
