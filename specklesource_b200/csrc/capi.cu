@@ -103,6 +103,10 @@ extern "C" int sb_context_create(int device, sb_context** out)
     for (int k = 0; k < 4; ++k) cudaEventCreate(&c->ev[k]);
     for (int k = 0; k < 16; ++k) cudaEventCreate(&c->sev[k]);
     for (int k = 0; k < SB_MAX_BANDS; ++k) cudaEventCreateWithFlags(&c->chunkEv[k], cudaEventDisableTiming);
+    if (cudaMallocHost((void**)&c->pin, SB_PIN_BYTES) != cudaSuccess) {
+        c->pin = nullptr;  // outputs are then copied one by one
+        cudaGetLastError();
+    }
     // Load sb_amp_match_noalloc's module (with its fixed workspace) and kernels
     // now, so that entry point never loads code or allocates inside its calls.
     // A failure here only disables that entry point; it reports the error.
@@ -126,6 +130,7 @@ extern "C" void sb_context_destroy(sb_context* c)
     for (int k = 0; k < 4; ++k) cudaEventDestroy(c->ev[k]);
     for (int k = 0; k < 16; ++k) cudaEventDestroy(c->sev[k]);
     for (int k = 0; k < SB_MAX_BANDS; ++k) cudaEventDestroy(c->chunkEv[k]);
+    if (c->pin) cudaFreeHost(c->pin);
     cudaStreamDestroy(c->copyStream);
     cudaStreamDestroy(c->stream);
     delete c;
@@ -271,53 +276,46 @@ extern "C" int sb_last_stage_timing(const sb_context* c, float ms[8])
 
 // ---------------------------------------------------------------- tables
 
-// Host-computed constant tables (double precision, rounded once to float).
-const void* sb_table(sb_context* c, const std::string& key, const std::vector<float2>& host)
-{
-    auto it = c->tables.find(key);
-    if (it != c->tables.end()) return it->second;
-    void* d = nullptr;
-    if (cudaMalloc(&d, host.size() * sizeof(float2)) != cudaSuccess) return nullptr;
-    cudaMemcpy(d, host.data(), host.size() * sizeof(float2), cudaMemcpyHostToDevice);
-    c->tables[key] = d;
-    c->tableBytes += host.size() * sizeof(float2);
-    return d;
-}
-
 static const double kPi = 3.14159265358979323846;
 
 const float2* tw_table(sb_context* c, int N)
 {
-    std::vector<float2> h(N);
-    for (int e = 0; e < N; ++e) {
-        double ang = -2.0 * kPi * (double)e / (double)N;
-        h[e] = make_float2((float)cos(ang), (float)sin(ang));
-    }
-    return (const float2*)sb_table(c, "tw" + std::to_string(N), h);
+    return (const float2*)sb_table(c, "tw" + std::to_string(N), [&] {
+        std::vector<float2> h(N);
+        for (int e = 0; e < N; ++e) {
+            double ang = -2.0 * kPi * (double)e / (double)N;
+            h[e] = make_float2((float)cos(ang), (float)sin(ang));
+        }
+        return h;
+    });
 }
 
 const float2* batch_tw_table(sb_context* c, int N1, int N2)
 {
-    const int N = N1 * N2;
-    std::vector<float2> h(N);
-    for (int k1 = 0; k1 < N1; ++k1)
-        for (int n2 = 0; n2 < N2; ++n2) {
-            const double ang = -2.0 * kPi * (double)(k1 * n2) / (double)N;
-            h[k1 * N2 + n2] = make_float2((float)cos(ang), (float)sin(ang));
-        }
-    return (const float2*)sb_table(c, "twb" + std::to_string(N), h);
+    return (const float2*)sb_table(c, "twb" + std::to_string(N1 * N2), [&] {
+        const int N = N1 * N2;
+        std::vector<float2> h(N);
+        for (int k1 = 0; k1 < N1; ++k1)
+            for (int n2 = 0; n2 < N2; ++n2) {
+                const double ang = -2.0 * kPi * (double)(k1 * n2) / (double)N;
+                h[k1 * N2 + n2] = make_float2((float)cos(ang), (float)sin(ang));
+            }
+        return h;
+    });
 }
 
 // tau_1[k'] = +exp(+2 pi i k'/(2W)) for k' < W/2, -exp(...) for k' >= W/2.
 const float2* tau_table(sb_context* c, int W)
 {
-    std::vector<float2> h(W);
-    for (int k = 0; k < W; ++k) {
-        double ang = 2.0 * kPi * (double)k / (2.0 * W);
-        double sgn = (k < W / 2) ? 1.0 : -1.0;
-        h[k] = make_float2((float)(sgn * cos(ang)), (float)(sgn * sin(ang)));
-    }
-    return (const float2*)sb_table(c, "tau" + std::to_string(W), h);
+    return (const float2*)sb_table(c, "tau" + std::to_string(W), [&] {
+        std::vector<float2> h(W);
+        for (int k = 0; k < W; ++k) {
+            double ang = 2.0 * kPi * (double)k / (2.0 * W);
+            double sgn = (k < W / 2) ? 1.0 : -1.0;
+            h[k] = make_float2((float)(sgn * cos(ang)), (float)(sgn * sin(ang)));
+        }
+        return h;
+    });
 }
 
 // Real form of the oversampling matrix: A[n][t] = p(n) exp(+i pi t/8) D[n][t]
@@ -325,40 +323,44 @@ const float2* tau_table(sb_context* c, int W)
 // stored as the 48 x 8 floats of D followed by the 16 phases exp(i pi s/8).
 const float2* osD_table(sb_context* c)
 {
-    std::vector<float2> h(OSW * NFAST / 2 + 16);
-    float* f = reinterpret_cast<float*>(h.data());
-    for (int n = 0; n < OSW; ++n)
-        for (int t = 0; t < NFAST; ++t) {
-            const int d = (n + 24) - NOVER * t;
-            double v = 0.0;
-            for (int g2 = 1; g2 < NFAST; g2 += 2)  // g = g2 / 2
-                v += 2.0 * cos(kPi * (double)g2 * (double)d / (double)(NFAST * NOVER));
-            f[n * NFAST + t] = (float)v;
-        }
-    for (int s = 0; s < 16; ++s)
-        h[OSW * NFAST / 2 + s] = make_float2((float)cos(kPi * s / 8.0), (float)sin(kPi * s / 8.0));
-    return (const float2*)sb_table(c, "osD", h);
+    return (const float2*)sb_table(c, "osD", [&] {
+        std::vector<float2> h(OSW * NFAST / 2 + 16);
+        float* f = reinterpret_cast<float*>(h.data());
+        for (int n = 0; n < OSW; ++n)
+            for (int t = 0; t < NFAST; ++t) {
+                const int d = (n + 24) - NOVER * t;
+                double v = 0.0;
+                for (int g2 = 1; g2 < NFAST; g2 += 2)  // g = g2 / 2
+                    v += 2.0 * cos(kPi * (double)g2 * (double)d / (double)(NFAST * NOVER));
+                f[n * NFAST + t] = (float)v;
+            }
+        for (int s = 0; s < 16; ++s)
+            h[OSW * NFAST / 2 + s] = make_float2((float)cos(kPi * s / 8.0), (float)sin(kPi * s / 8.0));
+        return h;
+    });
 }
 
 // computeHanning (speckleTrack.c:1830-1852), W x W, square windows.
 const float* hanning_table(sb_context* c, int W)
 {
-    std::vector<float2> h((W * W + 1) / 2);
-    float* f = reinterpret_cast<float*>(h.data());
-    for (int i = 0; i < W / 2; i++) {
-        int i1 = W / 2 + i, i2 = W / 2 - i - 1;
-        double wi = 0.5 * (1.0 + cos((2.0 * kPi) * (double)i / (double)(W - 1)));
-        for (int j = 0; j < W / 2; j++) {
-            int j1 = W / 2 + j, j2 = W / 2 - j - 1;
-            double wj = 0.5 * (1.0 + cos((2.0 * kPi) * (double)j / (double)(W - 1)));
-            float v = (float)(wi * wj);
-            f[i1 * W + j1] = v;
-            f[i2 * W + j2] = v;
-            f[i2 * W + j1] = v;
-            f[i1 * W + j2] = v;
+    return (const float*)sb_table(c, "han" + std::to_string(W), [&] {
+        std::vector<float2> h((W * W + 1) / 2);
+        float* f = reinterpret_cast<float*>(h.data());
+        for (int i = 0; i < W / 2; i++) {
+            int i1 = W / 2 + i, i2 = W / 2 - i - 1;
+            double wi = 0.5 * (1.0 + cos((2.0 * kPi) * (double)i / (double)(W - 1)));
+            for (int j = 0; j < W / 2; j++) {
+                int j1 = W / 2 + j, j2 = W / 2 - j - 1;
+                double wj = 0.5 * (1.0 + cos((2.0 * kPi) * (double)j / (double)(W - 1)));
+                float v = (float)(wi * wj);
+                f[i1 * W + j1] = v;
+                f[i2 * W + j2] = v;
+                f[i2 * W + j1] = v;
+                f[i1 * W + j2] = v;
+            }
         }
-    }
-    return (const float*)sb_table(c, "han" + std::to_string(W), h);
+        return h;
+    });
 }
 
 // ---------------------------------------------------------------- planning
@@ -566,14 +568,6 @@ static int check_image(sb_context* c, const sb_image* im)
     if (im->byteOrder != SB_LSB && im->byteOrder != SB_MSB)
         return sb_ctx_fail(c, SB_ERR_ARG, "invalid byteOrder %d", im->byteOrder);
     return SB_OK;
-}
-
-// Copies (or aliases) an output grid.
-static int out_copy(sb_context* c, void* dst, const void* src, size_t bytes, int onDevice)
-{
-    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                                    c->stream);
-    return sb_ctx_cuda(c, e, "cudaMemcpyAsync(output)");
 }
 
 static FitArgs make_fit_args(const sb_track_params* p, FitJob* fit, int nList, int stage, PointRec* rec)
@@ -972,18 +966,19 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
     cudaEventRecord(c->ev[2], c->stream);
 
     // ---- outputs
-    if ((rc = out_copy(c, out->offR, dR, sizeof(float) * n, out->onDevice)) != SB_OK) return rc;
-    if ((rc = out_copy(c, out->offA, dA, sizeof(float) * n, out->onDevice)) != SB_OK) return rc;
-    if ((rc = out_copy(c, out->corr, dC, sizeof(float) * n, out->onDevice)) != SB_OK) return rc;
-    if (out->azd && (rc = out_copy(c, out->azd, dZ, sizeof(float) * n, out->onDevice)) != SB_OK) return rc;
-    if ((rc = out_copy(c, out->type, dT, n, out->onDevice)) != SB_OK) return rc;
+    OutCopies oc(c);
+    if ((rc = oc.add(out->offR, dR, sizeof(float) * n, out->onDevice != 0)) != SB_OK) return rc;
+    if ((rc = oc.add(out->offA, dA, sizeof(float) * n, out->onDevice != 0)) != SB_OK) return rc;
+    if ((rc = oc.add(out->corr, dC, sizeof(float) * n, out->onDevice != 0)) != SB_OK) return rc;
+    if (out->azd && (rc = oc.add(out->azd, dZ, sizeof(float) * n, out->onDevice != 0)) != SB_OK) return rc;
+    if ((rc = oc.add(out->type, dT, n, out->onDevice != 0)) != SB_OK) return rc;
     unsigned long long st[8];
-    CK(cudaMemcpyAsync(st, dstats, sizeof(st), cudaMemcpyDeviceToHost, c->stream), "stats");
+    if ((rc = oc.add(st, dstats, sizeof(st))) != SB_OK) return rc;
     int stageCnt[4] = {0, 0, 0, 0}, tcBad = 0;
-    CK(cudaMemcpyAsync(stageCnt, dStageCnt, sizeof(stageCnt), cudaMemcpyDeviceToHost, c->stream), "counts");
-    if (tcErrFlag) CK(cudaMemcpyAsync(&tcBad, tcErrFlag, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "tcErr");
+    if ((rc = oc.add(stageCnt, dStageCnt, sizeof(stageCnt))) != SB_OK) return rc;
+    if (tcErrFlag && (rc = oc.add(&tcBad, tcErrFlag, sizeof(int))) != SB_OK) return rc;
     cudaEventRecord(c->ev[3], c->stream);
-    CK(cudaStreamSynchronize(c->stream), "strack");
+    if ((rc = oc.finish("strack")) != SB_OK) return rc;
     if (tcBad) return sb_ctx_fail(c, SB_ERR_TIMEOUT, "split-BF16 complex stage: a tensor-core wait timed out");
     if (nC > 0) {
         float t0 = 0, t1 = 0;
@@ -1444,25 +1439,24 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
     }
     cudaEventRecord(c->ev[2], c->stream);
     // ---- outputs, per pair
+    OutCopies oc(c);
     for (int k = 0; k < nPairs; ++k) {
         const size_t g = (size_t)gStart[k], m = (size_t)P[k].nR * P[k].nA;
-        const int od = out[k].onDevice;
-        if ((rc = out_copy(c, out[k].offR, dR + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if ((rc = out_copy(c, out[k].offA, dA + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if ((rc = out_copy(c, out[k].corr, dC + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if (out[k].azd && (rc = out_copy(c, out[k].azd, dZ + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if ((rc = out_copy(c, out[k].type, dT + g, m, od)) != SB_OK) return rc;
+        const bool od = out[k].onDevice != 0;
+        if ((rc = oc.add(out[k].offR, dR + g, sizeof(float) * m, od)) != SB_OK) return rc;
+        if ((rc = oc.add(out[k].offA, dA + g, sizeof(float) * m, od)) != SB_OK) return rc;
+        if ((rc = oc.add(out[k].corr, dC + g, sizeof(float) * m, od)) != SB_OK) return rc;
+        if (out[k].azd && (rc = oc.add(out[k].azd, dZ + g, sizeof(float) * m, od)) != SB_OK) return rc;
+        if ((rc = oc.add(out[k].type, dT + g, m, od)) != SB_OK) return rc;
     }
     std::vector<unsigned long long> st((size_t)8 * nPairs);
-    CK(cudaMemcpyAsync(st.data(), dstats, sizeof(unsigned long long) * 8 * nPairs, cudaMemcpyDeviceToHost, c->stream),
-       "stats");
+    if ((rc = oc.add(st.data(), dstats, sizeof(unsigned long long) * 8 * nPairs)) != SB_OK) return rc;
     int tcBad = 0;
-    CK(cudaMemcpyAsync(&tcBad, dTcErr, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "tcErr");
+    if ((rc = oc.add(&tcBad, dTcErr, sizeof(int))) != SB_OK) return rc;
     std::vector<int> stageCnt((size_t)3 * nBk);
-    CK(cudaMemcpyAsync(stageCnt.data(), dStageCnt, sizeof(int) * 3 * nBk, cudaMemcpyDeviceToHost, c->stream),
-       "counts");
+    if ((rc = oc.add(stageCnt.data(), dStageCnt, sizeof(int) * 3 * nBk)) != SB_OK) return rc;
     cudaEventRecord(c->ev[3], c->stream);
-    CK(cudaStreamSynchronize(c->stream), "strack_batch");
+    if ((rc = oc.finish("strack_batch")) != SB_OK) return rc;
     for (int bi = 0; bi < nBk; ++bi) {
         if (cmplxRan[bi]) {
             float t0 = 0;

@@ -1019,18 +1019,18 @@ int cull_stage_in(sb_context* c, const sb_cull_params* p, sb_cull_data* d, CullD
     return SB_OK;
 }
 
-int cull_stage_out(sb_context* c, const sb_cull_params* p, sb_cull_data* d, const CullDev* v)
+int cull_stage_out(OutCopies* oc, const sb_cull_params* p, sb_cull_data* d, const CullDev* v)
 {
     if (d->onDevice) return SB_OK;
     const size_t n = (size_t)p->nR * p->nA, fb = n * sizeof(float);
-    cudaStream_t s = c->stream;
-    CKC(cudaMemcpyAsync(d->offR, v->offR, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    CKC(cudaMemcpyAsync(d->offA, v->offA, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    CKC(cudaMemcpyAsync(d->type, v->type, n, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->offRS) CKC(cudaMemcpyAsync(d->offRS, v->offRS, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->offAS) CKC(cudaMemcpyAsync(d->offAS, v->offAS, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->sigmaR) CKC(cudaMemcpyAsync(d->sigmaR, v->sigmaR, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->sigmaA) CKC(cudaMemcpyAsync(d->sigmaA, v->sigmaA, fb, cudaMemcpyDeviceToHost, s), "d2h");
+    int rc;
+    if ((rc = oc->add(d->offR, v->offR, fb)) != SB_OK) return rc;
+    if ((rc = oc->add(d->offA, v->offA, fb)) != SB_OK) return rc;
+    if ((rc = oc->add(d->type, v->type, n)) != SB_OK) return rc;
+    if (d->offRS && (rc = oc->add(d->offRS, v->offRS, fb)) != SB_OK) return rc;
+    if (d->offAS && (rc = oc->add(d->offAS, v->offAS, fb)) != SB_OK) return rc;
+    if (d->sigmaR && (rc = oc->add(d->sigmaR, v->sigmaR, fb)) != SB_OK) return rc;
+    if (d->sigmaA && (rc = oc->add(d->sigmaA, v->sigmaA, fb)) != SB_OK) return rc;
     return SB_OK;
 }
 
@@ -1259,9 +1259,10 @@ int cull_run(sb_context* c, In stageIn, F body, Out stageOut)
     cudaEventRecord(c->ev[1], c->stream);
     if ((rc = body(v)) != SB_OK) return rc;
     cudaEventRecord(c->ev[2], c->stream);
-    if ((rc = stageOut(&v)) != SB_OK) return rc;
+    OutCopies oc(c);
+    if ((rc = stageOut(&oc, &v)) != SB_OK) return rc;
     cudaEventRecord(c->ev[3], c->stream);
-    CKC(cudaStreamSynchronize(c->stream), "cull");
+    if ((rc = oc.finish("cull")) != SB_OK) return rc;
     cudaEventElapsedTime(&c->timing[0], c->ev[0], c->ev[3]);
     cudaEventElapsedTime(&c->timing[1], c->ev[0], c->ev[1]);
     cudaEventElapsedTime(&c->timing[2], c->ev[1], c->ev[2]);
@@ -1276,7 +1277,7 @@ int cull_entry(sb_context* c, const sb_cull_params* p, sb_cull_data* d, F body, 
     if (rc != SB_OK) return rc;
     return cull_run(
         c, [&](CullDev* v) { return cull_stage_in(c, p, d, v, whole); }, body,
-        [&](const CullDev* v) { return cull_stage_out(c, p, d, v); });
+        [&](OutCopies* oc, const CullDev* v) { return cull_stage_out(oc, p, d, v); });
 }
 
 int cullls_check(sb_context* c, const sb_cullls_params* p, const sb_cullls_data* d)
@@ -1319,17 +1320,17 @@ int cullls_stage_in(sb_context* c, const sb_cullls_params* p, sb_cullls_data* d,
     return SB_OK;
 }
 
-int cullls_stage_out(sb_context* c, const sb_cullls_params* p, sb_cullls_data* d, const CullDev* v)
+int cullls_stage_out(OutCopies* oc, const sb_cullls_params* p, sb_cullls_data* d, const CullDev* v)
 {
     if (d->onDevice) return SB_OK;
     const size_t fb = (size_t)p->nx * p->ny * sizeof(float);
-    cudaStream_t s = c->stream;
-    CKC(cudaMemcpyAsync(d->X, v->offR, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    CKC(cudaMemcpyAsync(d->Y, v->offA, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->XS) CKC(cudaMemcpyAsync(d->XS, v->offRS, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->YS) CKC(cudaMemcpyAsync(d->YS, v->offAS, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->sigmaX) CKC(cudaMemcpyAsync(d->sigmaX, v->sigmaR, fb, cudaMemcpyDeviceToHost, s), "d2h");
-    if (d->sigmaY) CKC(cudaMemcpyAsync(d->sigmaY, v->sigmaA, fb, cudaMemcpyDeviceToHost, s), "d2h");
+    int rc;
+    if ((rc = oc->add(d->X, v->offR, fb)) != SB_OK) return rc;
+    if ((rc = oc->add(d->Y, v->offA, fb)) != SB_OK) return rc;
+    if (d->XS && (rc = oc->add(d->XS, v->offRS, fb)) != SB_OK) return rc;
+    if (d->YS && (rc = oc->add(d->YS, v->offAS, fb)) != SB_OK) return rc;
+    if (d->sigmaX && (rc = oc->add(d->sigmaX, v->sigmaR, fb)) != SB_OK) return rc;
+    if (d->sigmaY && (rc = oc->add(d->sigmaY, v->sigmaA, fb)) != SB_OK) return rc;
     return SB_OK;
 }
 
@@ -1415,5 +1416,5 @@ extern "C" int sb_cullls(sb_context* c, const sb_cullls_params* p, sb_cullls_dat
                 return r;
             return SB_OK;
         },
-        [&](const CullDev* v) { return cullls_stage_out(c, p, d, v); });
+        [&](OutCopies* oc, const CullDev* v) { return cullls_stage_out(oc, p, d, v); });
 }

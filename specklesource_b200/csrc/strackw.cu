@@ -909,23 +909,25 @@ extern "C" int sb_strackw(sb_context* c, const sb_track_params* p, const sb_imag
     float* dC = (float*)sb_ctx_buf(c, "corr", sizeof(float) * n, &e);
     uint8_t* dT = (uint8_t*)sb_ctx_buf(c, "type", n, &e);
     unsigned long long* dst = (unsigned long long*)sb_ctx_buf(c, "w_stats", 4 * sizeof(unsigned long long), &e);
-    double* dB = (double*)sb_ctx_buf(c, "w_B", sizeof(double) * W_OSW * W_N1, &e);
+    // the real oversampling kernel of the 21 -> 336 symmetric zero pad
+    const double* dB = (const double*)sb_table(c, "w_B", [] {
+        std::vector<double> B(W_OSW * W_N1);
+        for (int nn = 0; nn < W_OSW; ++nn)
+            for (int t = 0; t < W_N1; ++t) {
+                const int d = (nn + (W_N1 * W_NOVER) / 2 - W_NOVER * 2) - W_NOVER * t;
+                double v = 1.0;
+                for (int f = 1; f <= W_NFAST / 2; ++f)
+                    v += 2.0 * cos(2.0 * 3.14159265358979323846 * f * d / (W_N1 * W_NOVER));
+                B[nn * W_N1 + t] = v;
+            }
+        return B;
+    });
     if (!dplan || !dlist || !dR || !dA || !dC || !dT || !dst || !dB)
         return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
     if (nl) {
         CKW(cudaMemcpyAsync(dplan, plan.data(), sizeof(int4) * nl, cudaMemcpyHostToDevice, c->stream), "plan");
         CKW(cudaMemcpyAsync(dlist, list.data(), sizeof(int) * nl, cudaMemcpyHostToDevice, c->stream), "list");
     }
-    // the real oversampling kernel of the 21 -> 336 symmetric zero pad
-    std::vector<double> B(W_OSW * W_N1);
-    for (int nn = 0; nn < W_OSW; ++nn)
-        for (int t = 0; t < W_N1; ++t) {
-            const int d = (nn + (W_N1 * W_NOVER) / 2 - W_NOVER * 2) - W_NOVER * t;
-            double v = 1.0;
-            for (int f = 1; f <= W_NFAST / 2; ++f) v += 2.0 * cos(2.0 * 3.14159265358979323846 * f * d / (W_N1 * W_NOVER));
-            B[nn * W_N1 + t] = v;
-        }
-    CKW(cudaMemcpyAsync(dB, B.data(), sizeof(double) * B.size(), cudaMemcpyHostToDevice, c->stream), "B");
     CKW(cudaMemsetAsync(dst, 0, 4 * sizeof(unsigned long long), c->stream), "memset");
     cudaEventRecord(c->ev[1], c->stream);
     strackw_init_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(dR, dA, dC, dT, n);
@@ -955,16 +957,16 @@ extern "C" int sb_strackw(sb_context* c, const sb_track_params* p, const sb_imag
         cudaEventRecord(c->sev[1], c->stream);
     }
     cudaEventRecord(c->ev[2], c->stream);
-    const int od = out->onDevice;
-    const cudaMemcpyKind k = od ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CKW(cudaMemcpyAsync(out->offR, dR, sizeof(float) * n, k, c->stream), "out");
-    CKW(cudaMemcpyAsync(out->offA, dA, sizeof(float) * n, k, c->stream), "out");
-    CKW(cudaMemcpyAsync(out->corr, dC, sizeof(float) * n, k, c->stream), "out");
-    CKW(cudaMemcpyAsync(out->type, dT, n, k, c->stream), "out");
+    const bool od = out->onDevice != 0;
+    OutCopies oc(c);
+    if ((rc = oc.add(out->offR, dR, sizeof(float) * n, od)) != SB_OK) return rc;
+    if ((rc = oc.add(out->offA, dA, sizeof(float) * n, od)) != SB_OK) return rc;
+    if ((rc = oc.add(out->corr, dC, sizeof(float) * n, od)) != SB_OK) return rc;
+    if ((rc = oc.add(out->type, dT, n, od)) != SB_OK) return rc;
     unsigned long long st[4];
-    CKW(cudaMemcpyAsync(st, dst, sizeof(st), cudaMemcpyDeviceToHost, c->stream), "stats");
+    if ((rc = oc.add(st, dst, sizeof(st))) != SB_OK) return rc;
     cudaEventRecord(c->ev[3], c->stream);
-    CKW(cudaStreamSynchronize(c->stream), "strackw");
+    if ((rc = oc.finish("strackw")) != SB_OK) return rc;
     out->nComplex = 0;
     out->nAmp = (int64_t)st[0];
     out->nAmpL = 0;
