@@ -51,7 +51,7 @@ struct AmChunk {
     float2* R;        // 2 x N x Ws, azimuth doubled
     float2* z;        // N x N (a1, a2), then row spectra
     float2* T;        // N x corr_ts(N)
-    float* mag;       // N x N |c| (over F and R, which are spent by then)
+    float* mag;       // N x N |c|
     double* part;     // N/4 x 5 sums of am_detect
     double* pw;       // N/8 x 2 powers of am_fwd
     AmMoments* mom;
@@ -370,8 +370,12 @@ __global__ void __launch_bounds__(128) am_peak_kernel(AmChunk c)
     }
 }
 
-// Planes in flight (serve.py's memory estimate uses the same figure).
-constexpr size_t AM_CHUNK_BYTES = (size_t)512 << 20;
+// Planes in flight: nine planes of Ws x Ws complex values for two points per SM
+// (87 MB at window 64, 349 MB at 128), the figure serve.py admits jobs by, in
+// which the 64 Ws^2 bytes of a point leave room for 330 points.  The tries of a
+// 1024 x 2048 pair at windows 64 and 128 take 5.8 ms; four times that would
+// give 5.1, but jobs that a server's budget now admits would no longer fit.
+static size_t am_chunk_bytes(int numSM, int Ws) { return (size_t)2 * numSM * sizeof(float2) * 9 * Ws * Ws; }
 
 template <int WS>
 struct AmRun {
@@ -388,11 +392,14 @@ struct AmRun {
             return p;
         };
         const size_t nn = (size_t)N * N;
-        c.F = (float2*)take(sizeof(float2) * n * 2 * WS * WS);
-        c.R = (float2*)take(sizeof(float2) * n * 2 * N * WS);
-        c.mag = (float*)c.F;
+        // what a step is done with makes room for a later one: F, then z, then
+        // mag; R, then T
         c.z = (float2*)take(sizeof(float2) * n * nn);
-        c.T = (float2*)take(sizeof(float2) * n * N * corr_ts(N));
+        c.F = c.z;
+        c.mag = (float*)c.z;
+        c.R = (float2*)take(sizeof(float2) * n * 2 * N * WS);
+        c.T = c.R;
+        static_assert(corr_ts(N) <= 2 * WS, "T fits over R");
         c.part = (double*)take(sizeof(double) * n * (N / 4) * 5);
         c.pw = (double*)take(sizeof(double) * n * (N / 8) * 2);
         c.best = (unsigned long long*)take(sizeof(unsigned long long) * n * (N / 16));
@@ -463,7 +470,8 @@ struct AmRun {
         if (!c.twW || !c.twN) return sb_ctx_fail(ctx, SB_ERR_NOMEM, "table allocation failed");
         double* dop;
         const size_t one = layout(c, 16, nullptr, &dop) / 16 + 1;
-        int B = (int)(AM_CHUNK_BYTES / one);
+        int B = (int)(am_chunk_bytes(ctx->numSM, WS) / one);
+        B = B < 16 ? 16 : B;
         const int chunks = (cnt + B - 1) / B;
         B = (cnt + chunks - 1) / chunks;  // equal chunks: no short last one
         char* base = (char*)sb_ctx_buf(ctx, "ampScratch", layout(c, B, nullptr, &dop), &e);

@@ -628,13 +628,19 @@ __global__ void strackw_init_kernel(float* offR, float* offA, float* corr, uint8
     type[k] = SB_BAD;
 }
 
-// Planes in flight: large chunks, so that each launch is many waves of CTAs.
-// The 2000 x 4000 pair at W = 224 takes 48.0 ms with 128 MB of planes (about
-// L2), 36.0 with 512 MB, 30.0 with 1 GB and 28.6 with 2 GB: the kernels are
-// short of instruction issue and shared-memory bandwidth, not of DRAM
-// (10 to 45 % of its rate), so staying in L2 does not pay for short launches.
-// serve.py's memory estimate uses the same figure.
-constexpr size_t SW_CHUNK_BYTES = (size_t)1 << 30;
+// Planes in flight at a margin of e samples: two points' per SM of the working
+// set of one (window pair, upsampled pair, correlation), the figure serve.py
+// admits jobs by.  Large launches matter more than L2 (126 MB): the kernels are
+// short of instruction issue and shared-memory bandwidth, not of DRAM (10 to
+// 45 % of its rate).  At W = 224 (2 GB) the 2000 x 4000 pair takes 27.7 ms,
+// with 512 MB 36, with 128 MB 48.  At W = 64 (220 MB, 840 points) the 1024 x
+// 2048 pair takes 1.58 ms; four times that would give 1.38, but jobs that a
+// server's budget now admits would no longer fit.
+static size_t sw_chunk_bytes(int numSM, int W, int e)
+{
+    const size_t N = 2 * W, L = 4 * e + 1;
+    return (size_t)2 * numSM * sizeof(float2) * (3 * W * W + 3 * N * N + 2 * N * L + 3 * L * L);
+}
 
 // Workspace of a chunk, carved from one buffer; base null: returns its size.
 struct SwSpace {
@@ -658,17 +664,20 @@ struct SwRun {
     {
         const size_t L = 4 * a.e + 1, c2 = N - 4 * a.e, NN = (size_t)N * N;
         SwSpace s{base};
-        a.xv = s.take<float2>((size_t)n * 2 * W * W);
+        // what a step is done with makes room for a later one: xv, then A1, then
+        // T; H, then Z, then ncc (L <= N)
+        const size_t xt = (size_t)L * corr_ts(N) > 2 * W * W ? (size_t)L * corr_ts(N) : 2 * W * W;
+        a.xv = s.take<float2>(n * xt);
+        a.A1 = reinterpret_cast<float*>(a.xv);
+        a.T = a.xv;
         a.H = s.take<float>((size_t)n * 2 * NN);
         a.Z = reinterpret_cast<float2*>(a.H);
-        a.A1 = s.take<float>((size_t)n * NN);
+        a.ncc = reinterpret_cast<double*>(a.H);
         a.A2 = s.take<float>((size_t)n * c2 * c2);
         a.seg = s.take<double>((size_t)n * (N / W_SEG) * 2 * N);
         a.part = s.take<double>((size_t)n * (N / W_SEG) * 3);
         a.mom = s.take<SwMoments>(n);
         a.norm = s.take<double>((size_t)n * L * L);
-        a.T = s.take<float2>((size_t)n * L * corr_ts(N));
-        a.ncc = s.take<double>((size_t)n * L * L);
         a.bestV = s.take<double>((size_t)n * (L + 15) / 16 + n);
         a.bestE = s.take<int>((size_t)n * (L + 15) / 16 + n);
         *dop = s.take<double>(dop_scratch_doubles<W>(n));
@@ -747,7 +756,7 @@ static int run_sw(sb_context* c, SwArgs a, int nl)
     int* az;
     SwArgs probe = a;
     const size_t one = SwRun<W>::layout(probe, 16, nullptr, &dop, &az) / 16 + 1;
-    int B = (int)(SW_CHUNK_BYTES / one);
+    int B = (int)(sw_chunk_bytes(c->numSM, W, a.e) / one);
     B = B < 16 ? 16 : B;
     const int chunks = (nl + B - 1) / B;
     B = (nl + chunks - 1) / chunks;  // equal chunks: no short last one

@@ -33,10 +33,11 @@ _STRACK_POINT_BYTES = 20 + 80 + 16 + 160 + 17 + 64
 # most one list chunk (kPeakChunk in csrc/capi.cu)
 _PEAK_JOB_BYTES = 960
 _PEAK_CHUNK = 1 << 19
-# planes in flight of the amplitude tries from window 48 up and of strackw
-# (AM_CHUNK_BYTES, csrc/strack_amp.cu; SW_CHUNK_BYTES, csrc/strackw.cu)
-_AMP_CHUNK = 512 << 20
-_SW_CHUNK = 1 << 30
+# per-CTA workspaces (float2 elements), sized like the kernels' own
+_AMP_SCRATCH = {16: 3 * 16 * 16 + 32 * 32 * 3 // 2, 24: 3 * 24 * 24 + 48 * 48 * 3 // 2,
+                32: 3 * 32 * 32 + 64 * 64 * 3 // 2, 48: 3 * 48 * 48 + 96 * 96 * 3 // 2,
+                64: 3 * 64 * 64 + 128 * 128 * 3 // 2, 96: 3 * 96 * 96 + 192 * 192 * 3 // 2,
+                128: 3 * 128 * 128 + 256 * 256 * 3 // 2}
 
 
 @dataclass
@@ -72,23 +73,21 @@ def job_device_bytes(job, num_sm=148):
     p = job.params
     n = int(p.nR) * int(p.nA)
     b = _image_bytes(job.img1) + _image_bytes(job.img2)
+    ctas = 2 * num_sm
     if job.kind == "strack":
         b += n * _STRACK_POINT_BYTES
         if not getattr(p, "gaussFlag", 0):
             b += min(n, _PEAK_CHUNK) * _PEAK_JOB_BYTES
         if p.maxTries > 0:
             wa = int(p.wRa)
-            ws = wa if p.maxTries < 2 else 2 * wa  # the larger try's planes (one buffer)
-            if ws > 32:
-                point = 96 * ws * ws + 256 * ws + 8192
-                b += min(n * point, max(_AMP_CHUNK, 16 * point))
+            b += ctas * 8 * _AMP_SCRATCH.get(wa, _AMP_SCRATCH[128])
+            if p.maxTries > 1 and 2 * wa in _AMP_SCRATCH:
+                b += ctas * 8 * _AMP_SCRATCH[2 * wa]
     else:
         W = int(p.wRa)
         N = 2 * W
         L = 4 * (int(p.edgePadR) + 5) + 1
-        # planes of a chunk of points (strackw.cu)
-        point = 21 * N * N + 16 * L * L + 8 * L * (N // 2 + 8) + 4096
-        b += n * 40 + min(n * point, max(_SW_CHUNK, 16 * point))
+        b += n * 40 + ctas * 8 * (3 * W * W + 3 * N * N + 2 * N * L + 3 * L * L)
     if job.cull is not None:
         b += n * 64
     return int(b)
