@@ -34,6 +34,7 @@
 #include <stdint.h>
 
 #include "capi_internal.h"
+#include "chain.cuh"
 
 namespace sbk {
 
@@ -78,6 +79,7 @@ struct CullArgs {
 
 __global__ void cull_prepass_kernel(CullArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA) return;
     if (a.corr[k] < a.corrThresh) {  // cullSTData.c:38-43
@@ -350,6 +352,7 @@ __device__ __forceinline__ void warp_append(bool yes, int v, int* list, unsigned
 template <bool SLOW>
 __global__ void __launch_bounds__(256) cull_fix_first_kernel(FixArgs a)
 {
+    chain_begin();
     if (*a.stop) return;  // uniform
     const int j = blockIdx.x * 32 + (threadIdx.x & 31), i = blockIdx.y * 8 + (threadIdx.x >> 5);
     bool cull = false, ok = false;
@@ -419,12 +422,14 @@ __device__ __forceinline__ void fix_apply_list(const FixArgs& a, int step, int w
 template <bool SLOW>
 __global__ void __launch_bounds__(256) cull_fix_list_kernel(FixArgs a, int step)
 {
+    chain_begin();
     if (*a.stop) return;
     fix_decide_list<SLOW>(a, step, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 __global__ void __launch_bounds__(256) cull_fix_apply_kernel(FixArgs a, int step)
 {
+    chain_begin();
     if (*a.stop) return;
     fix_apply_list(a, step, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
 }
@@ -435,6 +440,7 @@ __global__ void __launch_bounds__(256) cull_fix_apply_kernel(FixArgs a, int step
 template <bool SLOW>
 __global__ void __cluster_dims__(kFixCluster, 1, 1) __launch_bounds__(1024) cull_fix_tail_kernel(FixArgs a, int step)
 {
+    chain_begin();
     if (*a.stop) return;
     auto sync = [] {
         __threadfence();
@@ -456,6 +462,7 @@ __global__ void __cluster_dims__(kFixCluster, 1, 1) __launch_bounds__(1024) cull
 __global__ void cull_apply_kernel(float* offR, float* offA, const uint8_t* c, long long n,
                                   unsigned long long* nCulled, const int* stop)
 {
+    chain_begin();
     if (*stop) return;
     unsigned long long k = 0;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
@@ -564,6 +571,7 @@ struct StatsArgs {
 constexpr int ST_BOX = 4;  // 9 x 9, cullStats.c:38-39
 __global__ void __launch_bounds__(256) cull_stats_kernel(StatsArgs a)
 {
+    chain_begin();
     constexpr int TX = 32, TY = 8, SX = TX + 2 * ST_BOX, SY = TY + 2 * ST_BOX;
     __shared__ float2 tile[SY][SX];
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
@@ -684,6 +692,7 @@ __device__ __forceinline__ float sweight(int m, int s)
 
 __global__ void cull_smooth_kernel(SmoothArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA) return;
     const int i = k / a.nR, j = k % a.nR;
@@ -721,6 +730,7 @@ __global__ void cull_smooth_kernel(SmoothArgs a)
 // per valid point.
 __global__ void cullls_smooth_kernel(SmoothArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA) return;
     const int i = k / a.nR, j = k % a.nR;
@@ -755,6 +765,7 @@ __global__ void cullls_smooth_kernel(SmoothArgs a)
 __global__ void cullls_count_kernel(const float* offR, const float* offA, const uint8_t* type, unsigned noDataMask,
                                     long long n, unsigned long long* cnt)
 {
+    chain_begin();
     unsigned long long nv = 0, nd = 0;
     for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n;
          p += (long long)gridDim.x * blockDim.x) {
@@ -773,6 +784,7 @@ __global__ void cullls_count_kernel(const float* offR, const float* offA, const 
 
 __global__ void cull_sim_kernel(float* offR, float* offA, const float* simR, const float* simA, int n, float sign)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     // cullst.c:109-121 with its local LARGEINT = -2e9: offA < 2e9 + 1
@@ -830,6 +842,7 @@ struct IslandArgs {
 
 __global__ void isl_init_kernel(IslandArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA) return;
     const float minRegion = (float)(-2000000000 + 1000);  // cullIslands.c:62
@@ -840,6 +853,7 @@ __global__ void isl_init_kernel(IslandArgs a)
 
 __global__ void isl_union_kernel(IslandArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA || a.par[k] < 0) return;
     const int i = k / a.nR, j = k % a.nR;
@@ -853,6 +867,7 @@ __global__ void isl_union_kernel(IslandArgs a)
 
 __global__ void isl_flatten_kernel(IslandArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA || a.par[k] < 0) return;
     int r = k;
@@ -870,6 +885,7 @@ __global__ void isl_flatten_kernel(IslandArgs a)
 
 __global__ void isl_cull_kernel(IslandArgs a)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nR * a.nA || a.par[k] < 0) return;
     const int r = a.par[k];
@@ -1081,11 +1097,11 @@ cudaError_t launch_fix_pass(sb_context* c, const FixArgs& f)
     cudaStream_t s = c->stream;
     const dim3 grid((f.nR + 31) / 32, (f.nA + 7) / 8);
     const int wide = c->numSM * 8;
-    cull_fix_first_kernel<SLOW><<<grid, 256, 0, s>>>(f);
-    cull_fix_apply_kernel<<<wide, 256, 0, s>>>(f, 0);
-    cull_fix_list_kernel<SLOW><<<wide, 256, 0, s>>>(f, 1);
-    cull_fix_apply_kernel<<<wide, 256, 0, s>>>(f, 1);
-    cull_fix_tail_kernel<SLOW><<<kFixCluster, 1024, 0, s>>>(f, 2);
+    chain(cull_fix_first_kernel<SLOW>, grid, 256, 0, s, f);
+    chain(cull_fix_apply_kernel, wide, 256, 0, s, f, 0);
+    chain(cull_fix_list_kernel<SLOW>, wide, 256, 0, s, f, 1);
+    chain(cull_fix_apply_kernel, wide, 256, 0, s, f, 1);
+    chain(cull_fix_tail_kernel<SLOW>, kFixCluster, 1024, 0, s, f, 2);
     c->launches += 5;
     return cudaGetLastError();
 }
@@ -1111,7 +1127,7 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
     a.progress = progress;
     cudaStream_t s = c->stream;
     if (p.prepass) {  // of later passes: nothing left to change
-        cull_prepass_kernel<<<(int)((n + 255) / 256), 256, 0, s>>>(a);
+        chain(cull_prepass_kernel, (int)((n + 255) / 256), 256, 0, s, a);
         CKC(cudaGetLastError(), "cull_prepass");
         c->launches++;
     }
@@ -1161,7 +1177,7 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
             CKC(f.slowType ? launch_fix_pass<true>(c, f) : launch_fix_pass<false>(c, f), "cull_fix");
             long long ab = (n + 255) / 256;
             if (ab > (long long)c->numSM * 16) ab = (long long)c->numSM * 16;
-            cull_apply_kernel<<<(int)ab, 256, 0, s>>>(v->offR, v->offA, C, n, culled + k, f.stop);
+            chain(cull_apply_kernel, (int)ab, 256, 0, s, v->offR, v->offA, C, n, culled + k, f.stop);
             CKC(cudaGetLastError(), "cull_apply");
             c->launches++;
         }
@@ -1181,7 +1197,7 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
 int run_stats(sb_context* c, const CullJob& p, const CullDev* v)
 {
     StatsArgs a{v->offR, v->offA, v->sigmaR, v->sigmaA, p.nR, p.nA, p.qvar};
-    cull_stats_kernel<<<dim3((p.nR + 31) / 32, (p.nA + 7) / 8), 256, 0, c->stream>>>(a);
+    chain(cull_stats_kernel, dim3((p.nR + 31) / 32, (p.nA + 7) / 8), 256, 0, c->stream, a);
     c->launches++;
     return sb_ctx_cuda(c, cudaGetLastError(), "cull_stats");
 }
@@ -1191,9 +1207,9 @@ int run_smooth(sb_context* c, const CullJob& p, const CullDev* v)
     const int n = p.nR * p.nA;
     SmoothArgs a{v->offR, v->offA, v->type, v->sigmaR, v->sigmaA, v->offRS, v->offAS, p.nR, p.nA, p.sR, p.sA};
     if (p.lsSmooth)
-        cullls_smooth_kernel<<<(n + 127) / 128, 128, 0, c->stream>>>(a);
+        chain(cullls_smooth_kernel, (n + 127) / 128, 128, 0, c->stream, a);
     else
-        cull_smooth_kernel<<<(n + 127) / 128, 128, 0, c->stream>>>(a);
+        chain(cull_smooth_kernel, (n + 127) / 128, 128, 0, c->stream, a);
     c->launches++;
     return sb_ctx_cuda(c, cudaGetLastError(), "cull_smooth");
 }
@@ -1223,10 +1239,10 @@ int run_islands(sb_context* c, const CullJob& p, const CullDev* v, int64_t* nIsl
     CKC(cudaMemsetAsync(a.lastRoot, 0xff, sizeof(int), s), "memset");
     CKC(cudaMemsetAsync(a.counts, 0, 2 * sizeof(unsigned long long), s), "memset");
     const int g = (n + 255) / 256;
-    isl_init_kernel<<<g, 256, 0, s>>>(a);
-    isl_union_kernel<<<g, 256, 0, s>>>(a);
-    isl_flatten_kernel<<<g, 256, 0, s>>>(a);
-    isl_cull_kernel<<<g, 256, 0, s>>>(a);
+    chain(isl_init_kernel, g, 256, 0, s, a);
+    chain(isl_union_kernel, g, 256, 0, s, a);
+    chain(isl_flatten_kernel, g, 256, 0, s, a);
+    chain(isl_cull_kernel, g, 256, 0, s, a);
     c->launches += 4;
     CKC(cudaGetLastError(), "cull_islands");
     unsigned long long cnt[2];
@@ -1240,7 +1256,7 @@ int run_islands(sb_context* c, const CullJob& p, const CullDev* v, int64_t* nIsl
 int run_sim(sb_context* c, const CullJob& p, const CullDev* v, float sign)
 {
     const int n = p.nR * p.nA;
-    cull_sim_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(v->offR, v->offA, v->simR, v->simA, n, sign);
+    chain(cull_sim_kernel, (n + 255) / 256, 256, 0, c->stream, v->offR, v->offA, v->simR, v->simA, n, sign);
     c->launches++;
     return sb_ctx_cuda(c, cudaGetLastError(), "cull_sim");
 }
@@ -1345,7 +1361,7 @@ int run_ls_counts(sb_context* c, const sb_cullls_params* p, const CullDev* v, sb
     CKC(cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), s), "memset");
     long long blocks = (n + 255) / 256;
     if (blocks > (long long)c->numSM * 16) blocks = (long long)c->numSM * 16;
-    cullls_count_kernel<<<(int)blocks, 256, 0, s>>>(v->offR, v->offA, v->type, p->noDataMask, n, cnt);
+    chain(cullls_count_kernel, (int)blocks, 256, 0, s, v->offR, v->offA, v->type, p->noDataMask, n, cnt);
     CKC(cudaGetLastError(), "cullls_count");
     c->launches++;
     unsigned long long h[2];

@@ -1,6 +1,7 @@
 // partition.cu -- ordered (stable) partition by key; see partition.h.
 #include <cuda_runtime.h>
 
+#include "chain.cuh"
 #include "partition.h"
 
 namespace sbk {
@@ -17,6 +18,7 @@ size_t partition_keyoff_at(int n, int K) { return (size_t)2 * part_tiles(n) * K;
 __global__ void __launch_bounds__(PART_TILE) part_count_kernel(const int* __restrict__ key, int n, int K,
                                                                int* __restrict__ tileCnt)
 {
+    chain_begin();
     __shared__ int h[PART_KMAX];
     if (threadIdx.x < PART_KMAX) h[threadIdx.x] = 0;
     __syncthreads();
@@ -31,6 +33,7 @@ __global__ void __launch_bounds__(PART_TILE) part_count_kernel(const int* __rest
 __global__ void __launch_bounds__(1024) part_scan_kernel(const int* __restrict__ tileCnt, int nTiles, int K,
                                                          int* __restrict__ tileOff, int* __restrict__ keyOff)
 {
+    chain_begin();
     __shared__ int ws[32];
     __shared__ int total;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -75,6 +78,7 @@ __global__ void __launch_bounds__(PART_TILE) part_write_kernel(const int* __rest
                                                                const int* __restrict__ tileOff,
                                                                const int* __restrict__ keyOff, int* __restrict__ out)
 {
+    chain_begin();
     __shared__ int wc[PART_KMAX][32];  // [key][warp]: count, then exclusive prefix over warps
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int e = tid; e < PART_KMAX * 32; e += PART_TILE) wc[e / 32][e % 32] = 0;
@@ -111,9 +115,9 @@ cudaError_t launch_partition(const int* key, const int* val, int n, int K, int* 
     int* tileOff = scratch + (size_t)nt * K;
     int* keyOff = scratch + partition_keyoff_at(n, K);
     if (nt == 0) return cudaMemsetAsync(keyOff, 0, sizeof(int) * (K + 1), st);
-    part_count_kernel<<<nt, PART_TILE, 0, st>>>(key, n, K, tileCnt);
-    part_scan_kernel<<<1, 1024, 0, st>>>(tileCnt, nt, K, tileOff, keyOff);
-    part_write_kernel<<<nt, PART_TILE, 0, st>>>(key, val, n, K, tileOff, keyOff, out);
+    chain(part_count_kernel, nt, PART_TILE, 0, st, key, n, K, tileCnt);
+    chain(part_scan_kernel, 1, 1024, 0, st, tileCnt, nt, K, tileOff, keyOff);
+    chain(part_write_kernel, nt, PART_TILE, 0, st, key, val, n, K, tileOff, keyOff, out);
     return cudaGetLastError();
 }
 

@@ -73,6 +73,7 @@ struct AmCfg {
 
 __global__ void am_prep_kernel(AmChunk c)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= c.win.n) return;
     const AmpArgs& a = c.a;
@@ -91,6 +92,7 @@ __global__ void am_prep_kernel(AmChunk c)
 template <int WS, bool F32>
 __global__ void __launch_bounds__(128) am_rows_kernel(AmChunk c)
 {
+    chain_begin();
     using C = AmCfg<WS>;
     constexpr int G = C::G, NT = C::NT, TILES = WS / G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(128) am_rows_kernel(AmChunk c)
 template <int WS>
 __global__ void __launch_bounds__(128) am_cols_kernel(AmChunk c)
 {
+    chain_begin();
     using C = AmCfg<WS>;
     constexpr int G = C::G, NT = C::NT, TILES = WS / G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -135,6 +138,7 @@ __global__ void __launch_bounds__(128) am_cols_kernel(AmChunk c)
 template <int WS>
 __global__ void __launch_bounds__(128) am_detect_kernel(AmChunk c)
 {
+    chain_begin();
     using C = AmCfg<WS>;
     constexpr int N = C::N, G = C::G, H = G / 2, NT = C::NT, TILES = N / H;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(128) am_detect_kernel(AmChunk c)
 template <int WS>
 __global__ void am_moments_kernel(AmChunk c)
 {
+    chain_begin();
     constexpr int N = 2 * WS, TILES = N / 4;
     const int pt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (pt >= c.win.n) return;
@@ -197,6 +202,7 @@ __global__ void am_moments_kernel(AmChunk c)
 template <int WS>
 __global__ void __launch_bounds__(128) am_fwd_kernel(AmChunk c)
 {
+    chain_begin();
     using C = AmCfg<WS>;
     constexpr int N = C::N, G = C::G, NT = C::NT, TILES = N / G;
     __shared__ double red[(NT / 32 + 1) * 2];
@@ -230,6 +236,7 @@ __global__ void __launch_bounds__(128) am_fwd_kernel(AmChunk c)
 template <int WS>
 __global__ void __launch_bounds__(ColCfg<2 * WS>::NT) am_corr_kernel(AmChunk c)
 {
+    chain_begin();
     constexpr int N = 2 * WS;
     using C = ColCfg<N>;
     const int pt = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
@@ -242,6 +249,7 @@ __global__ void __launch_bounds__(ColCfg<2 * WS>::NT) am_corr_kernel(AmChunk c)
 template <int WS>
 __global__ void __launch_bounds__(128) am_mag_kernel(AmChunk c)
 {
+    chain_begin();
     using C = AmCfg<WS>;
     constexpr int N = C::N, G = C::G, NT = C::NT, TS = corr_ts(N), TILES = N / (2 * G);
     __shared__ unsigned long long sc[NT / 32];
@@ -273,6 +281,7 @@ __global__ void __launch_bounds__(128) am_mag_kernel(AmChunk c)
 template <int WS, bool GAUSS>
 __global__ void __launch_bounds__(128) am_peak_kernel(AmChunk c)
 {
+    chain_begin();
     constexpr int N = 2 * WS, NT = 128;
     __shared__ __align__(16) float2 osd[OSW * NFAST / 2 + 16];
     __shared__ float2 Yb[NFAST * NFAST], T[NFAST * OSW];
@@ -373,8 +382,9 @@ __global__ void __launch_bounds__(128) am_peak_kernel(AmChunk c)
 // Planes in flight: nine planes of Ws x Ws complex values for two points per SM
 // (87 MB at window 64, 349 MB at 128), the figure serve.py admits jobs by, in
 // which the 64 Ws^2 bytes of a point leave room for 330 points.  The tries of a
-// 1024 x 2048 pair at windows 64 and 128 take 5.8 ms; four times that would
-// give 5.1, but jobs that a server's budget now admits would no longer fit.
+// 1024 x 2048 pair at windows 64 and 128 take 5.8 ms (plain launches), 6.6 with
+// half, 5.1 with four times that, where jobs that a server's budget admits
+// would no longer fit.
 static size_t am_chunk_bytes(int numSM, int Ws) { return (size_t)2 * numSM * sizeof(float2) * 9 * Ws * Ws; }
 
 template <int WS>
@@ -427,7 +437,7 @@ struct AmRun {
     static cudaError_t chunk(const AmChunk& c, double* dop, cudaStream_t st, int64_t* launches)
     {
         const int n = c.win.n;
-        am_prep_kernel<<<(n + 127) / 128, 128, 0, st>>>(c);
+        chain(am_prep_kernel, (n + 127) / 128, 128, 0, st, c);
         *launches += 9;
         if (c.a.noComplex != 0 && c.a.stage == 1) {
             const cudaError_t e = launch_dop<WS>(c.win, c.a.wA, dop, c.az, st);
@@ -436,19 +446,19 @@ struct AmRun {
         }
         const int g = n * 2 * (WS / C::G);
         if (c.win.sampleType == SB_CFLOAT32)
-            am_rows_kernel<WS, true><<<g, C::NT, C::smRows, st>>>(c);
+            chain(am_rows_kernel<WS, true>, g, C::NT, C::smRows, st, c);
         else
-            am_rows_kernel<WS, false><<<g, C::NT, C::smRows, st>>>(c);
-        am_cols_kernel<WS><<<g, C::NT, C::smCols, st>>>(c);
-        am_detect_kernel<WS><<<n * (N / 4), C::NT, C::smDetect, st>>>(c);
-        am_moments_kernel<WS><<<(n + 3) / 4, 128, 0, st>>>(c);
-        am_fwd_kernel<WS><<<n * (N / C::G), C::NT, C::smFwd, st>>>(c);
-        am_corr_kernel<WS><<<n * ColCfg<N>::TILES, ColCfg<N>::NT, ColCfg<N>::smem, st>>>(c);
-        am_mag_kernel<WS><<<n * (N / (2 * C::G)), C::NT, C::smFwd, st>>>(c);
+            chain(am_rows_kernel<WS, false>, g, C::NT, C::smRows, st, c);
+        chain(am_cols_kernel<WS>, g, C::NT, C::smCols, st, c);
+        chain(am_detect_kernel<WS>, n * (N / 4), C::NT, C::smDetect, st, c);
+        chain(am_moments_kernel<WS>, (n + 3) / 4, 128, 0, st, c);
+        chain(am_fwd_kernel<WS>, n * (N / C::G), C::NT, C::smFwd, st, c);
+        chain(am_corr_kernel<WS>, n * ColCfg<N>::TILES, ColCfg<N>::NT, ColCfg<N>::smem, st, c);
+        chain(am_mag_kernel<WS>, n * (N / (2 * C::G)), C::NT, C::smFwd, st, c);
         if (c.a.gauss)
-            am_peak_kernel<WS, true><<<n, 128, 0, st>>>(c);
+            chain(am_peak_kernel<WS, true>, n, 128, 0, st, c);
         else
-            am_peak_kernel<WS, false><<<n, 128, 0, st>>>(c);
+            chain(am_peak_kernel<WS, false>, n, 128, 0, st, c);
         return cudaGetLastError();
     }
 

@@ -27,6 +27,7 @@
 
 #include <type_traits>
 
+#include "chain.cuh"
 #include "strack_device.cuh"
 #include "strack_kernels.h"
 #include "warp_lines.cuh"
@@ -106,6 +107,7 @@ __device__ __forceinline__ float2 amps_decode(typename std::conditional<F32, uin
 template <int WS, int NT, bool F32, bool GAUSS>
 __global__ void __launch_bounds__(NT, (WS == 32 ? 3 : WS == 24 ? 3 : 8)) strack_amps_kernel(AmpArgs a)
 {
+    chain_begin();
     using M = AmpsSmem<WS, NT>;
     constexpr int N = M::N, RS = M::RS, RZ = M::RZ, S = M::S, NW = NT / 32;
     using LW = sbfft::WarpLines<WS, 8>;
@@ -497,7 +499,7 @@ static cudaError_t launch_amps_t(const AmpArgs& a, int nCta, cudaStream_t st)
     cudaError_t e = cudaFuncSetAttribute(strack_amps_kernel<WS, NT, F32, GAUSS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    strack_amps_kernel<WS, NT, F32, GAUSS><<<nCta, NT, sm, st>>>(a);
+    chain(strack_amps_kernel<WS, NT, F32, GAUSS>, nCta, NT, sm, st, a);
     return cudaGetLastError();
 }
 

@@ -23,6 +23,7 @@
 
 #include <type_traits>
 
+#include "chain.cuh"
 #include "strack_device.cuh"
 #include "strack_kernels.h"
 #include "warp_lines.cuh"
@@ -310,6 +311,7 @@ __host__ __device__ constexpr int cmplx_min_ctas(int W, int NT)
 template <int W, int NT, bool F32, bool GAUSS>
 __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx_kernel(CmplxArgs a)
 {
+    chain_begin();
     using S = CmplxSmem<W, NT>;
     constexpr int RS = S::RS, IMG = S::IMG;
     constexpr int W2 = 2 * W;

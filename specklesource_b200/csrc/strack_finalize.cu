@@ -3,12 +3,14 @@
 // the .dr/.da/.cc/.azd/.mt grids (speckleTrack.c:300-323).
 #include <cuda_runtime.h>
 
+#include "chain.cuh"
 #include "strack_finalize.h"
 
 namespace sbk {
 
 __global__ void rec_init_kernel(PointRec* rec, int n)
 {
+    chain_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     PointRec r;
@@ -27,6 +29,7 @@ __global__ void rec_init_kernel(PointRec* rec, int n)
 __global__ void select_stage_kernel(const PointPlan* plan, const PointRec* rec, int n, WalkParams w, int stage,
                                     int* key)
 {
+    chain_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const WalkOut o = strack_walk(plan[p], rec[p], w);
@@ -38,6 +41,7 @@ __global__ void select_stage_kernel(const PointPlan* plan, const PointRec* rec, 
 // Single CTA: chunked block scan over the grid.
 __global__ void az_fill_kernel(const PointRec* rec, int n, int* azEff)
 {
+    chain_begin();
     __shared__ int carry;
     __shared__ int lastIdx[1024];
     if (threadIdx.x == 0) carry = 0;
@@ -69,6 +73,7 @@ __global__ void finalize_kernel(const PointPlan* plan, const PointRec* rec, int 
                                 float* offR, float* offA, float* corr, float* azd, uint8_t* type,
                                 unsigned long long* stats, const int* pairOf)
 {
+    chain_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     if (pairOf) stats += 8 * pairOf[p];  // batched calls: statistics per pair
@@ -113,6 +118,7 @@ __global__ void finalize_kernel(const PointPlan* plan, const PointRec* rec, int 
 // host.  key[p] = 0 for complex candidates, else -1.
 __global__ void plan_poly_kernel(PlanArgs a, PointPlan* plan, int* key)
 {
+    chain_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.nR * a.nA) return;
     const int i = p / a.nR, j = p % a.nR;
@@ -183,6 +189,7 @@ __device__ __forceinline__ int point_band(const PointPlan& pl, int W, int rows1,
 __global__ void band_key_kernel(const PointPlan* plan, const int* list, int n, int W, int rows1, int rows2, int nb,
                                 int* bandOf)
 {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) bandOf[i] = point_band(plan[list[i]], W, rows1, rows2, nb);
 }
@@ -192,7 +199,7 @@ cudaError_t launch_band_key(const PointPlan* plan, const int* list, int n, int W
 {
     if (nb < 1 || nb > SB_BANDS_MAX) return cudaErrorInvalidValue;
     if (n == 0) return cudaSuccess;
-    band_key_kernel<<<(n + 255) / 256, 256, 0, st>>>(plan, list, n, W, rows1, rows2, nb, bandOf);
+    chain(band_key_kernel, (n + 255) / 256, 256, 0, st, plan, list, n, W, rows1, rows2, nb, bandOf);
     return cudaGetLastError();
 }
 
@@ -209,7 +216,7 @@ cudaError_t launch_select(const PointPlan* plan, const PointRec* rec, int n, con
 }
 cudaError_t launch_az_fill(const PointRec* rec, int n, int* azEff, cudaStream_t st)
 {
-    az_fill_kernel<<<1, 1024, 0, st>>>(rec, n, azEff);
+    chain(az_fill_kernel, 1, 1024, 0, st, rec, n, azEff);
     return cudaGetLastError();
 }
 cudaError_t launch_finalize(const PointPlan* plan, const PointRec* rec, int n, const WalkParams& w, int scaleFactor,
@@ -217,8 +224,8 @@ cudaError_t launch_finalize(const PointPlan* plan, const PointRec* rec, int n, c
                             unsigned long long* stats, cudaStream_t st, const int* pairOf)
 {
     if (n <= 0) return cudaSuccess;
-    finalize_kernel<<<(n + 255) / 256, 256, 0, st>>>(plan, rec, n, w, scaleFactor, offR, offA, corr, azd, type,
-                                                     stats, pairOf);
+    chain(finalize_kernel, (n + 255) / 256, 256, 0, st, plan, rec, n, w, scaleFactor, offR, offA, corr, azd, type,
+          stats, pairOf);
     return cudaGetLastError();
 }
 

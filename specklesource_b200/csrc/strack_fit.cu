@@ -14,6 +14,7 @@
 // singular matrix does in the reference's solver.
 #include <cuda_runtime.h>
 
+#include "chain.cuh"
 #include "strack_device.cuh"
 #include "strack_fit.h"
 
@@ -134,6 +135,7 @@ __device__ double fit_sigma(const float* samp, int x0, int sub, unsigned mask)
 template <int LPF>
 __global__ void __launch_bounds__(128) strack_fit_kernel(FitArgs a)
 {
+    chain_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int sub = t % LPF, job = t / (2 * LPF), f = t / LPF & 1;
     const unsigned mask = (LPF == 32 ? 0xffffffffu : (1u << LPF) - 1u) << (threadIdx.x & 31 & ~(LPF - 1));
@@ -184,7 +186,7 @@ cudaError_t launch_strack_fit(const FitArgs& a, cudaStream_t st)
     if (a.nList <= 0) return cudaSuccess;
     constexpr int LPF = 4;
     const long long threads = 2LL * a.nList * LPF;
-    strack_fit_kernel<LPF><<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(a);
+    chain(strack_fit_kernel<LPF>, (unsigned)((threads + 127) / 128), 128, 0, st, a);
     return cudaGetLastError();
 }
 

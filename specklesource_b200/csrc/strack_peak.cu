@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "strack_device.cuh"
 #include "strack_kernels.h"
 
@@ -22,6 +23,7 @@ constexpr int kPeakWarps = 8;  // warps per CTA
 
 __global__ void __launch_bounds__(32 * kPeakWarps) strack_peak_kernel(PeakArgs a)
 {
+    chain_begin();
     __shared__ __align__(16) float osD[OSW * NFAST + 2 * 16];
     __shared__ __align__(16) float2 Yb[kPeakWarps][NFAST * NFAST];
     __shared__ __align__(16) float2 T[kPeakWarps][NFAST * OSW];
@@ -88,7 +90,7 @@ cudaError_t launch_strack_peak(const PeakArgs& a, int numSM, cudaStream_t st)
     long long blocks = ((long long)a.nList + kPeakWarps - 1) / kPeakWarps;
     const long long cap = (long long)numSM * 8;
     if (blocks > cap) blocks = cap;
-    strack_peak_kernel<<<(unsigned)blocks, 32 * kPeakWarps, 0, st>>>(a);
+    chain(strack_peak_kernel, (unsigned)blocks, 32 * kPeakWarps, 0, st, a);
     return cudaGetLastError();
 }
 

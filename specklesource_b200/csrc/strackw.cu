@@ -152,6 +152,7 @@ struct SwCfg {
 template <int W, bool F32>
 __global__ void __launch_bounds__(128) sw_cols_kernel(SwArgs a)
 {
+    chain_begin();
     using C = SwCfg<W>;
     constexpr int G = C::G, NT = C::NTW, TILES = W / G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -183,6 +184,7 @@ __global__ void __launch_bounds__(128) sw_cols_kernel(SwArgs a)
 template <int W, bool F32>
 __global__ void __launch_bounds__(128) sw_rows_kernel(SwArgs a, int hr0, int hr1, int pad)
 {
+    chain_begin();
     using C = SwCfg<W>;
     constexpr int N = C::N, G = C::G, NT = C::NTW, TILES = N / G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -253,6 +255,7 @@ __global__ void __launch_bounds__(128) sw_rows_kernel(SwArgs a, int hr0, int hr1
 template <int W, int TAPS>
 __global__ void __launch_bounds__(2 * W) sw_amps_kernel(SwArgs a)
 {
+    chain_begin();
     constexpr int N = 2 * W, NT = N;
     __shared__ double red[(NT / 32 + 1) * 3];
     const int pt = blockIdx.x / (N / W_SEG), sg = blockIdx.x % (N / W_SEG), j = threadIdx.x;
@@ -322,6 +325,7 @@ __global__ void __launch_bounds__(2 * W) sw_amps_kernel(SwArgs a)
 template <int W>
 __global__ void sw_reduce_kernel(SwArgs a)
 {
+    chain_begin();
     constexpr int N = 2 * W, NS = N / W_SEG;
     const int pt = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (pt >= a.win.n) return;
@@ -348,6 +352,7 @@ __global__ void sw_reduce_kernel(SwArgs a)
 template <int W>
 __global__ void __launch_bounds__(SwCfg<W>::NTS) sw_stats_kernel(SwArgs a)
 {
+    chain_begin();
     using C = SwCfg<W>;
     constexpr int N = C::N, NT = C::NTS, CPT = N / NT, CL = C::CL, PS = C::PS, NW = NT / 32;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -447,6 +452,7 @@ __global__ void __launch_bounds__(SwCfg<W>::NTS) sw_stats_kernel(SwArgs a)
 template <int W>
 __global__ void __launch_bounds__(SwCfg<W>::NTN) sw_fwd_kernel(SwArgs a)
 {
+    chain_begin();
     using C = SwCfg<W>;
     constexpr int N = C::N, G = C::G, NT = C::NTN, TILES = N / G;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -472,6 +478,7 @@ __global__ void __launch_bounds__(SwCfg<W>::NTN) sw_fwd_kernel(SwArgs a)
 template <int W>
 __global__ void __launch_bounds__(ColCfg<2 * W>::NT) sw_corr_kernel(SwArgs a)
 {
+    chain_begin();
     constexpr int N = 2 * W;
     using C = ColCfg<N>;
     const int pt = blockIdx.x / C::TILES, tile = blockIdx.x % C::TILES;
@@ -485,6 +492,7 @@ __global__ void __launch_bounds__(ColCfg<2 * W>::NT) sw_corr_kernel(SwArgs a)
 template <int W>
 __global__ void __launch_bounds__(SwCfg<W>::NTN) sw_ncc_kernel(SwArgs a)
 {
+    chain_begin();
     using C = SwCfg<W>;
     constexpr int N = C::N, G = C::G, NT = C::NTN, TS = corr_ts(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -539,6 +547,7 @@ __global__ void __launch_bounds__(SwCfg<W>::NTN) sw_ncc_kernel(SwArgs a)
 // The peak of a point, oversampled; its outputs.
 __global__ void __launch_bounds__(512) sw_peak_kernel(SwArgs a, int tiles)
 {
+    chain_begin();
     constexpr int NT = 512;
     __shared__ double Bm[W_OSW * W_N1], X[W_N1 * W_N1], T[W_N1 * W_OSW], dsc[NT / 32];
     __shared__ int isc[NT / 32];
@@ -620,6 +629,7 @@ __global__ void __launch_bounds__(512) sw_peak_kernel(SwArgs a, int tiles)
 
 __global__ void strackw_init_kernel(float* offR, float* offA, float* corr, uint8_t* type, int n)
 {
+    chain_begin();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     offR[k] = -2.0e9f;
@@ -632,10 +642,11 @@ __global__ void strackw_init_kernel(float* offR, float* offA, float* corr, uint8
 // set of one (window pair, upsampled pair, correlation), the figure serve.py
 // admits jobs by.  Large launches matter more than L2 (126 MB): the kernels are
 // short of instruction issue and shared-memory bandwidth, not of DRAM (10 to
-// 45 % of its rate).  At W = 224 (2 GB) the 2000 x 4000 pair takes 27.7 ms,
-// with 512 MB 36, with 128 MB 48.  At W = 64 (220 MB, 840 points) the 1024 x
-// 2048 pair takes 1.58 ms; four times that would give 1.38, but jobs that a
-// server's budget now admits would no longer fit.
+// 45 % of its rate).  With plain launches the 2000 x 4000 pair at W = 224 takes
+// 27.7 ms with these 2 GB, 28.5 with half, 27.0 with four times that; the 1024 x
+// 2048 pair at W = 64 1.58 ms with 220 MB (840 points), 1.76 with half, 1.38
+// with four times that, where jobs that a server's budget admits would no
+// longer fit.
 static size_t sw_chunk_bytes(int numSM, int W, int e)
 {
     const size_t N = 2 * W, L = 4 * e + 1;
@@ -715,22 +726,22 @@ struct SwRun {
         const int tiles2 = (hr1 - hr0 + C::G) / C::G, tilesL = (L + 15) / 16, pad = row_pad(a);
         cudaError_t e = launch_dop<W>(a.win, W, dop, az, st);
         if (e != cudaSuccess) return e;
-        sw_cols_kernel<W, F32><<<n * 2 * (W / C::G), C::NTW, C::smCols, st>>>(a);
-        sw_rows_kernel<W, F32><<<n * (N / C::G + tiles2), C::NTW, C::smRows + sizeof(float) * C::G * (N + 2 * pad), st>>>(
-            a, hr0, hr1, pad);
+        chain(sw_cols_kernel<W, F32>, n * 2 * (W / C::G), C::NTW, C::smCols, st, a);
+        chain(sw_rows_kernel<W, F32>, n * (N / C::G + tiles2), C::NTW,
+              C::smRows + sizeof(float) * C::G * (N + 2 * pad), st, a, hr0, hr1, pad);
         const int ga = n * (N / W_SEG);
         switch (a.taps) {
-        case -1: sw_amps_kernel<W, -1><<<ga, N, 0, st>>>(a); break;
-        case 2: sw_amps_kernel<W, 2><<<ga, N, 0, st>>>(a); break;
-        case 3: sw_amps_kernel<W, 3><<<ga, N, 0, st>>>(a); break;
-        default: sw_amps_kernel<W, 0><<<ga, N, 0, st>>>(a); break;
+        case -1: chain(sw_amps_kernel<W, -1>, ga, N, 0, st, a); break;
+        case 2: chain(sw_amps_kernel<W, 2>, ga, N, 0, st, a); break;
+        case 3: chain(sw_amps_kernel<W, 3>, ga, N, 0, st, a); break;
+        default: chain(sw_amps_kernel<W, 0>, ga, N, 0, st, a); break;
         }
-        sw_reduce_kernel<W><<<(n + 3) / 4, 128, 0, st>>>(a);
-        sw_stats_kernel<W><<<n * tilesL, C::NTS, C::smStats, st>>>(a);
-        sw_fwd_kernel<W><<<n * (N / C::G), C::NTN, C::smFwd, st>>>(a);
-        sw_corr_kernel<W><<<n * ColCfg<N>::TILES, ColCfg<N>::NT, ColCfg<N>::smem, st>>>(a);
-        sw_ncc_kernel<W><<<n * tilesL, C::NTN, C::smNcc, st>>>(a);
-        sw_peak_kernel<<<n, 512, 0, st>>>(a, tilesL);
+        chain(sw_reduce_kernel<W>, (n + 3) / 4, 128, 0, st, a);
+        chain(sw_stats_kernel<W>, n * tilesL, C::NTS, C::smStats, st, a);
+        chain(sw_fwd_kernel<W>, n * (N / C::G), C::NTN, C::smFwd, st, a);
+        chain(sw_corr_kernel<W>, n * ColCfg<N>::TILES, ColCfg<N>::NT, ColCfg<N>::smem, st, a);
+        chain(sw_ncc_kernel<W>, n * tilesL, C::NTN, C::smNcc, st, a);
+        chain(sw_peak_kernel, n, 512, 0, st, a, tilesL);
         *launches += 12;
         return cudaGetLastError();
     }

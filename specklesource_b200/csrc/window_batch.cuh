@@ -8,6 +8,7 @@
 #include <type_traits>
 
 #include "capi_internal.h"
+#include "chain.cuh"
 #include "fft_batch.cuh"
 #include "strack_device.cuh"
 
@@ -76,6 +77,7 @@ struct DopCfg {
 template <int W, bool F32>
 __global__ void __launch_bounds__(256) dop_sum_kernel(WinArgs a, double* part)
 {
+    chain_begin();
     using C = DopCfg<W>;
     __shared__ double red[9 * 4];
     const int pt = blockIdx.x / C::NB, band = blockIdx.x % C::NB;
@@ -104,6 +106,7 @@ __global__ void __launch_bounds__(256) dop_sum_kernel(WinArgs a, double* part)
 template <int W, bool F32>
 __global__ void __launch_bounds__(256, 4) dop_lag_kernel(WinArgs a, const double* sums, double* part)
 {
+    chain_begin();
     using C = DopCfg<W>;
     __shared__ double red[9 * 4];
     const int pt = blockIdx.x / C::NB, band = blockIdx.x % C::NB;
@@ -154,6 +157,7 @@ __global__ void __launch_bounds__(256, 4) dop_lag_kernel(WinArgs a, const double
 template <int W>
 __global__ void dop_angle_kernel(int n, const double* part, int wOut, int* az)
 {
+    chain_begin();
     const int pt = blockIdx.x * blockDim.x + threadIdx.x;
     if (pt >= n) return;
     double d[4] = {0, 0, 0, 0};
@@ -182,13 +186,13 @@ inline cudaError_t launch_dop(const WinArgs& a, int wOut, double* part, int* az,
     using C = DopCfg<W>;
     double* lag = part + (size_t)4 * a.n * C::NB;
     if (a.sampleType == SB_CFLOAT32) {
-        dop_sum_kernel<W, true><<<a.n * C::NB, C::NT, 0, st>>>(a, part);
-        dop_lag_kernel<W, true><<<a.n * C::NB, C::NT, 0, st>>>(a, part, lag);
+        chain(dop_sum_kernel<W, true>, a.n * C::NB, C::NT, 0, st, a, part);
+        chain(dop_lag_kernel<W, true>, a.n * C::NB, C::NT, 0, st, a, part, lag);
     } else {
-        dop_sum_kernel<W, false><<<a.n * C::NB, C::NT, 0, st>>>(a, part);
-        dop_lag_kernel<W, false><<<a.n * C::NB, C::NT, 0, st>>>(a, part, lag);
+        chain(dop_sum_kernel<W, false>, a.n * C::NB, C::NT, 0, st, a, part);
+        chain(dop_lag_kernel<W, false>, a.n * C::NB, C::NT, 0, st, a, part, lag);
     }
-    dop_angle_kernel<W><<<(a.n + 127) / 128, 128, 0, st>>>(a.n, lag, wOut, az);
+    chain(dop_angle_kernel<W>, (a.n + 127) / 128, 128, 0, st, a.n, lag, wOut, az);
     return cudaGetLastError();
 }
 
