@@ -671,18 +671,26 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
     PointRec* drec = (PointRec*)sb_ctx_buf(c, "rec", sizeof(PointRec) * n, &e);
     int* dlist = (int*)sb_ctx_buf(c, "list", sizeof(int) * (n + 1), &e);
     FitJob* dfit = (FitJob*)sb_ctx_buf(c, "fit", sizeof(FitJob) * (n + 1), &e);
-    unsigned long long* dstats = (unsigned long long*)sb_ctx_buf(c, "stats", sizeof(unsigned long long) * 8, &e);
-    float* dR = (float*)sb_ctx_buf(c, "offR", sizeof(float) * n, &e);
-    float* dA = (float*)sb_ctx_buf(c, "offA", sizeof(float) * n, &e);
-    float* dC = (float*)sb_ctx_buf(c, "corr", sizeof(float) * n, &e);
-    float* dZ = (float*)sb_ctx_buf(c, "azd", sizeof(float) * n, &e);
-    uint8_t* dT = (uint8_t*)sb_ctx_buf(c, "type", n, &e);
+    Packed lay;
+    const size_t atR = lay.add(sizeof(float) * n), atA = lay.add(sizeof(float) * n), atC = lay.add(sizeof(float) * n);
+    const size_t atZ = lay.add(sizeof(float) * n), atT = lay.add(n);
+    const size_t atS = lay.add(sizeof(unsigned long long) * 8), atCnt = lay.add(sizeof(int) * 4);
+    char* dout = (char*)sb_ctx_buf(c, "out", lay.bytes(), &e);
+    if (!dout) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
+    float* dR = (float*)(dout + atR);
+    float* dA = (float*)(dout + atA);
+    float* dC = (float*)(dout + atC);
+    float* dZ = (float*)(dout + atZ);
+    uint8_t* dT = (uint8_t*)(dout + atT);
+    unsigned long long* dstats = (unsigned long long*)(dout + atS);
+    // list lengths: complex stage, amplitude tries; then the split-BF16 form's wait flag
+    int* dStageCnt = (int*)(dout + atCnt);
     int* dlist2 = (int*)sb_ctx_buf(c, "listBands", sizeof(int) * (n + 1), &e);
     int* dkey = (int*)sb_ctx_buf(c, "listKey", sizeof(int) * (n + 1), &e);
     int* dpart = (int*)sb_ctx_buf(c, "partScratch", sizeof(int) * partition_scratch_ints(n, PART_KMAX), &e);
-    if (!dplan || !drec || !dlist || !dfit || !dstats || !dR || !dA || !dC || !dZ || !dT || !dlist2 ||
-        !dkey || !dpart)
+    if (!dplan || !drec || !dlist || !dfit || !dlist2 || !dkey || !dpart)
         return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
+    CK(cudaMemsetAsync(dstats, 0, lay.bytes() - atS, c->stream), "memset");
     // images: banded upload on the copy stream, overlapping the planning and
     // the complex matching of earlier bands
     const sb_image* ims[2] = {img1, img2};
@@ -691,6 +699,17 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
     if ((rc = upload_banded(c, ims, dimg, &bands)) != SB_OK) return rc;
     const void *d1 = dimg[0], *d2 = dimg[1];
     if (!devPlan) plan_strack(p, img1->nr, img1->na, img2->nr, img2->na, plan, clist);
+    // peak hand-off buffer: list chunks of at most kPeakChunk patches, each
+    // launched as complex kernel + peak kernel (-gauss keeps the fit in the
+    // complex kernel)
+    constexpr int kPeakChunk = 1 << 19;  // bench.py and serve.py's memory estimate use the same figure
+    // the split-BF16 tensor-core form where it applies (see sb_set_form)
+    const bool tcForm = p->noComplex == 0 && c->form == SB_FORM_SPLIT_BF16 && cmplx_tc_supported(W) && !baseOn &&
+                        !p->intf && !p->gaussFlag && c->smMajor >= 10;
+    // The complex list's length stays on the device where one launch takes the
+    // whole grid: its kernels get the grid as the upper bound, and the host
+    // does not wait for the plan (10 of 225 us at 256 x 512, window 32).
+    const bool devCount = devPlan && bands.nb == 1 && n <= kPeakChunk && !tcForm;
     int nC = 0;
     if (devPlan) {
         PlanArgs pa;
@@ -722,12 +741,14 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         const int K = strips ? SB_BANDS_MAX : 1;
         pa.stripPx = strips ? (img1->nr + SB_BANDS_MAX - 1) / SB_BANDS_MAX : 0;
         CK(launch_plan_poly(pa, dplan, dkey, c->stream), "plan_poly");
-        CK(launch_partition(dkey, nullptr, n, K, dlist, dpart, c->stream), "partition");
+        CK(launch_partition(dkey, nullptr, n, K, dlist, dpart, c->stream, dStageCnt), "partition");
         c->launches += 4;
-        CK(cudaMemcpyAsync(&nC, dpart + partition_keyoff_at(n, K) + K, sizeof(int), cudaMemcpyDeviceToHost,
-                           c->stream),
-           "count");
-        CK(cudaStreamSynchronize(c->stream), "sync");
+        if (devCount) {
+            nC = p->noComplex == 0 ? n : 0;
+        } else {
+            CK(cudaMemcpyAsync(&nC, dStageCnt, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "count");
+            CK(cudaStreamSynchronize(c->stream), "sync");
+        }
     } else {
         CK(cudaMemcpyAsync(dplan, plan.data(), sizeof(PointPlan) * n, cudaMemcpyHostToDevice, c->stream), "plan");
         if (!clist.empty())
@@ -752,8 +773,6 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
     // ---- kernels
     CK(launch_rec_init(drec, n, c->stream), "rec_init");
     c->launches++;
-    CK(cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * 8, c->stream), "memset");
-    int* tcErrFlag = nullptr;  // set when the split-BF16 form ran
     c->lastForm = SB_FORM_FP32;
     if (nC > 0) {
         CmplxArgs a;
@@ -766,6 +785,7 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         a.plan = dplan;
         a.list = dlist;
         a.nList = nC;
+        a.nListDev = devCount ? dStageCnt : nullptr;
         a.hanning = p->hanningFlag ? hanning_table(c, W) : nullptr;
         a.hanCorr = p->hanningFlag ? 1.5 : 1.0;
         a.twW = tw_table(c, W);
@@ -805,18 +825,8 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         }
         if (!a.twW || !a.tau || !a.osD || (p->hanningFlag && !a.hanning))
             return sb_ctx_fail(c, SB_ERR_NOMEM, "table allocation failed");
-        // the split-BF16 tensor-core form where it applies (see sb_set_form)
-        const bool tcForm = c->form == SB_FORM_SPLIT_BF16 && cmplx_tc_supported(W) && !baseOn && !p->intf &&
-                            !p->gaussFlag && c->smMajor >= 10;
         c->lastForm = tcForm ? SB_FORM_SPLIT_BF16 : SB_FORM_FP32;
-        int* dTcErr = nullptr;
-        if (tcForm) {
-            dTcErr = (int*)sb_ctx_buf(c, "tcErr", sizeof(int), &e);
-            if (!dTcErr) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
-            CK(cudaMemsetAsync(dTcErr, 0, sizeof(int), c->stream), "memset");
-            a.tcErr = dTcErr;
-            tcErrFlag = dTcErr;
-        }
+        if (tcForm) a.tcErr = dStageCnt + 3;
         int cthreads = 0, bpsm = 0;
         complex_shape(c, W, tcForm, &cthreads, &bpsm);
         if (bpsm <= 0) return sb_ctx_fail(c, SB_ERR_CUDA, "complex kernel cannot be resident (W=%d)", W);
@@ -835,10 +845,6 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
             a.list = dlist2;
         }
         const int nBand = bands.nb > 1 ? bands.nb : 1;
-        // peak hand-off buffer: list chunks of at most kPeakChunk patches, each
-        // launched as complex kernel + peak kernel (-gauss keeps the fit in
-        // the complex kernel)
-        constexpr int kPeakChunk = 1 << 19;  // bench.py and serve.py's memory estimate use the same figure
         PeakJob* dpeak = nullptr;
         if (!p->gaussFlag) {
             const size_t pc = nC < kPeakChunk ? (size_t)nC : (size_t)kPeakChunk;
@@ -866,6 +872,7 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
                     PeakArgs pk;
                     pk.peak = dpeak;
                     pk.nList = cnt;
+                    pk.nListDev = a.nListDev;
                     pk.W = W;
                     pk.hanCorr = a.hanCorr;
                     pk.osD = a.osD;
@@ -878,10 +885,10 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         }
         cudaEventRecord(c->sev[1], c->stream);
         FitArgs f = make_fit_args(p, dfit, a.nList, 0, drec);
+        f.nListDev = a.nListDev;
         CK(launch_strack_fit(f, c->stream), "strack_fit");
         c->launches++;
         cudaEventRecord(c->sev[2], c->stream);
-        c->stage[5] = (float)a.nList;
     }
     // every band resident before the amplitude tries
     CK(cudaStreamWaitEvent(c->stream, c->chunkEv[bands.nb - 1], 0), "wait bands");
@@ -894,16 +901,12 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
     // The tries run without host round trips: each try's list length stays on
     // the device (kernels launched for the whole grid read it), and the
     // stage timings and the tensor-core wait flag are read after the call.
-    int* dStageCnt = (int*)sb_ctx_buf(c, "stageCnt", sizeof(int) * 4, &e);
-    if (!dStageCnt) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
-    CK(cudaMemsetAsync(dStageCnt, 0, sizeof(int) * 4, c->stream), "memset");
     bool stageRan[3] = {false, false, false};
     for (int stage = 1; stage <= 2 && stage <= p->maxTries; ++stage) {
         CK(launch_select(dplan, drec, n, w, stage, dkey, c->stream), "select");
-        CK(launch_partition(dkey, nullptr, n, 1, dlist, dpart, c->stream), "partition");
+        const int* dCnt = dStageCnt + stage;
+        CK(launch_partition(dkey, nullptr, n, 1, dlist, dpart, c->stream, dStageCnt + stage), "partition");
         c->launches += 4;
-        const int* dCnt = dpart + partition_keyoff_at(n, 1) + 1;
-        CK(cudaMemcpyAsync(dStageCnt + stage, dCnt, sizeof(int), cudaMemcpyDeviceToDevice, c->stream), "count");
         const int Ws = WA * (stage == 1 ? 1 : LA);
         // small windows (shared-memory kernel): launched for the whole grid,
         // the list length read on the device; larger windows run the list in
@@ -974,18 +977,18 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
     if ((rc = oc.add(out->type, dT, n, out->onDevice != 0)) != SB_OK) return rc;
     unsigned long long st[8];
     if ((rc = oc.add(st, dstats, sizeof(st))) != SB_OK) return rc;
-    int stageCnt[4] = {0, 0, 0, 0}, tcBad = 0;
+    int stageCnt[4] = {0, 0, 0, 0};
     if ((rc = oc.add(stageCnt, dStageCnt, sizeof(stageCnt))) != SB_OK) return rc;
-    if (tcErrFlag && (rc = oc.add(&tcBad, tcErrFlag, sizeof(int))) != SB_OK) return rc;
-    cudaEventRecord(c->ev[3], c->stream);
     if ((rc = oc.finish("strack")) != SB_OK) return rc;
-    if (tcBad) return sb_ctx_fail(c, SB_ERR_TIMEOUT, "split-BF16 complex stage: a tensor-core wait timed out");
+    if (stageCnt[3]) return sb_ctx_fail(c, SB_ERR_TIMEOUT, "split-BF16 complex stage: a tensor-core wait timed out");
+    if (devCount && nC > 0) nC = stageCnt[0];
     if (nC > 0) {
         float t0 = 0, t1 = 0;
         cudaEventElapsedTime(&t0, c->sev[0], c->sev[1]);
         cudaEventElapsedTime(&t1, c->sev[1], c->sev[2]);
         c->stage[0] = t0;
         c->stage[3] += t1;
+        c->stage[5] = (float)nC;
     }
     for (int stage = 1; stage <= 2; ++stage) {
         if (!stageRan[stage]) continue;
@@ -1163,17 +1166,25 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
     int* dlist = (int*)sb_ctx_buf(c, "list", sizeof(int) * (n + 1), &e);
     int* dpairOf = (int*)sb_ctx_buf(c, "pairOf", sizeof(int) * n, &e);
     FitJob* dfit = (FitJob*)sb_ctx_buf(c, "fit", sizeof(FitJob) * (n + 1), &e);
-    unsigned long long* dstats = (unsigned long long*)sb_ctx_buf(c, "stats", sizeof(unsigned long long) * 8 * nPairs, &e);
-    float* dR = (float*)sb_ctx_buf(c, "offR", sizeof(float) * n, &e);
-    float* dA = (float*)sb_ctx_buf(c, "offA", sizeof(float) * n, &e);
-    float* dC = (float*)sb_ctx_buf(c, "corr", sizeof(float) * n, &e);
-    float* dZ = (float*)sb_ctx_buf(c, "azd", sizeof(float) * n, &e);
-    uint8_t* dT = (uint8_t*)sb_ctx_buf(c, "type", n, &e);
+    Packed lay;
+    const size_t atR = lay.add(sizeof(float) * n), atA = lay.add(sizeof(float) * n), atC = lay.add(sizeof(float) * n);
+    const size_t atZ = lay.add(sizeof(float) * n), atT = lay.add(n);
+    const size_t atS = lay.add(sizeof(unsigned long long) * 8 * nPairs);
+    const size_t atCnt = lay.add(sizeof(int) * 3 * nBk), atErr = lay.add(sizeof(int));
+    char* dout = (char*)sb_ctx_buf(c, "out", lay.bytes(), &e);
+    if (!dout) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
+    float* dR = (float*)(dout + atR);
+    float* dA = (float*)(dout + atA);
+    float* dC = (float*)(dout + atC);
+    float* dZ = (float*)(dout + atZ);
+    uint8_t* dT = (uint8_t*)(dout + atT);
+    unsigned long long* dstats = (unsigned long long*)(dout + atS);
+    int* dStageCnt = (int*)(dout + atCnt);
+    int* dTcErr = (int*)(dout + atErr);
     int* dkey = (int*)sb_ctx_buf(c, "listKey", sizeof(int) * (n + 1), &e);
     int* dpart = (int*)sb_ctx_buf(c, "partScratch", sizeof(int) * partition_scratch_ints(n, PART_KMAX), &e);
     int* dAz = (int*)sb_ctx_buf(c, "azEff", sizeof(int) * n, &e);
-    if (!dplan || !drec || !dclist || !dlist || !dpairOf || !dfit || !dstats || !dR || !dA || !dC || !dZ || !dT ||
-        !dkey || !dpart || !dAz)
+    if (!dplan || !drec || !dclist || !dlist || !dpairOf || !dfit || !dkey || !dpart || !dAz)
         return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
     // Plans: on the device for a polynomial shift (each complex candidate keyed
     // by its bucket), on the host for an offset grid (its holes carry r2/a2
@@ -1271,7 +1282,7 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
                "clist");
         CK(cudaStreamSynchronize(c->stream), "sync");
     }
-    CK(cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * 8 * nPairs, c->stream), "memset");
+    CK(cudaMemsetAsync(dstats, 0, lay.bytes() - atS, c->stream), "memset");
     cudaEventRecord(c->ev[1], c->stream);
     CK(launch_rec_init(drec, n, c->stream), "rec_init");
     c->launches++;
@@ -1281,12 +1292,6 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
     BatchEvents bev(2 * nBk);
     if (!bev.ok()) return sb_ctx_fail(c, SB_ERR_CUDA, "event creation failed");
     std::vector<char> cmplxRan((size_t)nBk, 0);
-    int* dStageCnt = (int*)sb_ctx_buf(c, "stageCnt", sizeof(int) * 3 * nBk, &e);
-    if (!dStageCnt) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
-    CK(cudaMemsetAsync(dStageCnt, 0, sizeof(int) * 3 * nBk, c->stream), "memset");
-    int* dTcErr = (int*)sb_ctx_buf(c, "tcErr", sizeof(int), &e);
-    if (!dTcErr) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
-    CK(cudaMemsetAsync(dTcErr, 0, sizeof(int), c->stream), "memset");
     c->lastForm = SB_FORM_FP32;
     constexpr int kPeakChunk = 1 << 19;
     for (int bi = 0; bi < nBk; ++bi) {
@@ -1349,6 +1354,7 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
                     PeakArgs pk;
                     pk.peak = dpeak;
                     pk.nList = cnt;
+                    pk.nListDev = nullptr;
                     pk.W = W;
                     pk.hanCorr = a.hanCorr;
                     pk.osD = a.osD;
@@ -1375,12 +1381,10 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
         PointRec* brec = drec + b.g0;
         for (int stage = 1; stage <= 2 && stage <= p->maxTries; ++stage) {
             CK(launch_select(bplan, brec, nB, w, stage, dkey, c->stream), "select");
-            CK(launch_partition(dkey, nullptr, nB, 1, dlist, dpart, c->stream), "partition");
-            c->launches += 4;
             // the try's list length stays on the device (no host round trip)
-            const int* dCnt = dpart + partition_keyoff_at(nB, 1) + 1;
-            CK(cudaMemcpyAsync(dStageCnt + 3 * bi + stage, dCnt, sizeof(int), cudaMemcpyDeviceToDevice, c->stream),
-               "count");
+            int* dCnt = dStageCnt + 3 * bi + stage;
+            CK(launch_partition(dkey, nullptr, nB, 1, dlist, dpart, c->stream, dCnt), "partition");
+            c->launches += 4;
             const int Ws = WA * (stage == 1 ? 1 : LA);
             // as in sb_strack: the length is read back only for the chunked kernels
             const bool onChip = amps_supported(Ws);
@@ -1438,24 +1442,27 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
         c->launches++;
     }
     cudaEventRecord(c->ev[2], c->stream);
-    // ---- outputs, per pair
+    // ---- outputs, per array the pairs in the order they lie in
     OutCopies oc(c);
-    for (int k = 0; k < nPairs; ++k) {
-        const size_t g = (size_t)gStart[k], m = (size_t)P[k].nR * P[k].nA;
-        const bool od = out[k].onDevice != 0;
-        if ((rc = oc.add(out[k].offR, dR + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if ((rc = oc.add(out[k].offA, dA + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if ((rc = oc.add(out[k].corr, dC + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if (out[k].azd && (rc = oc.add(out[k].azd, dZ + g, sizeof(float) * m, od)) != SB_OK) return rc;
-        if ((rc = oc.add(out[k].type, dT + g, m, od)) != SB_OK) return rc;
-    }
+    for (int g = 0; g < 5; ++g)
+        for (int q = 0; q < nPairs; ++q) {
+            const int k = order[q];
+            const size_t at = (size_t)gStart[k], m = (size_t)P[k].nR * P[k].nA;
+            float* const f[4] = {out[k].offR, out[k].offA, out[k].corr, out[k].azd};
+            const float* const d[4] = {dR, dA, dC, dZ};
+            const bool od = out[k].onDevice != 0;
+            if (g == 4)
+                rc = oc.add(out[k].type, dT + at, m, od);
+            else if (f[g])  // azd may be left out
+                rc = oc.add(f[g], d[g] + at, sizeof(float) * m, od);
+            if (rc != SB_OK) return rc;
+        }
     std::vector<unsigned long long> st((size_t)8 * nPairs);
     if ((rc = oc.add(st.data(), dstats, sizeof(unsigned long long) * 8 * nPairs)) != SB_OK) return rc;
     int tcBad = 0;
-    if ((rc = oc.add(&tcBad, dTcErr, sizeof(int))) != SB_OK) return rc;
     std::vector<int> stageCnt((size_t)3 * nBk);
     if ((rc = oc.add(stageCnt.data(), dStageCnt, sizeof(int) * 3 * nBk)) != SB_OK) return rc;
-    cudaEventRecord(c->ev[3], c->stream);
+    if ((rc = oc.add(&tcBad, dTcErr, sizeof(int))) != SB_OK) return rc;
     if ((rc = oc.finish("strack_batch")) != SB_OK) return rc;
     for (int bi = 0; bi < nBk; ++bi) {
         if (cmplxRan[bi]) {

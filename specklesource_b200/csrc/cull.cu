@@ -986,6 +986,25 @@ int cull_check(sb_context* c, const sb_cull_params* p, const sb_cull_data* d)
         if (_e != cudaSuccess) return sb_ctx_cuda(c, _e, what);      \
     } while (0)
 
+// The grids of a host job that are (also) outputs, in one buffer.
+char* grid_block(sb_context* c, size_t n, CullDev* v, cudaError_t* e)
+{
+    Packed pk;
+    size_t at[6];
+    for (size_t& a : at) a = pk.add(n * sizeof(float));
+    const size_t atT = pk.add(n);
+    char* g = (char*)sb_ctx_buf(c, "c_grids", pk.bytes(), e);
+    if (!g) return nullptr;
+    v->offR = (float*)(g + at[0]);
+    v->offA = (float*)(g + at[1]);
+    v->offRS = (float*)(g + at[2]);
+    v->offAS = (float*)(g + at[3]);
+    v->sigmaR = (float*)(g + at[4]);
+    v->sigmaA = (float*)(g + at[5]);
+    v->type = (uint8_t*)(g + atT);
+    return g;
+}
+
 // Device views of the job's grids (copies host inputs in).  whole: every pass
 // runs, so the outputs are written before anything reads them.
 int cull_stage_in(sb_context* c, const sb_cull_params* p, sb_cull_data* d, CullDev* v, bool whole)
@@ -1002,19 +1021,12 @@ int cull_stage_in(sb_context* c, const sb_cull_params* p, sb_cull_data* d, CullD
         if (!v->sigmaA) v->sigmaA = (float*)sb_ctx_buf(c, "c_sigmaA", fb, &e);
         return SB_OK;
     }
-    v->offR = (float*)sb_ctx_buf(c, "c_offR", fb, &e);
-    v->offA = (float*)sb_ctx_buf(c, "c_offA", fb, &e);
+    char* grids = grid_block(c, n, v, &e);
     v->corr = (float*)sb_ctx_buf(c, "c_corr", fb, &e);
-    v->type = (uint8_t*)sb_ctx_buf(c, "c_type", n, &e);
-    v->offRS = (float*)sb_ctx_buf(c, "c_offRS", fb, &e);
-    v->offAS = (float*)sb_ctx_buf(c, "c_offAS", fb, &e);
-    v->sigmaR = (float*)sb_ctx_buf(c, "c_sigmaR", fb, &e);
-    v->sigmaA = (float*)sb_ctx_buf(c, "c_sigmaA", fb, &e);
     v->mask = d->mask ? (uint8_t*)sb_ctx_buf(c, "c_mask", n, &e) : nullptr;
     v->simR = p->useSim ? (float*)sb_ctx_buf(c, "c_simR", fb, &e) : nullptr;
     v->simA = p->useSim ? (float*)sb_ctx_buf(c, "c_simA", fb, &e) : nullptr;
-    if (!v->offR || !v->offA || !v->corr || !v->type || !v->offRS || !v->offAS || !v->sigmaR || !v->sigmaA ||
-        (d->mask && !v->mask) || (p->useSim && (!v->simR || !v->simA)))
+    if (!grids || !v->corr || (d->mask && !v->mask) || (p->useSim && (!v->simR || !v->simA)))
         return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
     cudaStream_t s = c->stream;
     CKC(cudaMemcpyAsync(v->offR, d->offR, fb, cudaMemcpyHostToDevice, s), "h2d");
@@ -1042,12 +1054,11 @@ int cull_stage_out(OutCopies* oc, const sb_cull_params* p, sb_cull_data* d, cons
     int rc;
     if ((rc = oc->add(d->offR, v->offR, fb)) != SB_OK) return rc;
     if ((rc = oc->add(d->offA, v->offA, fb)) != SB_OK) return rc;
-    if ((rc = oc->add(d->type, v->type, n)) != SB_OK) return rc;
     if (d->offRS && (rc = oc->add(d->offRS, v->offRS, fb)) != SB_OK) return rc;
     if (d->offAS && (rc = oc->add(d->offAS, v->offAS, fb)) != SB_OK) return rc;
     if (d->sigmaR && (rc = oc->add(d->sigmaR, v->sigmaR, fb)) != SB_OK) return rc;
     if (d->sigmaA && (rc = oc->add(d->sigmaA, v->sigmaA, fb)) != SB_OK) return rc;
-    return SB_OK;
+    return oc->add(d->type, v->type, n);
 }
 
 // Largest float not above t: d > t for a float d is d > float_down(t).
@@ -1277,7 +1288,6 @@ int cull_run(sb_context* c, In stageIn, F body, Out stageOut)
     cudaEventRecord(c->ev[2], c->stream);
     OutCopies oc(c);
     if ((rc = stageOut(&oc, &v)) != SB_OK) return rc;
-    cudaEventRecord(c->ev[3], c->stream);
     if ((rc = oc.finish("cull")) != SB_OK) return rc;
     cudaEventElapsedTime(&c->timing[0], c->ev[0], c->ev[3]);
     cudaEventElapsedTime(&c->timing[1], c->ev[0], c->ev[1]);
@@ -1319,18 +1329,15 @@ int cullls_stage_in(sb_context* c, const sb_cullls_params* p, sb_cullls_data* d,
         v->offR = d->X; v->offA = d->Y; v->type = (uint8_t*)d->type;
         v->offRS = d->XS; v->offAS = d->YS; v->sigmaR = d->sigmaX; v->sigmaA = d->sigmaY;
     } else {
-        v->offR = (float*)sb_ctx_buf(c, "c_offR", fb, &e);
-        v->offA = (float*)sb_ctx_buf(c, "c_offA", fb, &e);
-        v->type = (uint8_t*)sb_ctx_buf(c, "c_type", n, &e);
-        if (!v->offR || !v->offA || !v->type) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
+        if (!grid_block(c, n, v, &e)) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
         CKC(cudaMemcpyAsync(v->offR, d->X, fb, cudaMemcpyHostToDevice, c->stream), "h2d");
         CKC(cudaMemcpyAsync(v->offA, d->Y, fb, cudaMemcpyHostToDevice, c->stream), "h2d");
         CKC(cudaMemcpyAsync(v->type, d->type, n, cudaMemcpyHostToDevice, c->stream), "h2d");
     }
-    if (!d->onDevice || !v->offRS) v->offRS = (float*)sb_ctx_buf(c, "c_offRS", fb, &e);
-    if (!d->onDevice || !v->offAS) v->offAS = (float*)sb_ctx_buf(c, "c_offAS", fb, &e);
-    if (!d->onDevice || !v->sigmaR) v->sigmaR = (float*)sb_ctx_buf(c, "c_sigmaR", fb, &e);
-    if (!d->onDevice || !v->sigmaA) v->sigmaA = (float*)sb_ctx_buf(c, "c_sigmaA", fb, &e);
+    if (!v->offRS) v->offRS = (float*)sb_ctx_buf(c, "c_offRS", fb, &e);
+    if (!v->offAS) v->offAS = (float*)sb_ctx_buf(c, "c_offAS", fb, &e);
+    if (!v->sigmaR) v->sigmaR = (float*)sb_ctx_buf(c, "c_sigmaR", fb, &e);
+    if (!v->sigmaA) v->sigmaA = (float*)sb_ctx_buf(c, "c_sigmaA", fb, &e);
     if (!v->offRS || !v->offAS || !v->sigmaR || !v->sigmaA)
         return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
     return SB_OK;

@@ -22,7 +22,8 @@ size_t partition_scratch_ints(int n, int K);
 // position of key k, keyOff[K] = number of items kept.
 size_t partition_keyoff_at(int n, int K);
 
+// count (may be null) also receives keyOff[K].
 cudaError_t launch_partition(const int* key, const int* val, int n, int K, int* out, int* scratch,
-                             cudaStream_t st);
+                             cudaStream_t st, int* count = nullptr);
 
 }  // namespace sbk

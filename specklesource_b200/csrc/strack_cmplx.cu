@@ -340,17 +340,18 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
 
     // list entries are loaded two patches ahead and plans one patch ahead,
     // so a patch's window loads never wait on the dependent list -> plan loads
-    const int G = gridDim.x;
+    const int G = gridDim.x, nList = a.nListDev ? min(a.nList, *a.nListDev) : a.nList;
+    if ((int)blockIdx.x >= nList) return;
     int pNext = a.list[blockIdx.x];
-    int pAfter = (int)blockIdx.x + G < a.nList ? a.list[blockIdx.x + G] : 0;
+    int pAfter = (int)blockIdx.x + G < nList ? a.list[blockIdx.x + G] : 0;
     PointPlan plNext = a.plan[pNext];
-    for (int it = blockIdx.x; it < a.nList; it += G) {
+    for (int it = blockIdx.x; it < nList; it += G) {
         const int p = pNext;
         const PointPlan pl = plNext;
-        if (it + G < a.nList) {
+        if (it + G < nList) {
             pNext = pAfter;
             plNext = a.plan[pAfter];
-            if (it + 2 * G < a.nList) pAfter = a.list[it + 2 * G];
+            if (it + 2 * G < nList) pAfter = a.list[it + 2 * G];
         }
         // ---------------------------------------------------- getPatches
         // per-thread partial sums over the RPT rows in float, block totals in double

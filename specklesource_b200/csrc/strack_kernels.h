@@ -29,7 +29,8 @@ constexpr int32_t PJ_NODATA = -2000000;
 // Arguments of the peak kernel (one warp per list position).
 struct PeakArgs {
     const PeakJob* peak;
-    int nList;
+    int nList;             // list length, or its upper bound when nListDev is set
+    const int* nListDev;   // non-null: the list length, read on the device
     int W;                 // complex window (the surface is 2W x 2W)
     double hanCorr;
     const float2* osD;     // real oversampling table (48 x 8 floats D, 16 phases)
@@ -46,7 +47,8 @@ struct CmplxArgs {
     int sampleType, byteOrder;
     const PointPlan* plan;
     const int* list;
-    int nList;
+    int nList;             // list length, or its upper bound when nListDev is set
+    const int* nListDev;   // non-null: the list length, read on the device (FP32 form)
     const float* hanning;  // W x W, or nullptr when -noHanning
     double hanCorr;        // 1.5 with Hanning, else 1.0
     const float2* twW;     // W_W^e forward twiddles, W entries

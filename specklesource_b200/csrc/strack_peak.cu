@@ -32,8 +32,8 @@ __global__ void __launch_bounds__(32 * kPeakWarps) strack_peak_kernel(PeakArgs a
     for (int e = threadIdx.x; e < OSW * NFAST + 2 * 16; e += blockDim.x) osD[e] = reinterpret_cast<const float*>(a.osD)[e];
     __syncthreads();
     const int W2 = 2 * a.W;
-    const int nWarps = gridDim.x * kPeakWarps;
-    for (int it = blockIdx.x * kPeakWarps + w; it < a.nList; it += nWarps) {
+    const int nWarps = gridDim.x * kPeakWarps, nList = a.nListDev ? min(a.nList, *a.nListDev) : a.nList;
+    for (int it = blockIdx.x * kPeakWarps + w; it < nList; it += nWarps) {
         const PeakJob* pj = a.peak + it;
         const int iC = pj->iC, jC = pj->jC;
         if (iC == PJ_NODATA) continue;  // getPatches failed: the complex kernel wrote the record

@@ -924,11 +924,16 @@ extern "C" int sb_strackw(sb_context* c, const sb_track_params* p, const sb_imag
     const int nl = (int)list.size();
     int4* dplan = (int4*)sb_ctx_buf(c, "w_plan", sizeof(int4) * (nl + 1), &e);
     int* dlist = (int*)sb_ctx_buf(c, "w_list", sizeof(int) * (nl + 1), &e);
-    float* dR = (float*)sb_ctx_buf(c, "offR", sizeof(float) * n, &e);
-    float* dA = (float*)sb_ctx_buf(c, "offA", sizeof(float) * n, &e);
-    float* dC = (float*)sb_ctx_buf(c, "corr", sizeof(float) * n, &e);
-    uint8_t* dT = (uint8_t*)sb_ctx_buf(c, "type", n, &e);
-    unsigned long long* dst = (unsigned long long*)sb_ctx_buf(c, "w_stats", 4 * sizeof(unsigned long long), &e);
+    Packed lay;
+    const size_t atR = lay.add(sizeof(float) * n), atA = lay.add(sizeof(float) * n), atC = lay.add(sizeof(float) * n);
+    const size_t atT = lay.add(n), atS = lay.add(4 * sizeof(unsigned long long));
+    char* dout = (char*)sb_ctx_buf(c, "out", lay.bytes(), &e);
+    if (!dout) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
+    float* dR = (float*)(dout + atR);
+    float* dA = (float*)(dout + atA);
+    float* dC = (float*)(dout + atC);
+    uint8_t* dT = (uint8_t*)(dout + atT);
+    unsigned long long* dst = (unsigned long long*)(dout + atS);
     // the real oversampling kernel of the 21 -> 336 symmetric zero pad
     const double* dB = (const double*)sb_table(c, "w_B", [] {
         std::vector<double> B(W_OSW * W_N1);
@@ -942,7 +947,7 @@ extern "C" int sb_strackw(sb_context* c, const sb_track_params* p, const sb_imag
             }
         return B;
     });
-    if (!dplan || !dlist || !dR || !dA || !dC || !dT || !dst || !dB)
+    if (!dplan || !dlist || !dB)
         return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
     if (nl) {
         CKW(cudaMemcpyAsync(dplan, plan.data(), sizeof(int4) * nl, cudaMemcpyHostToDevice, c->stream), "plan");
@@ -985,7 +990,6 @@ extern "C" int sb_strackw(sb_context* c, const sb_track_params* p, const sb_imag
     if ((rc = oc.add(out->type, dT, n, od)) != SB_OK) return rc;
     unsigned long long st[4];
     if ((rc = oc.add(st, dst, sizeof(st))) != SB_OK) return rc;
-    cudaEventRecord(c->ev[3], c->stream);
     if ((rc = oc.finish("strackw")) != SB_OK) return rc;
     out->nComplex = 0;
     out->nAmp = (int64_t)st[0];

@@ -102,3 +102,22 @@ def test_batch_more_buckets_than_partition_keys(ctx):
             tv = t[key].cpu().numpy() if hasattr(t[key], "cpu") else t[key]
             assert np.array_equal(sv, tv, equal_nan=True), (k, key)
         assert s["stats"] == t["stats"], k
+
+
+@pytest.mark.parametrize("nR,nA,keep", [(1, 1, 1.0), (1, 1, 0.0), (7, 5, 0.2), (64, 37, 1.0), (64, 37, 0.0),
+                                        (64, 37, 0.02), (400, 390, 0.7)])
+def test_list_length_on_the_device(ctx, nR, nA, keep):
+    """One sb_strack call launches its complex stage for the whole grid and
+    reads the list's length on the device; the batch counts on the host.  Grids
+    of one tile and of more than four warps of tiles, lists that are empty,
+    shorter than the launch, and full."""
+    na, nr = 448, 512
+    s1, s2 = synth.small_pair(device="cuda", na=na, nr=nr, seed=77)
+    mk = (np.random.default_rng(3).random((na // 8, nr // 8)) < keep).astype(np.uint8)
+    p = abi.TrackParams(rStart=24, aStart=24, nR=nR, nA=nA, wR=16, wA=16, wRa=16, wAa=16, rShiftPoly=(1.0, 0.0, 0.0),
+                        mask={"r0": 0, "a0": 0, "nr": nr // 8, "na": na // 8, "nrl": 8, "nal": 8, "mask": mk})
+    s = ctx.strack(p, s1, s2)
+    t, = ctx.strack_batch([p], [s1], [s2])
+    for key in ("offR", "offA", "corr", "azd", "type"):
+        assert np.array_equal(s[key], t[key], equal_nan=True), key
+    assert s["stats"] == t["stats"]
