@@ -1126,15 +1126,31 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
         atlas[i] = (char*)sb_ctx_buf(c, i ? "atlas2" : "atlas1", (size_t)width[i] * height[i] * elem, &e);
         if (!atlas[i]) return sb_ctx_cuda(c, e, "cudaMalloc(atlas)");
     }
+    std::vector<AtlasJob> jobs;  // images on the device, copied by one kernel
+    int maxRows = 0;
     for (int k = 0; k < nPairs; ++k) {
         const sb_image* im[2] = {&I1[k], &I2[k]};
         for (int i = 0; i < 2; ++i) {
             const size_t pitch = (size_t)width[i] * elem, rowB = (size_t)im[i]->nr * elem;
+            if (im[i]->onDevice && reinterpret_cast<uintptr_t>(im[i]->data) % 4 == 0) {
+                jobs.push_back({(const char*)im[i]->data, atlas[i] + (size_t)rowOff[i][k] * pitch, rowB, pitch,
+                                im[i]->na});
+                maxRows = im[i]->na > maxRows ? im[i]->na : maxRows;
+                continue;
+            }
             CK(cudaMemcpy2DAsync(atlas[i] + (size_t)rowOff[i][k] * pitch, pitch, im[i]->data, rowB, rowB,
                                  (size_t)im[i]->na, im[i]->onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                  c->stream),
                "atlas copy");
         }
+    }
+    if (!jobs.empty()) {
+        AtlasJob* djobs = (AtlasJob*)sb_ctx_buf(c, "atlasJobs", sizeof(AtlasJob) * jobs.size(), &e);
+        if (!djobs) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
+        CK(cudaMemcpyAsync(djobs, jobs.data(), sizeof(AtlasJob) * jobs.size(), cudaMemcpyHostToDevice, c->stream),
+           "atlas jobs");
+        CK(launch_atlas_copy(djobs, (int)jobs.size(), maxRows, c->stream), "atlas_copy");
+        c->launches++;
     }
     // ---- plans of every pair, offset into the atlases; complex lists per bucket
     const int n = (int)total;

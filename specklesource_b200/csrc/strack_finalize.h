@@ -26,6 +26,17 @@ struct PlanArgs {
     int stripPx;
 };
 
+// One image to be copied into an atlas: rows of rowB bytes, pitch bytes apart
+// in dst.  Addresses, rowB and pitch are multiples of 4.
+struct AtlasJob {
+    const char* src;
+    char* dst;
+    size_t rowB, pitch;
+    int rows;
+};
+// jobs (device): n of them, the tallest with maxRows rows.
+cudaError_t launch_atlas_copy(const AtlasJob* jobs, int n, int maxRows, cudaStream_t st);
+
 // Writes the plan of every point and key[p] = keyValue for complex candidates, else -1.
 cudaError_t launch_plan_poly(const PlanArgs& a, PointPlan* plan, int* key, cudaStream_t st);
 

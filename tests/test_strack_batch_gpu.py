@@ -121,3 +121,30 @@ def test_list_length_on_the_device(ctx, nR, nA, keep):
     for key in ("offR", "offA", "corr", "azd", "type"):
         assert np.array_equal(s[key], t[key], equal_nan=True), key
     assert s["stats"] == t["stats"]
+
+
+@pytest.mark.parametrize("int16", [False, True])
+def test_device_images_of_any_row_length(ctx, int16):
+    """Device images into the atlases: rows of a multiple of 16, 8 and 4 bytes,
+    an image that starts between two words of that size, one-row remainders."""
+    import torch
+    cases = []
+    for k, (na, nr, shift) in enumerate([(120, 128, 0), (121, 131, 0), (127, 133, 1), (97, 161, 3)]):
+        s = []
+        for im in synth.small_pair(device="cuda", na=na, nr=nr, seed=80 + k):
+            if int16:
+                im = torch.view_as_real(im)
+                im = torch.clamp((im * (1000.0 / im.abs().max())).round(), -32767, 32767).to(torch.int16)
+            flat = torch.empty(im.numel() + 2 * shift, dtype=im.dtype, device="cuda")
+            off = 2 * shift if int16 else shift
+            v = flat[off:off + im.numel()].view(im.shape)
+            v.copy_(im)
+            s.append(v)
+        p = abi.TrackParams(rStart=24, aStart=24, deltaR=16, deltaA=16, nR=5, nA=4, wR=16, wA=16, wRa=16, wAa=16)
+        cases.append((p, s[0], s[1]))
+    single = [ctx.strack(*c) for c in cases]
+    batch = ctx.strack_batch([c[0] for c in cases], [c[1] for c in cases], [c[2] for c in cases])
+    for k, (s, t) in enumerate(zip(single, batch)):
+        for key in ("offR", "offA", "corr", "azd", "type"):
+            assert np.array_equal(s[key], t[key], equal_nan=True), (k, key)
+        assert s["stats"] == t["stats"]
