@@ -730,17 +730,21 @@ int cmplx_tc_threads() { return NT; }
 // two resident; the resources are counted here instead.)
 int cmplx_tc_blocks_per_sm()
 {
-    int dev = 0;
-    cudaDeviceProp pr;
+    // (attribute by attribute: the whole property record takes 3 ms and more)
+    int dev = 0, regs = 0, shared = 0, reserved = 0, threads = 0;
     cudaFuncAttributes fa;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaGetDeviceProperties(&pr, dev) != cudaSuccess ||
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&threads, cudaDevAttrMaxThreadsPerMultiProcessor, dev) != cudaSuccess ||
         cudaFuncGetAttributes(&fa, strack_cmplx_tc_kernel<true>) != cudaSuccess)
         return 0;
     const int regsPerWarp = ((fa.numRegs * 32 + 255) / 256) * 256;  // allocation unit of 256 registers per warp
-    const int byRegs = pr.regsPerMultiprocessor / (regsPerWarp * (NT / 32));
-    const size_t perCta = (size_t)SMEM_BYTES + fa.sharedSizeBytes + pr.reservedSharedMemPerBlock;
-    const int bySmem = (int)(pr.sharedMemPerMultiprocessor / perCta);
-    const int byThreads = pr.maxThreadsPerMultiProcessor / NT;
+    const int byRegs = regs / (regsPerWarp * (NT / 32));
+    const size_t perCta = (size_t)SMEM_BYTES + fa.sharedSizeBytes + (size_t)reserved;
+    const int bySmem = (int)((size_t)shared / perCta);
+    const int byThreads = threads / NT;
     int nb = byRegs < bySmem ? byRegs : bySmem;
     nb = nb < byThreads ? nb : byThreads;
     // two 256-column TMEM allocations fill an SM's 512 columns: never more

@@ -69,14 +69,16 @@ __global__ void az_fill_kernel(const PointRec* rec, int n, int* azEff)
     }
 }
 
+// Bound by the reads of the records.  With an addition per point to the same
+// few counters it was bound by those: 1,966,132 points 1.30 ms, now 0.063.
 __global__ void finalize_kernel(const PointPlan* plan, const PointRec* rec, int n, WalkParams w, int scaleFactor,
                                 float* offR, float* offA, float* corr, float* azd, uint8_t* type,
                                 unsigned long long* stats, const int* pairOf)
 {
     chain_begin();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned lanes = __ballot_sync(0xffffffffu, p < n);
     if (p >= n) return;
-    if (pairOf) stats += 8 * pairOf[p];  // batched calls: statistics per pair
     const PointPlan pl = plan[p];
     const PointRec r = rec[p];
     const WalkOut o = strack_walk(pl, r, w);
@@ -99,16 +101,18 @@ __global__ void finalize_kernel(const PointPlan* plan, const PointRec* rec, int 
     corr[p] = (float)o.cMax;
     if (azd) azd[p] = r.azd;
     type[p] = (uint8_t)o.type;
-    // statistics (printLineSummary)
-    const int isC = o.good && o.type == SB_CMATCH;
-    const int isA = o.good && o.type == SB_AMPMATCH;
-    const int isL = o.good && o.type == SB_AMPMATCHLARGE;
-    const int fail = !(o.good && mask) && o.haveData;
-    if (isC) atomicAdd(&stats[0], 1ull);
-    if (isA) atomicAdd(&stats[1], 1ull);
-    if (isL) atomicAdd(&stats[2], 1ull);
-    if (fail) atomicAdd(&stats[3], 1ull);
-    if (o.nSkip) atomicAdd(&stats[4], (unsigned long long)o.nSkip);
+    // statistics (printLineSummary), per pair in batched calls: one addition
+    // per warp, pair and counter
+    const int pair = pairOf ? pairOf[p] : 0;
+    const unsigned same = __match_any_sync(lanes, pair);
+    const auto count = [&](bool b) { return (unsigned long long)__popc(__ballot_sync(lanes, b) & same); };
+    const unsigned long long c[5] = {count(o.good && o.type == SB_CMATCH), count(o.good && o.type == SB_AMPMATCH),
+                                     count(o.good && o.type == SB_AMPMATCHLARGE),
+                                     count(!(o.good && mask) && o.haveData),
+                                     count(o.nSkip & 1) + 2 * count(o.nSkip & 2)};  // nSkip <= 3
+    if ((threadIdx.x & 31) == __ffs(same) - 1)
+        for (int k = 0; k < 5; ++k)
+            if (c[k]) atomicAdd(&stats[8 * pair + k], c[k]);
 }
 
 // Device plan of the grid for a polynomial initial shift, where every point is

@@ -128,10 +128,11 @@ __device__ double fit_sigma(const float* samp, int x0, int sub, unsigned mask)
 }
 
 // LPF lanes a fit.  A fit is a chain of up to six sums of 18 double
-// exponentials: with one lane a fit a list takes the chain's 35 us however short
-// it is.  Whole calls with 1, 2, 4, 8 lanes: 1.022, 0.998, 0.979, 0.990 ms
-// (1024 x 2048, window 32), 5.34, 5.16, 5.12, 5.12 ms (24 tiles in one call),
-// 42.1, 41.6, 41.6, 42.0 ms (6000 x 12000, window 64).
+// exponentials, so with one lane a fit a short list takes the chain's 35 us;
+// four lanes shorten the chain and cost a quarter more instructions.  One and
+// four lanes: 3,600 fits 34.8 and 19.4 us, 16,384 38.9 and 37.7, 32,400 71.7
+// and 66.5, 65,536 113 and 123, 518,400 739 and 903, 1,960,000 2,651 and 3,338;
+// the list's upper bound decides.  Two and eight lanes lie between.
 template <int LPF>
 __global__ void __launch_bounds__(128) strack_fit_kernel(FitArgs a)
 {
@@ -184,9 +185,13 @@ __global__ void __launch_bounds__(128) strack_fit_kernel(FitArgs a)
 cudaError_t launch_strack_fit(const FitArgs& a, cudaStream_t st)
 {
     if (a.nList <= 0) return cudaSuccess;
-    constexpr int LPF = 4;
-    const long long threads = 2LL * a.nList * LPF;
-    chain(strack_fit_kernel<LPF>, (unsigned)((threads + 127) / 128), 128, 0, st, a);
+    const bool wide = a.nList >= 50000;
+    const long long threads = 2LL * a.nList * (wide ? 1 : 4);
+    const unsigned g = (unsigned)((threads + 127) / 128);
+    if (wide)
+        chain(strack_fit_kernel<1>, g, 128, 0, st, a);
+    else
+        chain(strack_fit_kernel<4>, g, 128, 0, st, a);
     return cudaGetLastError();
 }
 

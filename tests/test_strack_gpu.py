@@ -288,3 +288,20 @@ def test_baseline_phase_flattening(ctx):
         assert (o["type"] == 1).mean() > 0.9 and (g["type"] == 1).mean() > 0.9
         plain = oracle.strack(abi.TrackParams(**kw), a, b)
         assert (plain["type"] == 1).mean() < 0.3  # without the baseline the fringe decorrelates the pair
+
+
+def test_width_fits_of_long_and_short_lists(ctx):
+    """Lists from 50,000 fits up take one lane a fit, shorter ones four: the
+    same grid in one call and in two halves.  Only the order of a fit's double
+    sums differs; a fit that converges feels that far below one float step
+    (6e-8), so azd agrees to a few of them wherever the width is well defined."""
+    a, b = synth.small_pair(device="cuda", na=400, nr=400, seed=31)
+    kw = dict(rStart=24, deltaR=1, deltaA=1, nR=320, wR=16, wA=16, wRa=16, wAa=16, maxTries=0)
+    whole = ctx.strack(abi.TrackParams(aStart=24, nA=160, **kw), a, b)
+    halves = [ctx.strack(abi.TrackParams(aStart=s, nA=80, **kw), a, b) for s in (24, 104)]
+    for key in ("offR", "offA", "corr", "type"):
+        assert np.array_equal(whole[key], np.concatenate([h[key] for h in halves]), equal_nan=True), key
+    z, h = whole["azd"], np.concatenate([h["azd"] for h in halves])
+    ok = whole["type"] == 1
+    assert ok.mean() > 0.5
+    assert np.mean(np.abs(z[ok] - h[ok]) <= 1e-6 * np.abs(z[ok])) > 0.99
