@@ -3,10 +3,10 @@
 // array instead of a cudaMalloc'd buffer, for callers that cannot allocate
 // device memory while they run (see include/speckle_b200.h).
 //
-// The kernel is a variant of strack_amp_kernel (strack_amp.cu): same stages,
-// but patches come from a contiguous caller array, the results go to plain
-// per-patch arrays, the constant tables are computed in shared memory by each
-// CTA, and the per-CTA workspace is a slice of g_noalloc_scratch.
+// The kernel runs the stages of strack_amp.cu with one CTA per patch: patches
+// come from a contiguous caller array, the results go to plain per-patch
+// arrays, the constant tables are computed in shared memory by each CTA, and
+// the per-CTA workspace is a slice of g_noalloc_scratch.
 #include <cuda_runtime.h>
 
 #include "capi_internal.h"
