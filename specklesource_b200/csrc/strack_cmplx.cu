@@ -46,6 +46,10 @@ struct CmplxSmem {
     static constexpr int IMG = W * RS;  // float2 per buffer; two buffers X, Z
     static constexpr size_t bytes = sizeof(float2) * (2 * IMG + W + NFAST * OSW) + sizeof(float) * (NFAST * NFAST) +
                                     sizeof(double) * (NT / 32 + 1) * 8 + 64 + 16;
+    // phase_correct_int works on 2 ps^2 float2 behind that; ps is checked by
+    // sb_strack: 2 ps^2 <= W (W + 1)
+    static constexpr size_t intAt = bytes / 16 * 16 + 16;
+    static constexpr size_t limit = intAt + sizeof(float2) * W * (W + 1);
 };
 
 // |c|^2 of the 2W x 2W surface at unshifted index (cy, cx): columns of parity
@@ -468,7 +472,7 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
             __syncthreads();
         }
         if (a.intf)  // its work space follows the kernel's own (launch_cmplx_t)
-            phase_correct_int<W, RS, NT>(a, pl, X, reinterpret_cast<float2*>(smem_raw + S::bytes / 16 * 16 + 16), red);
+            phase_correct_int<W, RS, NT>(a, pl, X, reinterpret_cast<float2*>(smem_raw + S::intAt), red);
         // ---------------------------------------------------- spectra of both patches (X and Z)
         // rows, then columns; the column pass stores row k of a spectrum at
         // row (k - azShift) mod W, which folds the Doppler roll in (the block
@@ -642,14 +646,23 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
     }
 }
 
+// The dynamic shared memory a kernel may be launched with belongs to the
+// function on the device, not to a context: contexts of other threads launch
+// the same kernel with and without an interferogram.  So every caller sets the
+// largest size that any launch asks for.
+template <int W, int NT, bool F32, bool GAUSS>
+static cudaError_t cmplx_attributes()
+{
+    return cudaFuncSetAttribute(strack_cmplx_kernel<W, NT, F32, GAUSS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)CmplxSmem<W, NT>::limit);
+}
+
 template <int W, int NT, bool F32, bool GAUSS>
 static cudaError_t launch_cmplx_t(const CmplxArgs& a, int nCta, cudaStream_t st)
 {
-    size_t sm = CmplxSmem<W, NT>::bytes;
-    // phase_correct_int works on 2 ps^2 float2 behind the kernel's own
-    if (a.intf) sm = sm / 16 * 16 + 16 + sizeof(float2) * 2 * a.intPs * a.intPs;
-    cudaError_t e = cudaFuncSetAttribute(strack_cmplx_kernel<W, NT, F32, GAUSS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    using S = CmplxSmem<W, NT>;
+    const size_t sm = a.intf ? S::intAt + sizeof(float2) * 2 * a.intPs * a.intPs : S::bytes;
+    const cudaError_t e = cmplx_attributes<W, NT, F32, GAUSS>();
     if (e != cudaSuccess) return e;
     strack_cmplx_kernel<W, NT, F32, GAUSS><<<nCta, NT, sm, st>>>(a);
     return cudaGetLastError();
@@ -668,10 +681,9 @@ template <int W, int NT>
 static int occupancy_cmplx()
 {
     int nb = 0;
-    const size_t sm = CmplxSmem<W, NT>::bytes;
-    cudaFuncSetAttribute(strack_cmplx_kernel<W, NT, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, strack_cmplx_kernel<W, NT, true, false>, NT, sm);
+    cmplx_attributes<W, NT, true, false>();
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, strack_cmplx_kernel<W, NT, true, false>, NT,
+                                                  CmplxSmem<W, NT>::bytes);
     return nb;
 }
 

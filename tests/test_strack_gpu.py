@@ -305,3 +305,42 @@ def test_width_fits_of_long_and_short_lists(ctx):
     ok = whole["type"] == 1
     assert ok.mean() > 0.5
     assert np.mean(np.abs(z[ok] - h[ok]) <= 1e-6 * np.abs(z[ok])) > 0.99
+
+
+def test_interferogram_beside_calls_without(ctx):
+    """The interferogram's work space makes its launches of the complex kernel
+    larger than the others'.  A context that uses one beside a thread whose
+    context matches without and asks for the kernel's launch shape: both keep
+    working."""
+    import threading
+
+    import torch
+    from specklesource_b200 import runtime
+    s1, s2 = synth.make_pair(256, 512, 12, dr=lambda y, x: 1.3 + 0 * x, da=lambda y, x: 0.4 + 0 * x, coherence=0.8,
+                             ramp=0.6)
+    a, b = (s.contiguous().cuda() for s in (s1, s2))
+    fi = torch.from_numpy(np.ascontiguousarray(synth.fringe_interferogram(256, 512, 4, 2, 0.6).astype("<i2"))).cuda()
+    kw = dict(rStart=72, aStart=72, deltaR=32, deltaA=32, nR=8, nA=3, wR=64, wA=64, wRa=64, wAa=64, maxTries=0)
+    pi, pp = abi.TrackParams(**kw, intf=dict(data=fi, nrl=4, nal=2)), abi.TrackParams(**kw)
+    want, plain = ctx.strack(pi, a, b), ctx.strack(pp, a, b)
+    keys = ("offR", "offA", "corr", "type")
+    stop, bad = threading.Event(), []
+
+    def others():
+        with runtime.Context(0) as c:
+            while not stop.is_set():
+                for _ in range(100):
+                    c.lib.sb_set_tuning(c.h, abi.SB_TUNE_COMPLEX, 64, 0, 0)
+                g = c.strack(pp, a, b)
+                bad.extend(k for k in keys if not np.array_equal(g[k], plain[k]))
+
+    t = threading.Thread(target=others)
+    t.start()
+    try:
+        for _ in range(300):
+            g = ctx.strack(pi, a, b)
+            assert all(np.array_equal(g[k], want[k]) for k in keys)
+    finally:
+        stop.set()
+        t.join()
+    assert not bad
