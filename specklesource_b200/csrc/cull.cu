@@ -348,16 +348,27 @@ __device__ __forceinline__ void warp_append(bool yes, int v, int* list, unsigned
     if (yes) list[base + __popc(m & ((1u << lane) - 1u))] = v;
 }
 
+// Tiles of 32 x 8 points, numbered along the rows in one launch dimension (a
+// second one ends at 65,535, which a grid of 524,281 rows exceeds).
+static int cull_tiles(int nR, int nA) { return ((nR + 31) / 32) * ((nA + 7) / 8); }
+__device__ __forceinline__ int2 tile_origin(int nR)
+{
+    const int nx = (nR + 31) / 32, y = blockIdx.x / nx;
+    return make_int2((blockIdx.x - y * nx) * 32, y * 8);
+}
+
 // Step 0: every point; a thread each, 32 x 8 points a block.
 template <bool SLOW>
 __global__ void __launch_bounds__(256) cull_fix_first_kernel(FixArgs a)
 {
     chain_begin();
     if (*a.stop) return;  // uniform
-    const int j = blockIdx.x * 32 + (threadIdx.x & 31), i = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int2 t = tile_origin(a.nR);
+    const int j = t.x + (threadIdx.x & 31), i = t.y + (threadIdx.x >> 5);
     bool cull = false, ok = false;
-    const int p = i * a.nR + j;
+    int p = 0;
     if (i < a.nA && j < a.nR) {
+        p = i * a.nR + j;
         const float oR = a.offR[p], oA = a.offA[p];
         ok = valid_pt(oR, oA);
         cull = fix_decide<true, SLOW>(a, i, j, oR, oA);
@@ -574,7 +585,8 @@ __global__ void __launch_bounds__(256) cull_stats_kernel(StatsArgs a)
     chain_begin();
     constexpr int TX = 32, TY = 8, SX = TX + 2 * ST_BOX, SY = TY + 2 * ST_BOX;
     __shared__ float2 tile[SY][SX];
-    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    const int2 org = tile_origin(a.nR);
+    const int x0 = org.x, y0 = org.y;
     for (int e = threadIdx.x; e < SX * SY; e += 256) {
         const int x = x0 - ST_BOX + e % SX, y = y0 - ST_BOX + e / SX;
         float2 v = make_float2(kCulled, kCulled);
@@ -1106,9 +1118,8 @@ template <bool SLOW>
 cudaError_t launch_fix_pass(sb_context* c, const FixArgs& f)
 {
     cudaStream_t s = c->stream;
-    const dim3 grid((f.nR + 31) / 32, (f.nA + 7) / 8);
     const int wide = c->numSM * 8;
-    chain(cull_fix_first_kernel<SLOW>, grid, 256, 0, s, f);
+    chain(cull_fix_first_kernel<SLOW>, cull_tiles(f.nR, f.nA), 256, 0, s, f);
     chain(cull_fix_apply_kernel, wide, 256, 0, s, f, 0);
     chain(cull_fix_list_kernel<SLOW>, wide, 256, 0, s, f, 1);
     chain(cull_fix_apply_kernel, wide, 256, 0, s, f, 1);
@@ -1208,7 +1219,7 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
 int run_stats(sb_context* c, const CullJob& p, const CullDev* v)
 {
     StatsArgs a{v->offR, v->offA, v->sigmaR, v->sigmaA, p.nR, p.nA, p.qvar};
-    chain(cull_stats_kernel, dim3((p.nR + 31) / 32, (p.nA + 7) / 8), 256, 0, c->stream, a);
+    chain(cull_stats_kernel, cull_tiles(p.nR, p.nA), 256, 0, c->stream, a);
     c->launches++;
     return sb_ctx_cuda(c, cudaGetLastError(), "cull_stats");
 }

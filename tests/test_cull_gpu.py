@@ -122,6 +122,22 @@ def test_cull_large_grid_keep_mask(ctx):
     assert o["nIslands"] > 0
 
 
+def test_cull_tall_grid(ctx):
+    """More than 524,280 rows, where tiles of 8 rows number more than 65,535."""
+    nA, nR = 524281 + 300, 2
+    rng = np.random.default_rng(5)
+    offR = rng.normal(0, 0.3, (nA, nR)).astype(np.float32)
+    offA = rng.normal(0, 0.3, (nA, nR)).astype(np.float32)
+    offR[rng.random((nA, nR)) < 0.05] = -2e9
+    corr = np.ones((nA, nR), np.float32)
+    mt = np.ones((nA, nR), np.uint8)
+    p = abi.CullParams(nR=nR, nA=nA, bR=3, bA=5, nGood=3, sR=1, sA=3, maxR=0.5, maxA=0.5)
+    g, o = ctx.cull(p, offR, offA, corr, mt), oracle.cull(p, offR, offA, corr, mt)
+    assert o["nCulled"] > 0 and (o["offR"] > -1.9e9).sum() > nA / 2
+    _check(g, o)
+    assert g["nCulled"] == o["nCulled"]
+
+
 # ---------------------------------------------------------------- cullls
 
 SLOW, NODATA_BIT = 0x10, 0x40  # stand-ins for lstrack.h's SLOWVEL / NODATATOUSE
