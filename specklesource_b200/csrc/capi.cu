@@ -63,6 +63,7 @@ void* sb_ctx_buf(sb_context* c, const char* name, size_t bytes, cudaError_t* err
         b.bytes = 0;
         cudaError_t e = cudaMallocAsync(&b.ptr, bytes > 0 ? bytes : 16, c->stream);
         if (e != cudaSuccess) {
+            cudaGetLastError();  // reported here: not to the next launch that is checked
             *err = e;
             return nullptr;
         }

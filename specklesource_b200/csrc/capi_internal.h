@@ -51,6 +51,24 @@ struct sb_context {
 int sb_ctx_fail(sb_context* c, int code, const char* fmt, ...);
 int sb_ctx_cuda(sb_context* c, cudaError_t e, const char* what);
 void* sb_ctx_buf(sb_context* c, const char* name, size_t bytes, cudaError_t* err);
+// Workspace for a list of cnt entries that runs *B of them at a time; size(b):
+// bytes for b entries.  It has its full size for all but the shortest lists,
+// because growing it from call to call stalls the other jobs of a server.
+// Where the free memory does not hold that, the list's own size is tried, then
+// half of it again and again down to one entry.  Sets *B to the entries of a
+// chunk (equal chunks: no short last one); null: not even one entry fits.
+template <typename Size>
+char* sb_chunk_buf(sb_context* c, const char* name, int cnt, int* B, Size size)
+{
+    for (int b = cnt < 32 && cnt < *B ? cnt : *B;; b = b > cnt ? cnt : (b + 1) / 2) {
+        cudaError_t e;
+        char* base = (char*)sb_ctx_buf(c, name, size(b), &e);
+        if (!base && b > 1) continue;
+        const int chunks = (cnt + b - 1) / b;
+        *B = (cnt + chunks - 1) / chunks;
+        return base;
+    }
+}
 int sb_image_to_device(sb_context* c, const sb_image* im, const char* name, const void** dptr);
 // A constant table of the context: build() gives its elements (double
 // precision, rounded once) when it is first asked for.  Later calls only look

@@ -482,12 +482,7 @@ struct AmRun {
         const size_t one = layout(c, 16, nullptr, &dop) / 16 + 1;
         int B = (int)(am_chunk_bytes(ctx->numSM, WS) / one);
         B = B < 16 ? 16 : B;
-        // the buffer at its full size for all but the shortest lists: growing it
-        // from call to call stalls the other jobs of a server
-        const size_t bytes = layout(c, cnt < 32 && cnt < B ? cnt : B, nullptr, &dop);
-        const int chunks = (cnt + B - 1) / B;
-        B = (cnt + chunks - 1) / chunks;  // equal chunks: no short last one
-        char* base = (char*)sb_ctx_buf(ctx, "ampScratch", bytes, &e);
+        char* base = sb_chunk_buf(ctx, "ampScratch", cnt, &B, [&](int b) { return layout(c, b, nullptr, &dop); });
         if (!base) return sb_ctx_fail(ctx, SB_ERR_NOMEM, "amplitude workspace allocation failed");
         layout(c, B, base, &dop);
         c.win.win = c.corner;

@@ -769,12 +769,8 @@ static int run_sw(sb_context* c, SwArgs a, int nl)
     const size_t one = SwRun<W>::layout(probe, 16, nullptr, &dop, &az) / 16 + 1;
     int B = (int)(sw_chunk_bytes(c->numSM, W, a.e) / one);
     B = B < 16 ? 16 : B;
-    // the buffer at its full size for all but the shortest lists: growing it
-    // from call to call stalls the other jobs of a server
-    const size_t bytes = SwRun<W>::layout(a, nl < 32 && nl < B ? nl : B, nullptr, &dop, &az);
-    const int chunks = (nl + B - 1) / B;
-    B = (nl + chunks - 1) / chunks;  // equal chunks: no short last one
-    char* base = (char*)sb_ctx_buf(c, "w_scratch", bytes, &e);
+    char* base = sb_chunk_buf(c, "w_scratch", nl, &B,
+                              [&](int b) { return SwRun<W>::layout(a, b, nullptr, &dop, &az); });
     if (!base) return sb_ctx_fail(c, SB_ERR_NOMEM, "strackw workspace allocation failed");
     SwRun<W>::layout(a, B, base, &dop, &az);
     a.az = az;

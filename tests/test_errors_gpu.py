@@ -85,3 +85,39 @@ def test_context_still_works_after_the_errors(ctx, pair):
     r = ctx.strack(_p(), a, b)
     assert (r["type"] == abi.SB_CMATCH).all()
     assert np.allclose(r["offR"], 2.0, atol=1 / 24) and np.allclose(r["offA"], 1.0, atol=1 / 24)
+
+
+@pytest.mark.parametrize("kind", ["strackw", "amplitude"])
+def test_less_memory_than_a_chunk(kind):
+    """A list of 40 points on a GPU whose free memory holds a part of the full
+    workspace (2.0 GB at window 224, 349 MB at amplitude window 128)."""
+    import torch
+    from specklesource_b200 import runtime, synth
+    s1, s2 = synth.shear_pair(device="cpu", na=768, nr=1024, seed=3)
+    a, b = synth.to_numpy(s1), synth.to_numpy(s2)
+    kw = dict(rStart=136, aStart=136, deltaR=70, deltaA=70, nR=8, nA=5)
+    if kind == "strackw":
+        p, leave = _p(**kw, wR=224, wA=224, wRa=224, wAa=224, edgePadR=48, edgePadA=48, navgR=2, navgA=2), 700 << 20
+    else:
+        p, leave = _p(**kw, wR=64, wA=64, wRa=128, wAa=128, noComplex=1, maxTries=1), 160 << 20
+
+    def call(c):
+        return (c.strackw if kind == "strackw" else c.strack)(p, a, b)
+
+    with runtime.Context(0) as c:
+        want = call(c)  # loads the kernels
+    with runtime.Context(0) as c:
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+        hold = torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+        try:
+            got = call(c)
+            held = c.device_bytes()
+        finally:
+            del hold
+            torch.cuda.empty_cache()
+        again = call(c)
+    assert 0 < held < leave
+    for k in ("offR", "offA", "corr", "type"):
+        assert np.array_equal(got[k], want[k]) and np.array_equal(again[k], want[k]), k
