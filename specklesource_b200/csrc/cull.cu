@@ -33,6 +33,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "capi_internal.h"
 #include "chain.cuh"
 
@@ -271,11 +273,23 @@ __global__ void cull_median_kernel(CullArgs a, long long spinLimit)
 // 0.07.  The limits are compared in float: for a float d and a double t,
 // d > t is d > t rounded down.
 //
-// Two steps run over the whole chip; the rest, whose lists are short, in one
-// cluster of CTAs that goes on until a list is empty, so a pass has no host
-// round trip.
+// Two steps run over the whole chip; the rest, whose lists are short as a rule,
+// in one cluster of CTAs that goes on until a list is empty, so a pass has no
+// host round trip.  A list of more than kFixLong points stops the cluster:
+// steps over the whole chip follow, kFixBatch of them per host round trip, then
+// the cluster again.  The line is half a list for the cluster's 8,192 threads.
+// With the cluster alone, with lines of 2,048, 4,096, 8,192 and 16,384, one
+// pass: 2000 x 2000 points, box 5, a tenth of them holes, nGood 20: 28.2, 3.7,
+// 3.7, 3.7, 3.7 ms; box 9, nGood 70: 39.7, 4.6, 4.5, 4.6, 4.6; culls that eat
+// their way in from the edges of 1000 x 1000 points (box 9, nGood 60): 23.6,
+// 11.8, 11.8, 15.2, 23.4; 1969 x 993 points, 2 % outliers, box 5: 1.25, 1.31,
+// 1.25, 1.26, 1.26.  Chains that do not end in kFixSteps steps (2000 x 1000
+// points, box 3 x 1) cost the same either way, 24 ms with the wavefront after
+// them.
 constexpr int kFixSteps = 512;       // bound on the steps of a pass (then the wavefront)
 constexpr int kFixCluster = 8;       // CTAs of the tail kernel
+constexpr unsigned kFixLong = 4096;
+constexpr int kFixBatch = 16;
 
 struct FixArgs {
     const float* offR;
@@ -286,7 +300,8 @@ struct FixArgs {
     int* mark;               // the step that listed a point last
     unsigned* nList;         // per step
     unsigned* nFlipped;      // per step
-    int* stop;               // set when an earlier pass did not converge
+    int* stop;               // 0, or the pass (from 1) that its tail kernel left unfinished
+    int* resume;             // the step that pass goes on from
     int nR, nA, hR, hA;
     int nGood;
     float maxR, maxA, slowMaxR, slowMaxA;  // rounded down to float
@@ -445,9 +460,9 @@ __global__ void __launch_bounds__(256) cull_fix_apply_kernel(FixArgs a, int step
     fix_apply_list(a, step, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5);
 }
 
-// Steps from `step` on until a list is empty, in one cluster.  C, the lists
-// and the counters are read past L1 (other CTAs of the cluster write them);
-// the cluster barriers order the two halves of a step.
+// Steps from `step` on until a list is empty or long or the steps run out, in
+// one cluster.  C, the lists and the counters are read past L1 (other CTAs of
+// the cluster write them); the cluster barriers order the two halves of a step.
 template <bool SLOW>
 __global__ void __cluster_dims__(kFixCluster, 1, 1) __launch_bounds__(1024) cull_fix_tail_kernel(FixArgs a, int step)
 {
@@ -459,14 +474,19 @@ __global__ void __cluster_dims__(kFixCluster, 1, 1) __launch_bounds__(1024) cull
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     };
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-    for (; step < kFixSteps; ++step) {
-        if (__ldcg(a.nList + step) == 0) return;  // the same value in every thread
+    for (;; ++step) {
+        const unsigned n = __ldcg(a.nList + step);  // the same value in every thread
+        if (n == 0) return;
+        if (n > kFixLong || step >= kFixSteps) break;
         fix_decide_list<SLOW>(a, step, tid, nt);
         sync();
         fix_apply_list(a, step, tid >> 5, nt >> 5);
         sync();
     }
-    if (tid == 0) *a.stop = a.pass + 1;
+    if (tid == 0) {
+        *a.resume = step;
+        *a.stop = a.pass + 1;
+    }
 }
 
 // Writes the culls of the converged pass; counts them.
@@ -1113,24 +1133,33 @@ int run_st_wavefront(sb_context* c, const CullArgs& a, int nv, int64_t* nCulledO
     return SB_OK;
 }
 
-// The fixpoint kernels of one pass, without a host round trip.
+// Steps [step, step + n) of a pass over the whole chip (step 0: every point),
+// the tail kernel and, when that converged, the culls, without a host round trip.
 template <bool SLOW>
-cudaError_t launch_fix_pass(sb_context* c, const FixArgs& f)
+cudaError_t launch_fix_steps(sb_context* c, const FixArgs& f, int step, int n, float* offR, float* offA,
+                             unsigned long long* nCulled)
 {
     cudaStream_t s = c->stream;
-    const int wide = c->numSM * 8;
-    chain(cull_fix_first_kernel<SLOW>, cull_tiles(f.nR, f.nA), 256, 0, s, f);
-    chain(cull_fix_apply_kernel, wide, 256, 0, s, f, 0);
-    chain(cull_fix_list_kernel<SLOW>, wide, 256, 0, s, f, 1);
-    chain(cull_fix_apply_kernel, wide, 256, 0, s, f, 1);
-    chain(cull_fix_tail_kernel<SLOW>, kFixCluster, 1024, 0, s, f, 2);
-    c->launches += 5;
+    const int wide = c->numSM * 8, end = step + n;
+    for (; step < end; ++step) {
+        if (step == 0)
+            chain(cull_fix_first_kernel<SLOW>, cull_tiles(f.nR, f.nA), 256, 0, s, f);
+        else
+            chain(cull_fix_list_kernel<SLOW>, wide, 256, 0, s, f, step);
+        chain(cull_fix_apply_kernel, wide, 256, 0, s, f, step);
+    }
+    chain(cull_fix_tail_kernel<SLOW>, kFixCluster, 1024, 0, s, f, end);
+    const long long points = (long long)f.nR * f.nA;
+    chain(cull_apply_kernel, (int)std::min<long long>((points + 255) / 256, c->numSM * 16), 256, 0, s, offR, offA, f.c,
+          points, nCulled, f.stop);
+    c->launches += 2 * n + 2;
     return cudaGetLastError();
 }
 
-// nPasses median passes.  All of them are enqueued as fixpoints; a pass that
-// does not converge stops the ones behind it, is done by the wavefront kernel,
-// and the rest follow.
+// nPasses median passes.  All of them are enqueued as fixpoints.  A pass that
+// its tail kernel leaves unfinished stops the ones behind it and goes on by
+// itself; where its steps run out the wavefront kernel does it.  Then the rest
+// follow.
 int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, int64_t* nCulledOut)
 {
     const long long n = (long long)p.nR * p.nA;
@@ -1178,6 +1207,7 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
     f.flipped = ibase + 2 * n;
     f.mark = ibase + 3 * n;
     f.stop = (int*)cnt;
+    f.resume = f.stop + 1;
     f.nR = p.nR; f.nA = p.nA; f.hR = p.bR / 2; f.hA = p.bA / 2;
     f.nGood = p.rule.nGood;
     f.maxR = float_down(p.rule.maxR);
@@ -1189,29 +1219,34 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
     f.selfTest = p.rule.selfTest;
     f.selfLim = p.rule.selfLim;
     CKC(cudaMemsetAsync(f.mark, 0, (size_t)n * sizeof(int), s), "memset");
+    auto steps_of = [&](int pass, int step, int count) {
+        f.pass = pass;
+        f.nList = steps + perPass * pass;
+        f.nFlipped = f.nList + kFixSteps + 2;
+        return f.slowType ? launch_fix_steps<true>(c, f, step, count, v->offR, v->offA, culled + pass)
+                          : launch_fix_steps<false>(c, f, step, count, v->offR, v->offA, culled + pass);
+    };
     while (done < nPasses) {
         CKC(cudaMemsetAsync(cnt, 0, 16 + sizeof(unsigned long long) * nPasses + sizeof(unsigned) * perPass * nPasses, s),
             "memset");
-        for (int k = done; k < nPasses; ++k) {
-            f.pass = k;
-            f.nList = steps + perPass * k;
-            f.nFlipped = f.nList + kFixSteps + 2;
-            CKC(f.slowType ? launch_fix_pass<true>(c, f) : launch_fix_pass<false>(c, f), "cull_fix");
-            long long ab = (n + 255) / 256;
-            if (ab > (long long)c->numSM * 16) ab = (long long)c->numSM * 16;
-            chain(cull_apply_kernel, (int)ab, 256, 0, s, v->offR, v->offA, C, n, culled + k, f.stop);
-            CKC(cudaGetLastError(), "cull_apply");
-            c->launches++;
+        for (int k = done; k < nPasses; ++k) CKC(steps_of(k, 0, 2), "cull_fix");
+        int pass = nPasses - 1, at[2];  // at: stop, resume
+        for (;;) {
+            unsigned long long k = 0;
+            CKC(cudaMemcpyAsync(at, f.stop, sizeof(at), cudaMemcpyDeviceToHost, s), "d2h");
+            CKC(cudaMemcpyAsync(&k, culled + pass, sizeof(k), cudaMemcpyDeviceToHost, s), "d2h");
+            CKC(cudaStreamSynchronize(s), "cull_fix");
+            *nCulledOut = (int64_t)k;
+            if (at[0] == 0) break;
+            pass = at[0] - 1;
+            if (at[1] >= kFixSteps) {
+                if ((rc = run_st_wavefront(c, a, nv, nCulledOut)) != SB_OK) return rc;
+                break;
+            }
+            CKC(cudaMemsetAsync(f.stop, 0, sizeof(int), s), "memset");
+            CKC(steps_of(pass, at[1], std::min(kFixBatch, kFixSteps - at[1])), "cull_fix");
         }
-        int stop = 0;
-        unsigned long long last = 0;
-        CKC(cudaMemcpyAsync(&stop, f.stop, sizeof(stop), cudaMemcpyDeviceToHost, s), "d2h");
-        CKC(cudaMemcpyAsync(&last, culled + nPasses - 1, sizeof(last), cudaMemcpyDeviceToHost, s), "d2h");
-        CKC(cudaStreamSynchronize(s), "cull_fix");
-        *nCulledOut = (int64_t)last;
-        if (stop == 0) return SB_OK;
-        if ((rc = run_st_wavefront(c, a, nv, nCulledOut)) != SB_OK) return rc;
-        done = stop;  // passes 0 .. stop - 1 are done
+        done = pass + 1;
     }
     return SB_OK;
 }

@@ -109,6 +109,29 @@ def test_cull_fixpoint_edges(ctx, nA, nR, kw):
     assert _same(g["offR"], o["offR"]) and _same(g["offA"], o["offA"]) and g["nCulled"] == o["nCulled"]
 
 
+@pytest.mark.parametrize("kw,sigma,holes", [
+    (dict(bR=9, bA=9, nGood=60, maxR=0.5, maxA=0.5), 0.01, 0.0),   # culls eat their way in from the edges
+    (dict(bR=5, bA=5, nGood=18, maxR=0.5, maxA=0.5), 0.01, 0.1),
+    (dict(bR=5, bA=5, nGood=12, maxR=0.05, maxA=0.05), 0.1, 0.0),
+])
+def test_cull_long_revisit_lists(ctx, kw, sigma, holes):
+    """Revisit lists too long for one cluster: steps over the whole chip (two
+    launches each), the cluster for the short lists after them."""
+    nA, nR = 410, 530
+    rng = np.random.default_rng(2)
+    offR, offA = (rng.normal(0, sigma, (nA, nR)).astype(np.float32) for _ in range(2))
+    offR[rng.random((nA, nR)) < holes] = -2e9
+    corr = np.ones((nA, nR), np.float32)
+    mt = np.ones((nA, nR), np.uint8)
+    for passes in (1, 3):
+        p = abi.CullParams(nR=nR, nA=nA, nCullPasses=passes, sR=1, sA=1, **kw)
+        g = ctx.cull(p, offR, offA, corr, mt)
+        assert ctx.launch_count() > 40
+        o = oracle.cull(p, offR, offA, corr, mt)
+        _check(g, o)
+        assert g["nCulled"] == o["nCulled"]
+
+
 def test_cull_large_grid_keep_mask(ctx):
     """Keep masks on a 700 x 993 grid (rows of the large strack workload's grid)."""
     nA, nR = 700, 993
@@ -193,6 +216,56 @@ def test_cullls_large_grid(ctx):
     o = oracle.cullls(p, X, Y, t)
     _check_ls(g, o)
     assert o["nIslands"] > 0
+
+
+def _chains(first, second, nR=1500):
+    """Rows whose points go one after the other, each because its left
+    neighbour went: with nGood=2 and a 3 x 3 box a row alone loses its end
+    point, then the next.  first: from the first pass on.  second: the end of
+    the row stays until the outlier below it has gone in the first pass.  The
+    rows at the bottom keep points for the later passes."""
+    rng = np.random.default_rng(11)
+    offR = rng.normal(0, 0.01, (9, nR)).astype(np.float32)
+    offA = rng.normal(0, 0.01, (9, nR)).astype(np.float32)
+    offR[6:][rng.random((3, nR)) < 0.2] += np.float32(3)
+    for row in range(6):
+        if not (row == 0 and first or row in (2, 3) and second):
+            offR[row] = offA[row] = -2e9
+    offR[3, 1:] = offA[3, 1:] = -2e9
+    if second:
+        offR[3, 0] = 100
+    return offR, offA
+
+
+@pytest.mark.parametrize("first,second", [(True, False), (False, True), (True, True)])
+def test_cull_passes_that_do_not_converge(ctx, first, second):
+    """Chains longer than the fixpoint's steps: the row-wavefront kernel does
+    such a pass and the rest follow, for cullst and for cullls's limits."""
+    offR, offA = _chains(first, second)
+    nA, nR = offR.shape
+    corr = np.ones((nA, nR), np.float32)
+    mt = np.ones((nA, nR), np.uint8)
+    for passes in (1, 2, 3, 5):
+        p = abi.CullParams(nR=nR, nA=nA, bR=3, bA=3, nGood=2, maxR=0.5, maxA=0.5, sR=2, sA=2, nCullPasses=passes)
+        g, o = ctx.cull(p, offR, offA, corr, mt), oracle.cull(p, offR, offA, corr, mt)
+        _check(g, o)
+        assert g["nCulled"] == o["nCulled"]
+        if passes == 5:
+            assert not first or (o["offR"][0] < -1e9).all()
+            assert not second or (o["offR"][2] < -1e9).all()
+        assert (o["offR"][6:] > -1e9).any()
+        t = np.full((nA, nR), SLOW, np.uint8)
+        t[:, ::3] = 1
+        q = abi.CullLSParams(nx=nR, ny=nA, boxSize=3, nGood=2, maxX=0.5, maxY=0.5, nCullPasses=passes, deltaT=16.0,
+                             dx=15.0, dy=15.0, nOver=10.0, slowVelMask=SLOW, noDataMask=NODATA_BIT)
+        _check_ls(ctx.cullls(q, offR, offA, t), oracle.cullls(q, offR, offA, t))
+    # the wavefront kernel was reached: without naps its waits run out
+    assert ctx.lib.sb_set_wait_limit(ctx.h, 0) == abi.SB_OK
+    try:
+        with pytest.raises(Exception, match="timed out"):
+            ctx.cull(p, offR, offA, corr, mt)
+    finally:
+        assert ctx.lib.sb_set_wait_limit(ctx.h, 1 << 26) == abi.SB_OK
 
 
 def test_wavefront_wait_times_out_and_context_stays_usable(ctx):
