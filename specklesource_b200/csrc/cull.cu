@@ -290,6 +290,7 @@ constexpr int kFixSteps = 512;       // bound on the steps of a pass (then the w
 constexpr int kFixCluster = 8;       // CTAs of the tail kernel
 constexpr unsigned kFixLong = 4096;
 constexpr int kFixBatch = 16;
+constexpr int kFixPasses = 16;       // passes enqueued together (4 KB of counters each)
 
 struct FixArgs {
     const float* offR;
@@ -300,7 +301,7 @@ struct FixArgs {
     int* mark;               // the step that listed a point last
     unsigned* nList;         // per step
     unsigned* nFlipped;      // per step
-    int* stop;               // 0, or the pass (from 1) that its tail kernel left unfinished
+    int* stop;               // 0, or the pass of the group (from 1) that its tail kernel left unfinished
     int* resume;             // the step that pass goes on from
     int nR, nA, hR, hA;
     int nGood;
@@ -1156,10 +1157,10 @@ cudaError_t launch_fix_steps(sb_context* c, const FixArgs& f, int step, int n, f
     return cudaGetLastError();
 }
 
-// nPasses median passes.  All of them are enqueued as fixpoints.  A pass that
-// its tail kernel leaves unfinished stops the ones behind it and goes on by
-// itself; where its steps run out the wavefront kernel does it.  Then the rest
-// follow.
+// nPasses median passes, kFixPasses of them enqueued as fixpoints at a time.  A
+// pass that its tail kernel leaves unfinished stops the ones behind it and goes
+// on by itself; where its steps run out the wavefront kernel does it.  Then the
+// rest follow.
 int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, int64_t* nCulledOut)
 {
     const long long n = (long long)p.nR * p.nA;
@@ -1192,12 +1193,13 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
     // C (bytes), then int arrays: two revisit lists, the flips, the marks
     uint8_t* C = (uint8_t*)sb_ctx_buf(c, "c_fix", (size_t)n + 16 + (size_t)n * 4 * sizeof(int), &e);
     // stop flag, culled counts, then list and flip counts per pass and step
+    const int group = std::min(nPasses, kFixPasses);
     const size_t perPass = 2 * (kFixSteps + 2);
-    unsigned* cnt = (unsigned*)sb_ctx_buf(
-        c, "c_fixcnt", 16 + sizeof(unsigned long long) * nPasses + sizeof(unsigned) * perPass * nPasses, &e);
+    const size_t cntBytes = 16 + (sizeof(unsigned long long) + sizeof(unsigned) * perPass) * group;
+    unsigned* cnt = (unsigned*)sb_ctx_buf(c, "c_fixcnt", cntBytes, &e);
     if (!C || !cnt) return sb_ctx_fail(c, SB_ERR_NOMEM, "device allocation failed");
     unsigned long long* culled = (unsigned long long*)(cnt + 4);
-    unsigned* steps = (unsigned*)(culled + nPasses);
+    unsigned* steps = (unsigned*)(culled + group);
     int* ibase = (int*)(((uintptr_t)(C + n) + 15) & ~(uintptr_t)15);
     FixArgs f;
     f.offR = v->offR; f.offA = v->offA;
@@ -1218,7 +1220,6 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
     f.slowMask = p.rule.slowMask;
     f.selfTest = p.rule.selfTest;
     f.selfLim = p.rule.selfLim;
-    CKC(cudaMemsetAsync(f.mark, 0, (size_t)n * sizeof(int), s), "memset");
     auto steps_of = [&](int pass, int step, int count) {
         f.pass = pass;
         f.nList = steps + perPass * pass;
@@ -1227,10 +1228,10 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
                           : launch_fix_steps<false>(c, f, step, count, v->offR, v->offA, culled + pass);
     };
     while (done < nPasses) {
-        CKC(cudaMemsetAsync(cnt, 0, 16 + sizeof(unsigned long long) * nPasses + sizeof(unsigned) * perPass * nPasses, s),
-            "memset");
-        for (int k = done; k < nPasses; ++k) CKC(steps_of(k, 0, 2), "cull_fix");
-        int pass = nPasses - 1, at[2];  // at: stop, resume
+        CKC(cudaMemsetAsync(f.mark, 0, (size_t)n * sizeof(int), s), "memset");
+        CKC(cudaMemsetAsync(cnt, 0, cntBytes, s), "memset");
+        int pass = std::min(group, nPasses - done) - 1, at[2];  // the group's last; stop, resume
+        for (int k = 0; k <= pass; ++k) CKC(steps_of(k, 0, 2), "cull_fix");
         for (;;) {
             unsigned long long k = 0;
             CKC(cudaMemcpyAsync(at, f.stop, sizeof(at), cudaMemcpyDeviceToHost, s), "d2h");
@@ -1246,7 +1247,7 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
             CKC(cudaMemsetAsync(f.stop, 0, sizeof(int), s), "memset");
             CKC(steps_of(pass, at[1], std::min(kFixBatch, kFixSteps - at[1])), "cull_fix");
         }
-        done = pass + 1;
+        done += pass + 1;
     }
     return SB_OK;
 }

@@ -132,6 +132,21 @@ def test_cull_long_revisit_lists(ctx, kw, sigma, holes):
         assert g["nCulled"] == o["nCulled"]
 
 
+def test_cull_many_passes():
+    """Passes enqueued in groups: any number of them on one workspace."""
+    from specklesource_b200 import runtime
+    offR, offA, corr, mt = offsets_field(40, 60, 3)
+    held = []
+    for passes in (1, 16, 17, 1000):
+        with runtime.Context(0) as c:
+            p = abi.CullParams(nR=60, nA=40, bR=5, bA=5, nGood=9, maxR=0.2, maxA=0.2, nCullPasses=passes)
+            g, o = c.cull(p, offR, offA, corr, mt), oracle.cull(p, offR, offA, corr, mt)
+            _check(g, o)
+            assert g["nCulled"] == o["nCulled"]
+            held.append(c.device_bytes())
+    assert held[3] == held[2] == held[1]
+
+
 def test_cull_large_grid_keep_mask(ctx):
     """Keep masks on a 700 x 993 grid (rows of the large strack workload's grid)."""
     nA, nR = 700, 993
