@@ -323,6 +323,10 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
     constexpr int N1 = L::N1, N2 = L::N2, LG = L::LG, R1 = L::R1, R2 = L::R2, NW = NT / 32;
     static_assert((W * W) % NT == 0 && NT % W == 0, "whole rows per thread");
     constexpr int RPT = W * W / NT;  // consecutive rows per thread in the load phase
+    // rows of a float partial sum: 4 at W = 32 with 128 and with 256 threads
+    // (the 128-thread shape is there for occupancy, not to sum over more rows)
+    constexpr int FR = W == 32 ? 4 : RPT;
+    static_assert(RPT % FR == 0, "whole partial sums");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* X = reinterpret_cast<float2*>(smem_raw);
     float2* Z = X + IMG;
@@ -358,8 +362,8 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
             if (it + 2 * G < nList) pAfter = a.list[it + 2 * G];
         }
         // ---------------------------------------------------- getPatches
-        // per-thread partial sums over the RPT rows in float, block totals in double
-        float f[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        // per-thread partial sums over FR rows in float, block totals in double
+        float f[RPT / FR][6] = {};
         int nLow = 0;
         // batches of LB rows: every load of a batch is issued before any is
         // used (the Hanning taper and the byte order are predicates, not
@@ -392,17 +396,22 @@ __global__ void __launch_bounds__(NT, cmplx_min_ctas<GAUSS>(W, NT)) strack_cmplx
             const float pw1 = __fadd_rn(__fmul_rn(z1.x, z1.x), __fmul_rn(z1.y, z1.y));
             const float pw2 = __fadd_rn(__fmul_rn(z2.x, z2.x), __fmul_rn(z2.y, z2.y));
             nLow += (pw1 < thr || pw2 < thr);
-            f[0] += pw1;
-            f[1] += pw2;
-            f[2] += z1.x;
-            f[3] += z1.y;
-            f[4] += z2.x;
-            f[5] += z2.y;
+            float(&g)[6] = f[(r0 + u) / FR];
+            g[0] += pw1;
+            g[1] += pw2;
+            g[2] += z1.x;
+            g[3] += z1.y;
+            g[4] += z2.x;
+            g[5] += z2.y;
             X[i * RS + jc] = z1;
             Z[i * RS + jc] = z2;
             }
         }
-        double s[7] = {f[0], f[1], f[2], f[3], f[4], f[5], (double)nLow};
+        double s[7] = {0, 0, 0, 0, 0, 0, (double)nLow};
+#pragma unroll
+        for (int r = 0; r < RPT / FR; ++r)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) s[k] += f[r][k];
         block_allsum<7, NT>(s, red);
         const bool haveData = !(s[6] > 20.0) && !(s[0] < thrAll || s[1] < thrAll);
         if (!haveData) {

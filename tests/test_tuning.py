@@ -68,3 +68,25 @@ def test_every_compiled_shape_keeps_parity():
                         for k in ("offR", "offA", "corr", "type"):
                             assert np.array_equal(ref[k], g[k]), (W, t, k)
             ctx.lib.sb_set_tuning(ctx.h, abi.SB_TUNE_COMPLEX, W, 0, 0)
+
+
+@pytest.mark.gpu
+def test_window_32_thread_counts_agree():
+    """Both thread counts of window 32 sum the patch powers in float over runs
+    of four rows and in double beyond: the same grids."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from specklesource_b200 import build, runtime, synth
+    build.build()
+    s1, s2 = synth.small_pair(na=512, nr=1024)
+    a, b = synth.to_numpy(s1), synth.to_numpy(s2)
+    p = abi.TrackParams(rStart=40, aStart=40, deltaR=16, deltaA=16, nR=59, nA=27, wR=32, wA=32, wRa=32, wAa=32,
+                        maxTries=0)
+    g = []
+    with runtime.Context(0, tuning=False) as c:
+        for threads in (128, 256):
+            assert c.lib.sb_set_tuning(c.h, abi.SB_TUNE_COMPLEX, 32, threads, 0) == abi.SB_OK
+            g.append(c.strack(p, a, b))
+    for k in ("offR", "offA", "corr", "azd", "type"):
+        assert np.array_equal(g[0][k], g[1][k]), k
