@@ -11,9 +11,16 @@
 // to 225, the 1024 x 2048 pair through strackw at W = 64 from 1.58 to 1.44 ms.
 //
 // Every kernel launched this way calls chain_begin() first, in every thread, so
-// nothing is read or written before the earlier kernels are done.  A kernel
-// that follows anything but a kernel (a wait for the copy stream's event) is
-// launched plainly.
+// nothing is read or written before the earlier kernels are done.  What the
+// kernel before it writes must not be promised to be read-only (__ldg, const
+// __restrict__ kernel parameters): the promise holds for a kernel's lifetime,
+// which begins before that write is done, and lets a load move above
+// chain_begin().  Tables, images and what older kernels wrote are read-only for
+// it.
+// Where the operation before a launch is a copy, a memset or an event, full
+// stream order applies with or without the attribute.  The plan, the records'
+// first values, the stage selections and the complex stage always come after
+// one and are launched plainly.
 #pragma once
 #include <cuda_runtime.h>
 

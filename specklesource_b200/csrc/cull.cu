@@ -328,7 +328,7 @@ __device__ __forceinline__ bool fix_decide(const FixArgs& a, int i, int j, float
 #pragma unroll 4
         for (int jj = j1; jj <= j2; ++jj) {
             const int q = q0 + jj;
-            const float r = __ldg(a.offR + q), z = __ldg(a.offA + q);
+            const float r = a.offR[q], z = a.offA[q];
             const bool gone = !FIRST && (ii < i || (ii == i && jj < j)) && __ldcg(a.c + q);
             const bool v = valid_pt(r, z) && !gone;
             const float dr = oR - r, da = oA - z;
@@ -404,7 +404,7 @@ __device__ __forceinline__ void fix_decide_list(const FixArgs& a, int step, int 
         int v = 0;
         if (t < n) {
             const int p = __ldcg(list + t);
-            const float oR = __ldg(a.offR + p), oA = __ldg(a.offA + p);
+            const float oR = a.offR[p], oA = a.offA[p];
             flip = fix_decide<false, SLOW>(a, p / a.nR, p % a.nR, oR, oA) != (__ldcg(a.c + p) != 0);
             v = valid_pt(oR, oA) ? p : ~p;
         }

@@ -6,6 +6,7 @@
 
 namespace sbk {
 
+// No __restrict__ on the kernels' pointers: chain.cuh says why.
 static int part_tiles(int n) { return (n + PART_TILE - 1) / PART_TILE; }
 
 size_t partition_scratch_ints(int n, int K)
@@ -15,8 +16,7 @@ size_t partition_scratch_ints(int n, int K)
 }
 size_t partition_keyoff_at(int n, int K) { return (size_t)2 * part_tiles(n) * K; }
 
-__global__ void __launch_bounds__(PART_TILE) part_count_kernel(const int* __restrict__ key, int n, int K,
-                                                               int* __restrict__ tileCnt)
+__global__ void __launch_bounds__(PART_TILE) part_count_kernel(const int* key, int n, int K, int* tileCnt)
 {
     chain_begin();
     __shared__ int h[PART_KMAX];
@@ -30,9 +30,8 @@ __global__ void __launch_bounds__(PART_TILE) part_count_kernel(const int* __rest
 }
 
 // One CTA of 1024 threads: exclusive scan over tiles, key by key.
-__global__ void __launch_bounds__(1024) part_scan_kernel(const int* __restrict__ tileCnt, int nTiles, int K,
-                                                         int* __restrict__ tileOff, int* __restrict__ keyOff,
-                                                         int* count)
+__global__ void __launch_bounds__(1024) part_scan_kernel(const int* tileCnt, int nTiles, int K, int* tileOff,
+                                                         int* keyOff, int* count)
 {
     chain_begin();
     __shared__ int ws[32];
@@ -83,9 +82,8 @@ __global__ void __launch_bounds__(1024) part_scan_kernel(const int* __restrict__
 // the block, and a longer chain of tiles (a million points and more) is shorter
 // there.
 constexpr int PART_SCAN_WARP = 1024;
-__global__ void __launch_bounds__(32 * PART_KMAX) part_scan_keys_kernel(const int* __restrict__ tileCnt, int nTiles,
-                                                                        int K, int* __restrict__ tileOff,
-                                                                        int* __restrict__ keyOff, int* count)
+__global__ void __launch_bounds__(32 * PART_KMAX) part_scan_keys_kernel(const int* tileCnt, int nTiles, int K,
+                                                                        int* tileOff, int* keyOff, int* count)
 {
     chain_begin();
     __shared__ int total[PART_KMAX];
@@ -128,10 +126,8 @@ __global__ void __launch_bounds__(32 * PART_KMAX) part_scan_keys_kernel(const in
     }
 }
 
-__global__ void __launch_bounds__(PART_TILE) part_write_kernel(const int* __restrict__ key,
-                                                               const int* __restrict__ val, int n, int K,
-                                                               const int* __restrict__ tileOff,
-                                                               const int* __restrict__ keyOff, int* __restrict__ out)
+__global__ void __launch_bounds__(PART_TILE) part_write_kernel(const int* key, const int* val, int n, int K,
+                                                               const int* tileOff, const int* keyOff, int* out)
 {
     chain_begin();
     __shared__ int wc[PART_KMAX][32];  // [key][warp]: count, then exclusive prefix over warps
