@@ -946,14 +946,14 @@ extern "C" int sb_strack(sb_context* c, const sb_track_params* p, const sb_image
         a.azThresh = p->azDefocusThresh;
         a.checkAzFocus = p->checkAzFocus;
         a.azEff = needFill ? dAz : nullptr;
-        a.twWs = tw_table(c, Ws);
-        a.tw2Ws = tw_table(c, 2 * Ws);
+        a.twWs = onChip ? tw_table(c, Ws) : nullptr;
+        a.tw2Ws = onChip ? tw_table(c, 2 * Ws) : nullptr;
         a.tau = tau_table(c, Ws);
         a.osD = osD_table(c);
         a.gauss = p->gaussFlag ? 1 : 0;
         a.rec = drec;
         a.fit = dfit;
-        if (!a.twWs || !a.tw2Ws || !a.tau || !a.osD)
+        if ((onChip && (!a.twWs || !a.tw2Ws)) || !a.tau || !a.osD)
             return sb_ctx_fail(c, SB_ERR_NOMEM, "amplitude workspace allocation failed");
         cudaEventRecord(c->sev[2 + 2 * stage], c->stream);
         if ((rc = amp_try(c, Ws, a)) != SB_OK) return rc;
@@ -1331,7 +1331,7 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
             a.hanCorr = p->hanningFlag ? 1.5 : 1.0;
             a.twW = tw_table(c, W);
             a.tau = tau_table(c, W);
-                a.osD = osD_table(c);
+            a.osD = osD_table(c);
             a.gauss = p->gaussFlag ? 1 : 0;
             a.azThresh = p->azDefocusThresh;
             a.checkAzFocus = p->checkAzFocus;
@@ -1438,14 +1438,14 @@ extern "C" int sb_strack_batch(sb_context* c, int32_t nPairs, const sb_track_par
             a.azThresh = p->azDefocusThresh;
             a.checkAzFocus = p->checkAzFocus;
             a.azEff = needFill ? dAz : nullptr;
-            a.twWs = tw_table(c, Ws);
-            a.tw2Ws = tw_table(c, 2 * Ws);
+            a.twWs = onChip ? tw_table(c, Ws) : nullptr;
+            a.tw2Ws = onChip ? tw_table(c, 2 * Ws) : nullptr;
             a.tau = tau_table(c, Ws);
             a.osD = osD_table(c);
             a.gauss = p->gaussFlag ? 1 : 0;
             a.rec = brec;
             a.fit = dfit;
-            if (!a.twWs || !a.tw2Ws || !a.tau || !a.osD)
+            if ((onChip && (!a.twWs || !a.tw2Ws)) || !a.tau || !a.osD)
                 return sb_ctx_fail(c, SB_ERR_NOMEM, "amplitude workspace allocation failed");
             if ((rc = amp_try(c, Ws, a)) != SB_OK) return rc;
             FitArgs f = make_fit_args(p, dfit, cnt, stage, brec);

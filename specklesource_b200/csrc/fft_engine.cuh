@@ -264,165 +264,57 @@ struct RegDFT {
 };
 
 // ---------------------------------------------------------------- line FFTs
-// Step 2 of the line transforms (see fft_lines_io): radix-N2 DFTs over the N2
-// contiguous slots of every (line, k1), all loaded before the first store;
-// outputs go to dst(l, k1, k2, value).  Ends with a barrier.
-template <int N1, int N2, int DIR, int NL, int NLI, int NT, int LS, int ES, int IS, typename Dst>
-__device__ __forceinline__ void fft_step2(float2* base, Dst dst, const float2* __restrict__ tw)
-{
-    constexpr int N = N1 * N2;
-    constexpr int T2 = NL * N1;
-    constexpr int R2 = (T2 + NT - 1) / NT;
-    const int tid = threadIdx.x;
-    float2 v2[R2][N2];
-#pragma unroll
-    for (int r = 0; r < R2; ++r) {
-        const int t = tid + r * NT;
-        if (T2 % NT == 0 || t < T2) {
-            const int l = t % NL, k1 = t / NL;
-            const float2* p = base + (l % NLI) * LS + (l / NLI) * IS + (N2 * k1) * ES;
-#pragma unroll
-            for (int n2 = 0; n2 < N2; ++n2) v2[r][n2] = p[n2 * ES];
-            RegDFT<N2, DIR, N>::run(v2[r], tw);
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int r = 0; r < R2; ++r) {
-        const int t = tid + r * NT;
-        if (T2 % NT == 0 || t < T2) {
-            const int l = t % NL, k1 = t / NL;
-#pragma unroll
-            for (int k2 = 0; k2 < N2; ++k2) dst(l, k1, k2, v2[r][k2]);
-        }
-    }
-    __syncthreads();
-}
-
-// Lines are addressed as base + (l % NLI) * LS + (l / NLI) * IS (NLI lines per
-// image, several images side by side).  Element k of a line is at k * ES.
-// All strides are compile-time constants, so addresses fold to immediates.
-//
-// Step 1 takes its inputs from `src(l, k)` and step 2 hands its outputs to
-// `dst(l, k1, k2, value)` (output index k = k1 + N1 * k2, k2 a compile-time
-// constant after unrolling); `base` holds the intermediate.  With the identity
-// functors the transform is in place.  src may gather from another buffer or
-// apply an element-wise map (in place is then still safe: step 1 of a thread
-// writes exactly the slots it read).  When src reads slots of `base` that other
-// threads write in step 1 (a permuting gather within the same buffer), set
-// SYNC1: every input is loaded before the first store.  dst is called after a
-// barrier that follows the last read of `base`, so it may overwrite `base`.
-template <int N1, int N2, int DIR, int NL, int NLI, int NT, int LS, int ES, int IS, bool SYNC1, typename Src,
-          typename Dst>
-__device__ __forceinline__ void fft_lines_io(float2* base, Src src, Dst dst, const float2* __restrict__ tw)
-{
-    constexpr int N = N1 * N2;
-    constexpr int T1 = NL * N2;
-    constexpr int R1 = (T1 + NT - 1) / NT;
-    const int tid = threadIdx.x;
-    float2 v[R1][N1];
-    auto step1 = [&](int r) {
-        const int t = tid + r * NT;
-        const int l = t % NL, n2 = t / NL;
-        float2* p = base + (l % NLI) * LS + (l / NLI) * IS + n2 * ES;
-        RegDFT<N1, DIR, N>::run(v[r], tw);
-        // k1 * n2 < N1 * N2 = N: the twiddle index needs no reduction
-#pragma unroll
-        for (int k1 = 1; k1 < N1; ++k1) v[r][k1] = twmul_rt<DIR>(v[r][k1], tw, k1 * n2);
-#pragma unroll
-        for (int k1 = 0; k1 < N1; ++k1) p[(N2 * k1) * ES] = v[r][k1];
-    };
-#pragma unroll
-    for (int r = 0; r < R1; ++r) {
-        const int t = tid + r * NT;
-        if (T1 % NT == 0 || t < T1) {
-            const int l = t % NL, n2 = t / NL;
-#pragma unroll
-            for (int n1 = 0; n1 < N1; ++n1) v[r][n1] = src(l, N2 * n1 + n2);
-            if constexpr (!SYNC1) step1(r);
-        }
-    }
-    if constexpr (SYNC1) {
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < R1; ++r) {
-            const int t = tid + r * NT;
-            if (T1 % NT == 0 || t < T1) step1(r);
-        }
-    }
-    __syncthreads();
-    fft_step2<N1, N2, DIR, NL, NLI, NT, LS, ES, IS>(base, dst, tw);
-}
-
-// In-place transform of the lines (identity src/dst).
-template <int N1, int N2, int DIR, int NL, int NLI, int NT, int LS, int ES, int IS>
+// In-place transform of NL lines with NT threads: element k of line l at
+// l LS + k ES.  All strides are compile-time constants, so addresses fold to
+// immediates.  In the first step a thread stores exactly the slots it read; in
+// the second every input is loaded before the first store.  Ends with a barrier.
+template <int N1, int N2, int DIR, int NL, int NT, int LS, int ES>
 __device__ __forceinline__ void fft_lines(float2* base, const float2* __restrict__ tw)
 {
-    auto at = [base](int l, int k) -> float2* { return base + (l % NLI) * LS + (l / NLI) * IS + k * ES; };
-    auto src = [at](int l, int k) { return *at(l, k); };
-    auto dst = [at](int l, int k1, int k2, float2 z) { *at(l, k1 + N1 * k2) = z; };
-    fft_lines_io<N1, N2, DIR, NL, NLI, NT, LS, ES, IS, false>(base, src, dst, tw);
-}
-
-// Two transforms of the same NL input lines in one pass: with u = src(l, k),
-// the lines at base get DFT(u) and the lines at base + IS get
-// DFT(u * mul(l, k)).  Each input is read once; step 2 then runs over all
-// 2 NL lines (dst sees l in [0, 2 NL): l / NL selects the transform).
-// SYNC1 as in fft_lines_io.
-template <int N1, int N2, int DIR, int NL, int NT, int LS, int ES, int IS, bool SYNC1, typename Src, typename Mul,
-          typename Dst>
-__device__ __forceinline__ void fft_lines_dual(float2* base, Src src, Mul mul, Dst dst,
-                                               const float2* __restrict__ tw)
-{
     constexpr int N = N1 * N2;
-    constexpr int T1 = NL * N2;
-    constexpr int R1 = (T1 + NT - 1) / NT;
+    constexpr int T1 = NL * N2, T2 = NL * N1;
+    constexpr int R1 = (T1 + NT - 1) / NT, R2 = (T2 + NT - 1) / NT;
     const int tid = threadIdx.x;
-    float2 va[R1][N1], vb[R1][N1];
-    auto step1 = [&](int r) {
-        const int t = tid + r * NT;
-        const int l = t % NL, n2 = t / NL;
-        RegDFT<N1, DIR, N>::run(va[r], tw);
-        RegDFT<N1, DIR, N>::run(vb[r], tw);
-        float2* pa = base + l * LS + n2 * ES;
-        float2* pb = pa + IS;
-#pragma unroll
-        for (int k1 = 0; k1 < N1; ++k1) {
-            if (k1 > 0) {
-                float2 w = tw[k1 * n2];
-                if (DIR > 0) w.y = -w.y;
-                va[r][k1] = cmul(va[r][k1], w);
-                vb[r][k1] = cmul(vb[r][k1], w);
-            }
-            pa[(N2 * k1) * ES] = va[r][k1];
-            pb[(N2 * k1) * ES] = vb[r][k1];
-        }
-    };
 #pragma unroll
     for (int r = 0; r < R1; ++r) {
         const int t = tid + r * NT;
         if (T1 % NT == 0 || t < T1) {
             const int l = t % NL, n2 = t / NL;
+            float2* p = base + l * LS + n2 * ES;
+            float2 v[N1];
 #pragma unroll
-            for (int n1 = 0; n1 < N1; ++n1) {
-                const int k = N2 * n1 + n2;
-                const float2 u = src(l, k);
-                va[r][n1] = u;
-                vb[r][n1] = cmul(u, mul(l, k));
-            }
-            if constexpr (!SYNC1) step1(r);
-        }
-    }
-    if constexpr (SYNC1) {
-        __syncthreads();
+            for (int n1 = 0; n1 < N1; ++n1) v[n1] = p[(N2 * n1) * ES];
+            RegDFT<N1, DIR, N>::run(v, tw);
+            // k1 * n2 < N1 * N2 = N: the twiddle index needs no reduction
 #pragma unroll
-        for (int r = 0; r < R1; ++r) {
-            const int t = tid + r * NT;
-            if (T1 % NT == 0 || t < T1) step1(r);
+            for (int k1 = 1; k1 < N1; ++k1) v[k1] = twmul_rt<DIR>(v[k1], tw, k1 * n2);
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) p[(N2 * k1) * ES] = v[k1];
         }
     }
     __syncthreads();
-    fft_step2<N1, N2, DIR, 2 * NL, NL, NT, LS, ES, IS>(base, dst, tw);
+    float2 v[R2][N2];
+#pragma unroll
+    for (int r = 0; r < R2; ++r) {
+        const int t = tid + r * NT;
+        if (T2 % NT == 0 || t < T2) {
+            const float2* p = base + (t % NL) * LS + (N2 * (t / NL)) * ES;
+#pragma unroll
+            for (int n2 = 0; n2 < N2; ++n2) v[r][n2] = p[n2 * ES];
+            RegDFT<N2, DIR, N>::run(v[r], tw);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R2; ++r) {
+        const int t = tid + r * NT;
+        if (T2 % NT == 0 || t < T2) {
+            float2* p = base + (t % NL) * LS + (t / NL) * ES;
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) p[(N1 * k2) * ES] = v[r][k2];
+        }
+    }
+    __syncthreads();
 }
 
 // Factorisation used for each supported transform length.
@@ -436,16 +328,6 @@ template <> struct Split<48>  { static constexpr int N1 = 6,  N2 = 8;  };
 template <> struct Split<64>  { static constexpr int N1 = 8,  N2 = 8;  };
 template <> struct Split<96>  { static constexpr int N1 = 6,  N2 = 16; };
 template <> struct Split<128> { static constexpr int N1 = 8,  N2 = 16; };
-
-// 2-D transform of NIMG row-major N x N images in shared memory (row stride
-// RS float2, image stride IS float2): rows (range) then columns (azimuth).
-template <int N, int DIR, int NIMG, int NT, int RS, int IS>
-__device__ __forceinline__ void fft2d_smem(float2* base, const float2* __restrict__ tw)
-{
-    constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
-    fft_lines<N1, N2, DIR, N * NIMG, N, NT, RS, 1, IS>(base, tw);  // rows: line = row
-    fft_lines<N1, N2, DIR, N * NIMG, N, NT, 1, RS, IS>(base, tw);  // columns: line = column
-}
 
 // ---------------------------------------------------------------- staged planes
 // Tile of G lines of an N x N row-major array in a global workspace.
@@ -461,7 +343,7 @@ template <int N, int DIR, int NT, int LS, int ES>
 __device__ __forceinline__ void staged_tile_fft(float2* tile, const float2* __restrict__ tw)
 {
     constexpr int G = StagedTile<N>::G;
-    fft_lines<Split<N>::N1, Split<N>::N2, DIR, G, G, NT, LS, ES, 0>(tile, tw);
+    fft_lines<Split<N>::N1, Split<N>::N2, DIR, G, NT, LS, ES>(tile, tw);
 }
 
 // 2-D transform of an N x N row-major array anywhere in memory (row stride N;

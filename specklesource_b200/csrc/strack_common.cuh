@@ -178,23 +178,4 @@ __host__ __device__ inline WalkOut strack_walk(const PointPlan& pl, const PointR
 __device__ __forceinline__ uint32_t bswap32(uint32_t v) { return __byte_perm(v, 0, 0x0123); }
 __device__ __forceinline__ uint32_t bswap16x2(uint32_t v) { return __byte_perm(v, 0, 0x2301); }
 
-// One complex sample of an SLC image (loadBuffer, speckleTrack.c:1369-1399).
-__device__ __forceinline__ float2 load_sample(const void* __restrict__ img, int nr, int row, int col, int sampleType,
-                                              int byteOrder)
-{
-    const size_t k = (size_t)row * (size_t)nr + (size_t)col;
-    if (sampleType == SB_CFLOAT32) {
-        uint2 w = __ldg(reinterpret_cast<const uint2*>(img) + k);
-        if (byteOrder == SB_MSB) {
-            w.x = bswap32(w.x);
-            w.y = bswap32(w.y);
-        }
-        return make_float2(__uint_as_float(w.x), __uint_as_float(w.y));
-    } else {
-        uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(img) + k);
-        if (byteOrder == SB_MSB) w = bswap16x2(w);
-        return make_float2((float)(int16_t)(w & 0xffffu), (float)(int16_t)(w >> 16));
-    }
-}
-
 }  // namespace sbk

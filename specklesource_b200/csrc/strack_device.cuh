@@ -335,161 +335,7 @@ __device__ __forceinline__ ArgMax oversample_peak_warp(const float* blk, const f
     return osr_result(best);
 }
 
-// ---------------------------------------------------------------- LM fit
-// gaussPeak1D (speckleTrack.c:2137-2202) with mrqminMod/mrqcofMod
-// (:2309-2416) and a full-pivot Gauss-Jordan solve, in double precision.
-// One warp per fit; lanes 0..17 hold the samples (x, y).  Every lane runs the
-// 3x3 algebra redundantly on warp-reduced sums.
-
-struct LMSums {
-    double al[6];  // alpha 11, 21, 22, 31, 32, 33
-    double be[3];
-    double chisq;
-};
-
-__device__ __forceinline__ LMSums lm_cof(double x, double y, bool active, const double a[4])
-{
-    LMSums s;
-    double dyda[4] = {0, 0, 0, 0};
-    double ymod = 0.0;
-    if (active) {
-        const double sig = a[3];
-        const double t = x - a[2];
-        const double argx = 0.5 * t * t / (sig * sig);
-        const double ex = exp(-argx);
-        ymod = a[1] * ex;
-        dyda[1] = ex;
-        dyda[2] = ymod * t / (sig * sig);
-        dyda[3] = ymod * t * t / (sig * sig * sig);
-    }
-    const double sig2i = active ? 1.0 / (0.1 * 0.1) : 0.0;
-    const double dy = active ? y - ymod : 0.0;
-    const double w1 = dyda[1] * sig2i, w2 = dyda[2] * sig2i, w3 = dyda[3] * sig2i;
-    s.al[0] = w1 * dyda[1];
-    s.al[1] = w2 * dyda[1];
-    s.al[2] = w2 * dyda[2];
-    s.al[3] = w3 * dyda[1];
-    s.al[4] = w3 * dyda[2];
-    s.al[5] = w3 * dyda[3];
-    s.be[0] = dy * w1;
-    s.be[1] = dy * w2;
-    s.be[2] = dy * w3;
-    s.chisq = dy * dy * sig2i;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) s.al[k] = warp_allsum(s.al[k]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) s.be[k] = warp_allsum(s.be[k]);
-    s.chisq = warp_allsum(s.chisq);
-    return s;
-}
-
-__device__ __forceinline__ void lm_unpack(const LMSums& s, double al[4][4], double be[4])
-{
-    al[1][1] = s.al[0];
-    al[2][1] = al[1][2] = s.al[1];
-    al[2][2] = s.al[2];
-    al[3][1] = al[1][3] = s.al[3];
-    al[3][2] = al[2][3] = s.al[4];
-    al[3][3] = s.al[5];
-    be[1] = s.be[0];
-    be[2] = s.be[1];
-    be[3] = s.be[2];
-}
-
-// Gauss-Jordan with full pivoting (3x3, one right-hand side); false if singular.
-__device__ __forceinline__ bool gaussj3(double a[4][4], double b[4])
-{
-    int indxc[4], indxr[4], ipiv[4] = {0, 0, 0, 0};
-    int irow = 1, icol = 1;
-    for (int i = 1; i <= 3; i++) {
-        double big = 0.0;
-        for (int j = 1; j <= 3; j++)
-            if (ipiv[j] != 1)
-                for (int k = 1; k <= 3; k++) {
-                    if (ipiv[k] == 0) {
-                        if (fabs(a[j][k]) >= big) {
-                            big = fabs(a[j][k]);
-                            irow = j;
-                            icol = k;
-                        }
-                    } else if (ipiv[k] > 1)
-                        return false;
-                }
-        ++(ipiv[icol]);
-        if (irow != icol) {
-            for (int l = 1; l <= 3; l++) {
-                double t = a[irow][l];
-                a[irow][l] = a[icol][l];
-                a[icol][l] = t;
-            }
-            double t = b[irow];
-            b[irow] = b[icol];
-            b[icol] = t;
-        }
-        indxr[i] = irow;
-        indxc[i] = icol;
-        if (a[icol][icol] == 0.0) return false;
-        const double pivinv = 1.0 / a[icol][icol];
-        a[icol][icol] = 1.0;
-        for (int l = 1; l <= 3; l++) a[icol][l] *= pivinv;
-        b[icol] *= pivinv;
-        for (int ll = 1; ll <= 3; ll++)
-            if (ll != icol) {
-                const double dum = a[ll][icol];
-                a[ll][icol] = 0.0;
-                for (int l = 1; l <= 3; l++) a[ll][l] -= a[icol][l] * dum;
-                b[ll] -= b[icol] * dum;
-            }
-    }
-    (void)indxr;
-    (void)indxc;
-    return true;
-}
-
-// Returns sigma = a[3]/2 of the fit (all lanes).
-__device__ __forceinline__ double gauss_peak_1d(float sample, int xpos, int lane)
-{
-    const bool active = lane < NGAUSS;
-    float mx = active ? sample : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const double maxC = (double)fmaxf(mx, 0.f);
-    const double x = (double)xpos;
-    const double y = active ? (double)sample / maxC : 0.0;
-    const double xc = (double)__shfl_sync(0xffffffffu, xpos, NGAUSS / 2);
-    double a[4] = {0.0, 1.0, xc, 2.0};
-    double alamda = 0.001;
-    LMSums s0 = lm_cof(x, y, active, a);
-    double alpha[4][4], beta[4];
-    lm_unpack(s0, alpha, beta);
-    double ochisq = s0.chisq;
-    double lasti = 2e9;
-    for (int it = 0; it < 5; ++it) {
-        double covar[4][4], da[4];
-        for (int j = 1; j <= 3; j++) {
-            for (int k = 1; k <= 3; k++) covar[j][k] = alpha[j][k];
-            covar[j][j] = alpha[j][j] * (1.0 + alamda);
-            da[j] = beta[j];
-        }
-        if (!gaussj3(covar, da)) break;
-        double atry[4] = {0.0, a[1] + da[1], a[2] + da[2], a[3] + da[3]};
-        LMSums s1 = lm_cof(x, y, active, atry);
-        if (s1.chisq < ochisq) {
-            alamda *= 0.1;
-            ochisq = s1.chisq;
-            lm_unpack(s1, alpha, beta);
-            a[1] = atry[1];
-            a[2] = atry[2];
-            a[3] = atry[3];
-        } else {
-            alamda *= 10.0;
-        }
-        if (fabs(a[2] - lasti) < 0.001) break;
-        lasti = a[2];
-    }
-    return a[3] * .5;
-}
-
+// ---------------------------------------------------------------- Doppler, -gauss
 // Doppler roll from the lag-1 sums (estDopCarrier1, dopplerEstimation.c:25-40),
 // rescaled to wA.  A NaN angle (all-zero sums) gives roll 0.
 __device__ __forceinline__ int dop_shift(double sr1, double si1, double sr2, double si2, int nAz, int wA)

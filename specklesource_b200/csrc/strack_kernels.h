@@ -94,8 +94,8 @@ struct AmpArgs {
     float azThresh;
     int checkAzFocus;
     const int* azEff;     // azShift in effect for each point (nullptr: use rec.azset)
-    const float2* twWs;   // W_Ws table (Ws = wa*s)
-    const float2* tw2Ws;  // W_{2Ws} table
+    const float2* twWs;   // W_Ws table (Ws = wa*s); the shared-memory tries
+    const float2* tw2Ws;  // W_{2Ws} table; the same
     const float2* tau;    // parity twiddles for Ws
     const float2* osD;    // real form of the oversampling matrix
     PointRec* rec;
