@@ -230,6 +230,11 @@ __global__ void __launch_bounds__(128) sw_rows_kernel(SwArgs a, int hr0, int hr1
     float* H = a.H + ((size_t)pt * 2 + q) * N * N;
     const int c0 = q ? 2 * a.e : 0, c1 = q ? N - 2 * a.e : N;  // image 2: the chip's columns
     const int rows = q ? min(G, hr1 - j0 + 1) : G;
+    // Half width 2, the 5 x 5 box that fast-flow pairs are run with, has its own
+    // loop: 2.87 ms for 3.05 in the general one at W = 64 (7,018 points), 1.96
+    // for 2.13 at 128 (1,566), 3.57 for 3.81 at 224 (836).  The other widths take
+    // the general one; half width 3 would gain as much (3.17 -> 2.92, 2.23 ->
+    // 2.00, 3.94 -> 3.61) and has no loop of its own here.
     const int lane = threadIdx.x & 31;
     for (int l = threadIdx.x >> 5; l < rows; l += NT / 32) {
         const float* p = in + l * PR;

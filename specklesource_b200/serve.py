@@ -33,7 +33,11 @@ _STRACK_POINT_BYTES = 20 + 80 + 16 + 160 + 17 + 64
 # most one list chunk (kPeakChunk in csrc/capi.cu)
 _PEAK_JOB_BYTES = 960
 _PEAK_CHUNK = 1 << 19
-# per-CTA workspaces (float2 elements), sized like the kernels' own
+# chunk planes of an amplitude try, in float2 elements per CTA slot (two slots
+# an SM): the full size that csrc/strack_amp.cu allocates for windows from 48
+# up.  Tries of windows 16 to 32 keep their arrays in shared memory; their
+# entries only make the estimate of small jobs more careful (tables, grids
+# rounded up).
 _AMP_SCRATCH = {16: 3 * 16 * 16 + 32 * 32 * 3 // 2, 24: 3 * 24 * 24 + 48 * 48 * 3 // 2,
                 32: 3 * 32 * 32 + 64 * 64 * 3 // 2, 48: 3 * 48 * 48 + 96 * 96 * 3 // 2,
                 64: 3 * 64 * 64 + 128 * 128 * 3 // 2, 96: 3 * 96 * 96 + 192 * 192 * 3 // 2,
@@ -67,7 +71,10 @@ def _image_bytes(img):
 
 
 def job_device_bytes(job, num_sm=148):
-    """Upper estimate of the device memory a job holds while it runs."""
+    """Upper estimate of the device memory a job holds while it runs.  The
+    chunk planes of strackw and of the larger amplitude tries count at their
+    full size (csrc/strackw.cu's sw_chunk_bytes, csrc/strack_amp.cu's
+    am_chunk_bytes); a call makes do with less where the device has less."""
     if job.kind == "cull":
         return int(job.cull.nR) * int(job.cull.nA) * 64
     p = job.params

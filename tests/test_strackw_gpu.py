@@ -77,6 +77,14 @@ def test_strackw_every_window_and_box(ctx, shear, W, pad, navg, n, step):
     _check(ctx, _p(W, pad, navg, n=n, step=step), ai, bi)
 
 
+def test_strackw_several_chunks(ctx, shear):
+    """More points than two chunks hold (about 860 each), the last chunk
+    shorter than the others; then a short list on the same planes."""
+    a, b = shear
+    _check(ctx, _p(32, 5, 1, n=(44, 43), step=22, deltaA=15), a, b)
+    _check(ctx, _p(32, 5, 1, n=(3, 5), step=40), a, b)
+
+
 def test_strackw_int16_msb_and_mask(ctx, shear):
     a, b = shear
     ai = np.stack([np.round(a.real * 2000), np.round(a.imag * 2000)], -1).astype(">i2")
