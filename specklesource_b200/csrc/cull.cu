@@ -364,13 +364,18 @@ __device__ __forceinline__ void warp_append(bool yes, int v, int* list, unsigned
     if (yes) list[base + __popc(m & ((1u << lane) - 1u))] = v;
 }
 
-// Tiles of 32 x 8 points, numbered along the rows in one launch dimension (a
-// second one ends at 65,535, which a grid of 524,281 rows exceeds).
-static int cull_tiles(int nR, int nA) { return ((nR + 31) / 32) * ((nA + 7) / 8); }
-__device__ __forceinline__ int2 tile_origin(int nR)
+// Launch of a block per tile of 32 x 8 points.  Rows of tiles past 65,535, where
+// the second launch dimension ends (grids of 524,281 rows and more), go into
+// the third; numbering the tiles in one dimension cost the first step 3 % for
+// the division.
+static dim3 cull_tiles(int nR, int nA)
 {
-    const int nx = (nR + 31) / 32, y = blockIdx.x / nx;
-    return make_int2((blockIdx.x - y * nx) * 32, y * 8);
+    const unsigned ny = (nA + 7) / 8;
+    return dim3((nR + 31) / 32, std::min(ny, 65535u), (ny + 65534) / 65535);
+}
+__device__ __forceinline__ int2 tile_origin()
+{
+    return make_int2(blockIdx.x * 32, (blockIdx.z * 65535 + blockIdx.y) * 8);
 }
 
 // Step 0: every point; a thread each, 32 x 8 points a block.
@@ -379,7 +384,7 @@ __global__ void __launch_bounds__(256) cull_fix_first_kernel(FixArgs a)
 {
     chain_begin();
     if (*a.stop) return;  // uniform
-    const int2 t = tile_origin(a.nR);
+    const int2 t = tile_origin();
     const int j = t.x + (threadIdx.x & 31), i = t.y + (threadIdx.x >> 5);
     bool cull = false, ok = false;
     int p = 0;
@@ -606,7 +611,7 @@ __global__ void __launch_bounds__(256) cull_stats_kernel(StatsArgs a)
     chain_begin();
     constexpr int TX = 32, TY = 8, SX = TX + 2 * ST_BOX, SY = TY + 2 * ST_BOX;
     __shared__ float2 tile[SY][SX];
-    const int2 org = tile_origin(a.nR);
+    const int2 org = tile_origin();
     const int x0 = org.x, y0 = org.y;
     for (int e = threadIdx.x; e < SX * SY; e += 256) {
         const int x = x0 - ST_BOX + e % SX, y = y0 - ST_BOX + e / SX;
