@@ -275,20 +275,20 @@ __global__ void cull_median_kernel(CullArgs a, long long spinLimit)
 //
 // Two steps run over the whole chip; the rest, whose lists are short as a rule,
 // in one cluster of CTAs that goes on until a list is empty, so a pass has no
-// host round trip.  A list of more than kFixLong points stops the cluster:
-// steps over the whole chip follow, kFixBatch of them per host round trip, then
-// the cluster again.  The line is half a list for the cluster's 8,192 threads.
-// With the cluster alone, with lines of 2,048, 4,096, 8,192 and 16,384, one
-// pass: 2000 x 2000 points, box 5, a tenth of them holes, nGood 20: 28.2, 3.7,
-// 3.7, 3.7, 3.7 ms; box 9, nGood 70: 39.7, 4.6, 4.5, 4.6, 4.6; culls that eat
-// their way in from the edges of 1000 x 1000 points (box 9, nGood 60): 23.6,
-// 11.8, 11.8, 15.2, 23.4; 1969 x 993 points, 2 % outliers, box 5: 1.25, 1.31,
-// 1.25, 1.26, 1.26.  Chains that do not end in kFixSteps steps (2000 x 1000
-// points, box 3 x 1) cost the same either way, 24 ms with the wavefront after
-// them.
+// host round trip.  A list of more than kFixLong points, half a list for the
+// cluster's 8,192 threads, stops the cluster once its lists add up to more than
+// kFixSum: steps over the whole chip follow, kFixBatch of them per host round
+// trip, then the cluster again.  With the cluster alone and with this rule, one
+// pass: 2000 x 2000 points, box 5, a tenth of them holes, nGood 20: 28.2 and
+// 3.7 ms; box 9, nGood 70: 39.7 and 4.5; culls that eat their way in from the
+// edges of 1000 x 1000 points (box 9, nGood 60): 23.6 and 14.6.  Lists that
+// only start long are left to the cluster: 1969 x 993 points with 8 % outliers,
+// box 5, three passes and the statistics 1.84 and 1.85 ms (2.00 to 2.09 without
+// kFixSum).  Chains that do not end in kFixSteps steps (1000 rows of 2000
+// points, box 3 x 1) take 24 ms either way, the wavefront after them included.
 constexpr int kFixSteps = 512;       // bound on the steps of a pass (then the wavefront)
 constexpr int kFixCluster = 8;       // CTAs of the tail kernel
-constexpr unsigned kFixLong = 4096;
+constexpr unsigned kFixLong = 4096, kFixSum = 32768;
 constexpr int kFixBatch = 16;
 constexpr int kFixPasses = 16;       // passes enqueued together (4 KB of counters each)
 
@@ -480,10 +480,12 @@ __global__ void __cluster_dims__(kFixCluster, 1, 1) __launch_bounds__(1024) cull
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     };
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+    unsigned sum = 0;
     for (;; ++step) {
         const unsigned n = __ldcg(a.nList + step);  // the same value in every thread
         if (n == 0) return;
-        if (n > kFixLong || step >= kFixSteps) break;
+        sum += n;
+        if ((n > kFixLong && sum > kFixSum) || step >= kFixSteps) break;
         fix_decide_list<SLOW>(a, step, tid, nt);
         sync();
         fix_apply_list(a, step, tid >> 5, nt >> 5);
