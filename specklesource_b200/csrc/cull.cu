@@ -1237,22 +1237,24 @@ int run_st_data(sb_context* c, const CullJob& p, const CullDev* v, int nPasses, 
     while (done < nPasses) {
         CKC(cudaMemsetAsync(f.mark, 0, (size_t)n * sizeof(int), s), "memset");
         CKC(cudaMemsetAsync(cnt, 0, cntBytes, s), "memset");
-        int pass = std::min(group, nPasses - done) - 1, at[2];  // the group's last; stop, resume
+        int pass = std::min(group, nPasses - done) - 1;  // the last of the group
         for (int k = 0; k <= pass; ++k) CKC(steps_of(k, 0, 2), "cull_fix");
         for (;;) {
-            unsigned long long k = 0;
-            CKC(cudaMemcpyAsync(at, f.stop, sizeof(at), cudaMemcpyDeviceToHost, s), "d2h");
-            CKC(cudaMemcpyAsync(&k, culled + pass, sizeof(k), cudaMemcpyDeviceToHost, s), "d2h");
+            struct {
+                int stop, resume, unused[2];
+                unsigned long long culled[kFixPasses];
+            } at;
+            CKC(cudaMemcpyAsync(&at, cnt, 16 + sizeof(unsigned long long) * group, cudaMemcpyDeviceToHost, s), "d2h");
             CKC(cudaStreamSynchronize(s), "cull_fix");
-            *nCulledOut = (int64_t)k;
-            if (at[0] == 0) break;
-            pass = at[0] - 1;
-            if (at[1] >= kFixSteps) {
+            if (at.stop) pass = at.stop - 1;
+            *nCulledOut = (int64_t)at.culled[pass];
+            if (at.stop == 0) break;
+            if (at.resume >= kFixSteps) {
                 if ((rc = run_st_wavefront(c, a, nv, nCulledOut)) != SB_OK) return rc;
                 break;
             }
             CKC(cudaMemsetAsync(f.stop, 0, sizeof(int), s), "memset");
-            CKC(steps_of(pass, at[1], std::min(kFixBatch, kFixSteps - at[1])), "cull_fix");
+            CKC(steps_of(pass, at.resume, std::min(kFixBatch, kFixSteps - at.resume)), "cull_fix");
         }
         done += pass + 1;
     }

@@ -78,7 +78,7 @@ def test_strackw_every_window_and_box(ctx, shear, W, pad, navg, n, step):
 
 
 def test_strackw_several_chunks(ctx, shear):
-    """More points than two chunks hold (about 860 each), the last chunk
+    """More points than two chunks hold (about 880 each), the last chunk
     shorter than the others; then a short list on the same planes."""
     a, b = shear
     _check(ctx, _p(32, 5, 1, n=(44, 43), step=22, deltaA=15), a, b)
